@@ -129,8 +129,8 @@ def _blocks(g, fmt, N, K):
         out[:, :2] = half(spread / 73.6)
         out[:, 2:] = _bytes(g, -127, 128, nb, 32).to(torch.int8).view(torch.uint8)
     elif fmt == "Q4_0":
-        out[:, :2] = half(spread / 4.6)
-        out[:, 2:] = _bytes(g, 0, 256, nb, 16).to(torch.uint8)
+        out[:, :2] = half(spread / 4.3)
+        out[:, 2:] = (_bytes(g, 1, 16, nb, 16) | (_bytes(g, 1, 16, nb, 16) << 4)).to(torch.uint8)  # -7 .. 7
     else:  # sub-blocks with scales 32 .. 63 and minima 7.5 d sc, the middle of the quants
         d = spread / (4.6 * 47.5)
         out[:, :2], out[:, 2:4] = half(d), half(7.5 * d)
