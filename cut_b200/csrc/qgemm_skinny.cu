@@ -170,8 +170,9 @@ __global__ void __launch_bounds__(sk_threads(FMT), 1)
   auto aborted = [&]() { return *reinterpret_cast<volatile uint32_t *>(abort_flag) != 0; };
 
   if (warp == 0) {
-    // ---- MMA issuer ----------------------------------------------------------------------
-    if (lane == 0 && nunits) {
+    // ---- MMA issuer (converged, one elected lane: loop variables and descriptors stay in uniform registers) ----
+    const bool leader = elect_one();
+    if (nunits) {
       const uint64_t proto = umma_desc_sw128(0);
       const uint32_t desc_hi = (uint32_t)(proto >> 32), lo0 = (uint32_t)proto;
       const uint32_t w_lo0 = lo0 + ((smem_u32(b_ring) & 0x3FFFFu) >> 4), t_lo0 = lo0 + ((smem_u32(a_ring) & 0x3FFFFu) >> 4);
@@ -182,26 +183,28 @@ __global__ void __launch_bounds__(sk_threads(FMT), 1)
       uint32_t d = tmem_base, acc = 0;           // acc 0: the next MMA starts a tile's accumulator
       bool dead = false;
       for (uint32_t j = 0; j < nstages; ++j) {
-        if (!mbar_spin_bounded(fullb_u + sb * 8, pb) || !mbar_spin_bounded(fulla_u + sa * 8, pa)) {
-          give_up();
+        const bool ok = mbar_spin_bounded(fullb_u + sb * 8, pb) && mbar_spin_bounded(fulla_u + sa * 8, pa);
+        if (!__all_sync(0xffffffffu, ok)) {
+          if (leader) give_up();
           dead = true;
           break;
         }
         tc_fence_after();
         const uint32_t t_lo = t_lo0 + sa * a_tile_desc, w_lo = w_lo0 + sb * w_tile_desc;
-        // 16 k = 32 bytes = 2 descriptor units along the swizzled row
-        umma_f16(d, t_lo, w_lo, desc_hi, idesc, acc);
-        umma_f16(d, t_lo + 2, w_lo + 2, desc_hi, idesc, 1);
-        umma_f16(d, t_lo + 4, w_lo + 4, desc_hi, idesc, 1);
-        umma_f16(d, t_lo + 6, w_lo + 6, desc_hi, idesc, 1);
+        if (leader) {  // 16 k = 32 bytes = 2 descriptor units along the swizzled row
+          umma_f16(d, t_lo, w_lo, desc_hi, idesc, acc);
+          umma_f16(d, t_lo + 2, w_lo + 2, desc_hi, idesc, 1);
+          umma_f16(d, t_lo + 4, w_lo + 4, desc_hi, idesc, 1);
+          umma_f16(d, t_lo + 6, w_lo + 6, desc_hi, idesc, 1);
+          umma_commit(cons_u + sc * 8);  // the stage is consumed when these MMAs have read it
+        }
         acc = 1;
-        umma_commit(cons_u + sc * 8);  // the stage is consumed when these MMAs have read it
         if (++sa == SA) sa = 0, pa ^= 1u;
         if (++sb == NB) sb = 0, pb ^= 1u;
         if (++sc == NC) sc = 0;
         if (--left == 0) left = nk * SK_SUBS, d += SK_BW, acc = 0;  // the next tile's columns
       }
-      if (!dead) umma_commit(accum_u);
+      if (!dead && leader) umma_commit(accum_u);
     }
     __syncwarp();
   } else if (warp == 1) {

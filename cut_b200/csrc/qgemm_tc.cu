@@ -18,10 +18,8 @@
 // of tensor memory.
 //   warp 0      allocates the TMEM columns; one lane issues the MMAs of every K stage
 //               and commits them to the stage's "consumed" barrier, which frees both
-//               the activation stage and the weight slot.  Its instruction stream is the kernel's critical
-//               path (a lone thread retires an instruction every ~6 cycles), so the
-//               loop keeps ring indices and descriptor words incrementally and
-//               waits by polling, not by parking;
+//               the activation stage and the weight slot.  The loop keeps ring indices
+//               and descriptor words incrementally and waits by polling, not by parking;
 //   warp 2      a second issuer for the second token pair (independent accumulator);
 //   warp 1      one lane issues the TMA tensor copies of the activation blocks
 //               (64 k x 128 tokens of fp16, 128-byte swizzle, rows past M are
@@ -51,7 +49,7 @@ namespace cutb {
 namespace {
 
 template <int FMT>
-__global__ void __launch_bounds__(TC_MAX_THREADS, 1) qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmapA, const TcParams p) {
+__global__ void __launch_bounds__(tc_max_threads(FMT), 1) qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmapA, const TcParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // tiles must start on a 1024-byte boundary (the 128-byte swizzle repeats every 8 rows)
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -104,8 +102,11 @@ __global__ void __launch_bounds__(TC_MAX_THREADS, 1) qgemm_tc_kernel(const __gri
 
   if (warp == 0 || warp == 2) {
     // ---- MMA issuers: issuer i owns the token pairs i, i + NI (256 tokens = 256 TMEM columns) ----
+    // The warp runs converged and one elected lane issues, so that loop variables and descriptors stay in uniform
+    // registers (behind a lane test every MMA first moved its operands there: 95-140 cycles per instruction).
     const uint32_t me = warp >> 1;
-    if (lane == 0 && me < NI) {
+    const bool leader = elect_one();
+    if (me < NI) {
       const uint32_t npairs = (MB + 1) >> 1;
       // descriptor words: start address in the low word, stride / version / swizzle in the high word
       const uint64_t proto = umma_desc_sw128(0);
@@ -115,8 +116,9 @@ __global__ void __launch_bounds__(TC_MAX_THREADS, 1) qgemm_tc_kernel(const __gri
       uint32_t sa = 0, pa = 0, sb = 0, pb = 0, sc = 0;
       bool dead = false;
       for (uint32_t ks = 0; ks < nk; ++ks) {
-        if (!mbar_spin_bounded(fullb_u + sb * 8, pb) || !mbar_spin_bounded(fulla_u + sa * 8, pa)) {
-          give_up();
+        const bool ok = mbar_spin_bounded(fullb_u + sb * 8, pb) && mbar_spin_bounded(fulla_u + sa * 8, pa);
+        if (!__all_sync(0xffffffffu, ok)) {
+          if (leader) give_up();
           dead = true;
           break;
         }
@@ -128,18 +130,20 @@ __global__ void __launch_bounds__(TC_MAX_THREADS, 1) qgemm_tc_kernel(const __gri
             const uint32_t idesc = (2 * pr + 2 <= MB) ? idesc256 : idesc128;
             const uint32_t tl = t_lo + pr * 2 * TC_TILE_DESC, d = tmem_base + pr * 256;
             // 16 k = 32 bytes = 2 descriptor units along the swizzled row
-            umma_f16(d, w_lo, tl, desc_hi, idesc, acc);
-            umma_f16(d, w_lo + 2, tl + 2, desc_hi, idesc, 1);
-            umma_f16(d, w_lo + 4, tl + 4, desc_hi, idesc, 1);
-            umma_f16(d, w_lo + 6, tl + 6, desc_hi, idesc, 1);
+            if (leader) {
+              umma_f16(d, w_lo, tl, desc_hi, idesc, acc);
+              umma_f16(d, w_lo + 2, tl + 2, desc_hi, idesc, 1);
+              umma_f16(d, w_lo + 4, tl + 4, desc_hi, idesc, 1);
+              umma_f16(d, w_lo + 6, tl + 6, desc_hi, idesc, 1);
+            }
           }
         }
-        umma_commit(cons_u + sc * 8);  // the stage is consumed when these MMAs have read it
+        if (leader) umma_commit(cons_u + sc * 8);  // the stage is consumed when these MMAs have read it
         if (++sa == SA) sa = 0, pa ^= 1u;
         if (++sb == NB) sb = 0, pb ^= 1u;
         if (++sc == NC) sc = 0;
       }
-      if (!dead) umma_commit(accum_u);  // this issuer's accumulators are complete
+      if (!dead && leader) umma_commit(accum_u);  // this issuer's accumulators are complete
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -329,25 +333,47 @@ __global__ void __launch_bounds__(TC_MAX_THREADS, 1) qgemm_tc_kernel(const __gri
   }
 }
 
-// K split: the planes of partial sums added in a fixed order, then the fused epilogue (paired rows included).
-__global__ void tc_splitk_reduce_kernel(const TcParams p) {
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t total = (size_t)p.M * p.N;
-  float sum = 0.f;
-  uint32_t m = 0, n = 0;
-  const bool in = idx < total;
-  if (in) {
-    m = (uint32_t)(idx / p.N), n = (uint32_t)(idx % p.N);
-    for (uint32_t z = 0; z < p.ksplit; ++z) sum += p.partial[(size_t)z * total + idx];
+// K split: the planes of partial sums added in a fixed order, then the fused epilogue (paired rows included).  Bound by L2
+// (the planes were just written); V = 4 sums per thread with every plane's load in flight where N and the rows allow 16-byte
+// accesses (512 x 4096, four planes: 20.1 us with one sum per thread).
+template <int V> __global__ void __launch_bounds__(256) tc_splitk_reduce_kernel(const TcParams p) {
+  const size_t total = (size_t)p.M * p.N, idx = ((size_t)blockIdx.x * 256 + threadIdx.x) * V;
+  if (idx >= total) return;
+  const uint32_t m = (uint32_t)(idx / p.N), n = (uint32_t)(idx % p.N);
+  float sum[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i) sum[i] = 0.f;
+#pragma unroll 4
+  for (uint32_t z = 0; z < p.ksplit; ++z) {
+    const float *src = p.partial + z * total + idx;
+    if constexpr (V == 4) {
+      const float4 f = __ldg(reinterpret_cast<const float4 *>(src));
+      sum[0] += f.x, sum[1] += f.y, sum[2] += f.z, sum[3] += f.w;
+    } else {
+#pragma unroll
+      for (int i = 0; i < V; ++i) sum[i] += __ldg(src + i);
+    }
   }
-  if (p.glu) {  // gate and up columns sit in neighbouring threads (N is even, so a pair never straddles a row)
-    const float up = __shfl_xor_sync(0xffffffffu, sum, 1);
-    if (in && !(n & 1u)) p.C[(size_t)m * p.ldc + (n >> 1)] = apply_epilogue(sum, CUTB_FUSION_UNARY, p.fusion_op, 0.f) * up;
-    return;
+  if constexpr (V > 1) {
+    if (p.glu) {  // gate and up columns are neighbours (N is even, so a pair never straddles a row)
+#pragma unroll
+      for (int i = 0; i < V; i += 2)
+        p.C[(size_t)m * p.ldc + (n + i) / 2] = apply_epilogue(sum[i], CUTB_FUSION_UNARY, p.fusion_op, 0.f) * sum[i + 1];
+      return;
+    }
   }
-  if (!in) return;
-  const float dv = p.fusion_type == CUTB_FUSION_BINARY ? p.D[(size_t)m * p.ldd + n] : 0.f;
-  p.C[(size_t)m * p.ldc + n] = apply_epilogue(sum, p.fusion_type, p.fusion_op, dv);
+  if constexpr (V == 4) {
+    float d[4] = {};
+    if (p.fusion_type == CUTB_FUSION_BINARY) {
+      const float4 f = *reinterpret_cast<const float4 *>(p.D + (size_t)m * p.ldd + n);
+      d[0] = f.x, d[1] = f.y, d[2] = f.z, d[3] = f.w;
+    }
+    apply_epilogue_n<4>(sum, d, p.fusion_type, p.fusion_op);
+    *reinterpret_cast<float4 *>(p.C + (size_t)m * p.ldc + n) = make_float4(sum[0], sum[1], sum[2], sum[3]);
+  } else {
+    const float dv = p.fusion_type == CUTB_FUSION_BINARY ? p.D[(size_t)m * p.ldd + n] : 0.f;
+    p.C[(size_t)m * p.ldc + n] = apply_epilogue(sum[0], p.fusion_type, p.fusion_op, dv);
+  }
 }
 
 size_t tc_smem_bytes(uint32_t mb, uint32_t sa, uint32_t nb, uint32_t ksub) {
@@ -393,28 +419,33 @@ bool qgemm_tc_supported(const cutb_qmatmul_desc &d) {
 }
 
 namespace {
-// Token blocks per CTA and K split.  Few weight rows (a 4096-row projection is 32 column tiles) would leave most SMs
-// idle at 512 tokens per CTA.  With a long K (the down projection, K = 14336) the K stages are shared out over
-// blockIdx.z instead: every weight is still dequantised once, 512 tokens amortise it, and the partial sums meet in
-// the workspace (512 x 14336 x 4096: 112 us with 128 tokens per CTA).  Otherwise fewer tokens per CTA until the grid
-// covers at least half of the SMs: each weight tile is then dequantised once per token group, which costs far less
-// than the idle SMs.
-void tc_shape_plan(const cutb_qmatmul_desc &d, uint32_t sm_count, uint32_t *mb_out, uint32_t *ksplit_out) {
+// Up to 256 tokens the tensor work of a 64-k stage (256-512 cycles) is less than what the stage's two barrier waits and four
+// to eight MMA issues take the issuer: stages of 128 k halve the waits per k, and shared memory has room for them there.
+uint32_t tc_ksub(uint32_t mb) { return mb <= 2 ? 2u : 1u; }
+
+// Token blocks per CTA and K split, by an estimate of the time (us) that follows measurements on all the shapes below within
+// a tenth: a 64-k stage of a CTA, the CTA's start and epilogue, and for a split the planes of partial sums through L2 and a second
+// launch.  A stage costs almost the same for one to three token blocks (dequantising 128 weight rows sets the pace; with four it is
+// the activations through L2), so few large CTAs with their K shared out beat many small ones.  Rule before (token blocks only,
+// K split only for 512 tokens and K >= 8192) -> now, us:  333 x 11008 x 4096 Q8_0 111 -> 50 (3 blocks, 4 shares);
+// 512 x 4096 x 4096 Q4_K 37.9 -> 29.2 (4, 4);  512 x 4096 x 6144 42.5 -> 37.4 (4, 3);  200 x 4096 x 4096 Q4_0 36.4 -> 21.0 (2, 4);
+// 256 x 8192 x 8192 68.6 -> 52.2 (2, 2);  400 x 2048 x 2048 21.5 -> 15.9 (2, 4);  1500 x 4096 x 4096 Q8_0 63.0 -> 55.3 (3, 1);
+// unchanged: 512 x 14336 x 4096 (4, 4), 512 x 4096 x 14336 and x 28672 (4, 1), 2048 x 4096 x 11008 (4, 1).
+void tc_shape_plan(const cutb_qmatmul_desc &d, uint32_t sm_count, bool split, uint32_t *mb_out, uint32_t *ksplit_out) {
+  static const float stage[TC_MAX_MB] = {0.58f, 0.56f, 0.65f, 0.71f}, fixed[TC_MAX_MB] = {6.f, 8.f, 9.f, 11.f};
   const uint32_t mblocks = (d.M + TC_BT - 1) / TC_BT, ctiles = (d.N + TC_BW - 1) / TC_BW;
-  uint32_t mb = mblocks < TC_MAX_MB ? mblocks : TC_MAX_MB, ksplit = 1;
-  const uint32_t ctas = ctiles * ((mblocks + mb - 1) / mb);
-  const uint32_t nk_all = d.K / TC_BK;  // (such CTAs run 64-k stages)
-  // (K = 4096 measured no better split than not: 512 x 4096 x 4096 35.3 against 36.2 us, 6144 rows 51 against 38)
-  if (mb == TC_MAX_MB && d.K >= 8192 && ctas * 2 <= sm_count) {
-    uint32_t want = sm_count / ctas;
-    if (want > 8) want = 8;
-    const uint32_t per = (nk_all + want - 1) / want;
-    ksplit = (nk_all + per - 1) / per;  // no empty share
-  } else {
-    while (mb > 1 && ctiles * ((mblocks + mb - 1) / mb) * 2 <= sm_count) mb = (mb + 1) / 2;
+  float best = 1e30f;
+  for (uint32_t mb = mblocks < TC_MAX_MB ? mblocks : TC_MAX_MB; mb >= 1; --mb) {
+    const uint32_t ksub = tc_ksub(mb), nk = d.K / (TC_BK * ksub);
+    for (uint32_t want = 1; want <= (split ? 8u : 1u) && want * 4 <= nk + 3; ++want) {
+      const uint32_t per = (nk + want - 1) / want, ks = (nk + per - 1) / per;  // no empty share
+      const uint64_t ctas = (uint64_t)ctiles * ((mblocks + mb - 1) / mb) * ks;
+      const float waves = (float)((ctas + sm_count - 1) / sm_count);
+      float t = waves * (fixed[mb - 1] + (float)(per * ksub) * stage[mb - 1]);
+      if (ks > 1) t += 2.f + (float)ks * (float)d.M * (float)d.N * (4.f / 6.6e6f);
+      if (t < best) best = t, *mb_out = mb, *ksplit_out = ks;
+    }
   }
-  *mb_out = mb;
-  *ksplit_out = ksplit;
 }
 uint64_t tc_cast_bytes(const cutb_qmatmul_desc &d) {
   return d.a_dtype == CUTB_F32 ? (((uint64_t)d.M * d.K * sizeof(__half) + 15) & ~(uint64_t)15) : 0;
@@ -427,7 +458,7 @@ uint64_t qgemm_tc_workspace(const cutb_qmatmul_desc &d) {
   DeviceInfo di;
   const uint32_t sms = get_device_info(&di) == CUTB_OK ? (uint32_t)di.sm_count : 148u;
   uint32_t mb, ksplit;
-  tc_shape_plan(d, sms, &mb, &ksplit);
+  tc_shape_plan(d, sms, true, &mb, &ksplit);
   return tc_cast_bytes(d) + (ksplit > 1 ? (uint64_t)ksplit * d.M * d.N * sizeof(float) : 0);
 }
 
@@ -453,32 +484,25 @@ int qgemm_tc_launch(const cutb_qmatmul_desc &d, cudaStream_t stream) {
   p.ldb = d.ldb;
   p.lds = d.lds;
   p.blocksK = (d.K + 31) / 32;
-  tc_shape_plan(d, (uint32_t)di.sm_count, &p.mb, &p.ksplit);
+  tc_shape_plan(d, (uint32_t)di.sm_count, true, &p.mb, &p.ksplit);
   const uint64_t cast_bytes = tc_cast_bytes(d), partial_bytes = p.ksplit > 1 ? (uint64_t)p.ksplit * d.M * d.N * sizeof(float) : 0;
   p.partial = nullptr;
   if (p.ksplit > 1) {
-    // without room for the partial sums: the tokens-per-CTA rule (a K split of one never asks for any)
+    // without room for the partial sums: the best plan that leaves K whole (it asks for none)
     if (!d.workspace || d.workspace_bytes < cast_bytes + partial_bytes || reinterpret_cast<uintptr_t>(d.workspace) % 16 != 0) {
-      const uint32_t mblocks = (d.M + TC_BT - 1) / TC_BT, ctiles = (d.N + TC_BW - 1) / TC_BW;
-      p.ksplit = 1;
-      while (p.mb > 1 && ctiles * ((mblocks + p.mb - 1) / p.mb) * 2 <= (uint32_t)di.sm_count) p.mb = (p.mb + 1) / 2;
+      tc_shape_plan(d, (uint32_t)di.sm_count, false, &p.mb, &p.ksplit);
     } else {
       p.partial = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(d.workspace) + cast_bytes);
     }
   }
-  // weight slots: two (one per converter group) when the activation stages need the room; up to 256 tokens per
-  // CTA a third one loosens the hand-off chain converter -> issuer -> tensor core -> converter (512 x 4096 x 4096
-  // 39.1 -> 36.5 us, 512 x 14336 x 4096 121.4 -> 112.4 us; no change with four); the rest of shared memory holds
-  // activation stages in flight
-  p.nb = p.mb <= 2 ? 3 : 2;
-  p.groups = TC_MAX_GROUPS;
-  if (p.groups > p.nb) p.groups = p.nb;
+  // Weight slots, one per converter group: three where a stage's weights set the pace and shared memory has room (128 tokens:
+  // stages of 128 k; 384 tokens: 333 x 11008 x 4096 56 -> 50 us), two at 256 and 512 tokens (a third one costs an activation
+  // stage there: 512 x 4096 x 14336 62 -> 70 us); the rest of shared memory holds activation stages in flight.
+  p.nb = p.mb == 1 || p.mb == 3 ? 3 : 2;
+  p.groups = d.layout == CUTB_LAYOUT_KN_PLANES ? 2 : p.nb;
   p.issuers = 2;
   if (p.issuers > (p.mb + 1) / 2) p.issuers = (p.mb + 1) / 2;
-  // Up to 256 tokens the tensor work of a 64-k stage (256-512 cycles) is less than what the issuer
-  // thread spends on the stage's two barrier waits and four to eight MMA issues: stages of 128 k
-  // halve the waits per k, and shared memory has room for them there.
-  p.ksub = p.mb <= 2 ? 2u : 1u;
+  p.ksub = tc_ksub(p.mb);
   p.sa = 0;
   for (uint32_t sa = 6; sa >= 2; --sa)
     if (tc_smem_bytes(p.mb, sa, p.nb, p.ksub) <= di.smem_optin) {
@@ -521,7 +545,13 @@ int qgemm_tc_launch(const cutb_qmatmul_desc &d, cudaStream_t stream) {
   }
   if (rc != CUTB_OK || p.ksplit <= 1) return rc;
   const size_t total = (size_t)d.M * d.N;
-  tc_splitk_reduce_kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(p);
+  const bool quads = d.N % 4 == 0 && (p.glu || (reinterpret_cast<uintptr_t>(d.C) % 16 == 0 && d.ldc % 4 == 0)) &&
+                     (d.fusion_type != CUTB_FUSION_BINARY || (reinterpret_cast<uintptr_t>(d.D) % 16 == 0 && d.ldd % 4 == 0));
+  const int v = quads ? 4 : (p.glu ? 2 : 1);
+  const unsigned blocks = (unsigned)((total / v + 255) / 256);
+  if (v == 4) tc_splitk_reduce_kernel<4><<<blocks, 256, 0, stream>>>(p);
+  else if (v == 2) tc_splitk_reduce_kernel<2><<<blocks, 256, 0, stream>>>(p);
+  else tc_splitk_reduce_kernel<1><<<blocks, 256, 0, stream>>>(p);
   CUTB_CUDA_TRY(cudaGetLastError());
   return CUTB_OK;
 }

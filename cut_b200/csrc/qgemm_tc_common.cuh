@@ -16,9 +16,7 @@ constexpr int TC_BW = 128;            // weight rows per CTA (MMA M, one per TME
 constexpr int TC_BT = 128;            // tokens per activation tile (rows of one TMA box)
 constexpr int TC_BK = 64;             // k per stage: one 128-byte swizzled row of fp16
 constexpr int TC_MAX_MB = 4;          // token blocks per CTA (4 x 128 columns = all of tensor memory)
-constexpr int TC_MAX_GROUPS = 2;      // converter groups of 128 threads; group g dequantises K stages g, g + G, ...
 constexpr int TC_CTRL_THREADS = 128;  // warps 0-3: issuer, copy producer, second issuer, spare
-constexpr int TC_MAX_THREADS = TC_CTRL_THREADS + 128 * TC_MAX_GROUPS;
 constexpr uint32_t TC_TILE_BYTES = 128 * TC_BK * 2;  // 16 KB: one token block, or the weight tile, per stage
 constexpr uint32_t TC_TILE_DESC = TC_TILE_BYTES >> 4;  // the same in descriptor address units
 
@@ -52,6 +50,10 @@ struct TcParams {
 // and the same with per-block mins behind the scales (the runner's affine re-encode of Q4_K).
 constexpr int TC_PLANE_Q8 = 100, TC_PLANE_Q4 = 101, TC_PLANE_Q4A = 102;
 __host__ __device__ constexpr bool tc_is_plane(int fmt) { return fmt >= TC_PLANE_Q8; }
+// Converter groups of 128 threads; group g dequantises K stages g, g + G, ...  More than three groups slow one another down
+// (333 x 11008 x 4096 Q8_0: 50 us with three, 61 with four).  The plane formats' converters need the register file of two.
+__host__ __device__ constexpr int tc_max_groups(int fmt) { return tc_is_plane(fmt) ? 2 : 3; }
+__host__ __device__ constexpr int tc_max_threads(int fmt) { return TC_CTRL_THREADS + 128 * tc_max_groups(fmt); }
 
 // Byte offset of 16-byte chunk `c` (0..7) of row `r` inside a swizzled tile.
 __device__ __forceinline__ uint32_t sw128(uint32_t r, uint32_t c) { return r * 128u + ((c ^ (r & 7u)) << 4); }

@@ -1,0 +1,49 @@
+"""GPU parity of the matmul's plans at their edges: shares of K, token blocks, ragged columns, scratch that holds no partial sums.
+
+Tolerance: operands are rounded to fp16 (half an ulp, 2^-11, each: at most 2^-10 of a product), sums are fp32: 1e-3 rel-L2 as in
+test_gpu_qmatmul.py; Q4_K rounds its scale and its minimum as well: 2.5e-3."""
+import numpy as np
+import pytest
+
+from cut_b200 import _lib as L
+from cut_b200 import ops, synth
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _tol(fmt):
+    return 2.5e-3 if fmt == synth.Q4_K else 1e-3
+
+
+def _run(fmt, A, W, N, workspace=None, **kw):
+    import torch
+
+    from gpu_util import dev
+
+    D = dev(kw.pop("D")) if "D" in kw else None
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    a, w = dev(A), dev(W)
+    d, out, keep = ops.make_desc(a, w, fmt, N, D=D, status=status, **kw)
+    need = ops.workspace_bytes(d) if workspace is None else workspace
+    ws = torch.full((max(need, 16),), 0xFF, dtype=torch.uint8, device="cuda")  # (NaNs: nothing may be read before it is written)
+    d.workspace, d.workspace_bytes = ws.data_ptr(), need
+    ops.launch(d)
+    ops.launch(d)
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    return out.cpu().numpy()
+
+
+@pytest.mark.parametrize("fmt", [synth.Q8_0, synth.Q4_0, synth.Q4_K])
+@pytest.mark.parametrize("M,K,N,act,op", [(129, 2048, 390, np.float16, None), (333, 2816, 256, np.float32, 0), (512, 2048, 130, np.float16, 2),
+                                          (257, 4096, 384, np.float32, None), (520, 768, 129, np.float16, 0)])
+def test_shares_of_k(fmt, M, K, N, act, op):
+    from gpu_util import rel_l2
+
+    W, A = synth.make_weights(fmt, N, K, M), synth.make_activations(M, K, 7, act)
+    fuse = {} if op is None else {"fusion_type": L.FUSION_BINARY, "fusion_op": op, "D": np.random.default_rng(3).standard_normal((M, N)).astype(np.float32)}
+    ref = O.qmatmul_blocks(fmt, A.astype(np.float32), W, M, K, N, **fuse)
+    cast = (M * K * 2 + 15) // 16 * 16 if act == np.float32 else 0
+    for workspace in (None, cast):  # with and without room for partial sums
+        assert rel_l2(_run(fmt, A, W, N, workspace, **fuse), ref) <= _tol(fmt), workspace
