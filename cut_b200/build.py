@@ -21,7 +21,7 @@ QUANT_SOURCES = ["cabi.cu", "qgemv_blocks.cu", "qmatmul_generic.cu", "dequant.cu
 SOURCES = QUANT_SOURCES + LAYER_SOURCES
 LAYERS_LIB = os.path.join(HERE, "libcutb_layers.so")
 HEADERS = ["common.cuh", "kernels.h", "tcgen05.cuh", "qgemm_tc_common.cuh", "dense_common.cuh", "norm_stage.cuh",
-           "attn_common.cuh", "moe_common.cuh",
+           "attn_common.cuh", "prefill_attention.cuh", "moe_common.cuh",
            os.path.join("..", "..", "include", "cutb.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC,-fvisibility=hidden"]

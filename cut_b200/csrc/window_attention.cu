@@ -3,11 +3,12 @@
 // which serve the llama path (whole-context caches, half-split rotation of the whole head).
 //
 //  * window_kv_write_kernel: a batch of tokens into the ring;
-//  * window_attention_tc_kernel: prefill with a bf16 cache.  A block of four warps owns 64 consecutive tokens of one query
-//    head; only the key tiles that some token of the block sees are visited, and a warp skips those its own 16 tokens do not
-//    see.  K / V tiles of 64 ring rows stream through a two-deep cp.async ring (a tile never wraps: ring_rows is a multiple of
-//    64 and tiles are aligned), products are m16n8k16 warp MMAs with fp32 accumulators, the softmax runs online.  The weights
-//    enter the value product as the sum of two bf16 terms, so they keep 16 significant bits;
+//  * prefill with a bf16 cache and heads of up to 128: prefill_attention_kernel (prefill_attention.cuh);
+//  * window_attention_tc_kernel: the same for heads of up to 64 that see few keys.  A block of four warps owns 64 consecutive
+//    tokens of one query head; only the key tiles that some token of the block sees are visited, and a warp skips those its own
+//    16 tokens do not see.  K / V tiles of 64 ring rows stream through a two-deep cp.async ring (a tile never wraps: ring_rows is
+//    a multiple of 64 and tiles are aligned), products are m16n8k16 warp MMAs with fp32 accumulators, the softmax runs online.
+//    The weights enter the value product as the sum of two bf16 terms, so they keep 16 significant bits;
 //  * window_attention_simt_kernel: the same in fp32 arithmetic, one warp per (token, head);
 //  * window_attention_decode_kernel: one token.  The slices of the window are the blocks of a cluster; every block rotates
 //    its query heads itself, the first slice takes the new token's key and value from registers of this step and stores them
@@ -19,6 +20,7 @@
 #include "common.cuh"
 #include "dense_common.cuh"
 #include "kernels.h"
+#include "prefill_attention.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -621,6 +623,22 @@ template <int DK, int DV> int wt_launch(const cutb_window_attn_desc &d, cudaStre
   return CUTB_OK;
 }
 
+template <int KP, int VP> int wp_launch(const cutb_window_attn_desc &d, cudaStream_t stream) {
+  DeviceInfo di;
+  if (int rc = get_device_info(&di)) return rc;
+  PaParams p{};
+  p.q = d.q, p.ldq = d.ldqkv, p.n_tokens = d.n_tokens, p.n_heads = d.n_heads, p.rep = d.n_heads / d.n_kv_heads, p.q_head = d.dim;
+  p.rot = d.rot_dims, p.pairing = d.rot_pairing != 0, p.cos_t = d.cos_table, p.sin_t = d.sin_table;
+  p.pos_ptr = d.pos_ptr, p.pos = d.pos, p.max_pos = d.max_pos, p.window = d.window, p.ring_rows = d.ring_rows;
+  p.step = pa_step(d.n_tokens, d.n_heads, (uint32_t)di.sm_count), p.ksteps = (d.dim + 15) / 16, p.key_planes = KP;
+  p.zero_sink = d.sink != 0, p.out = d.out, p.ldo = d.ldo, p.vdim = d.vdim, p.out_bf16 = d.out_dtype == CUTB_BF16, p.status = d.status;
+  pa_set_scale(&p, d.scale);
+  CUtensorMap mk, mv;
+  if (int rc = pa_map(&mk, true, d.k_cache, d.k_head, d.n_kv_heads, d.k_head, d.ring_rows, (uint64_t)d.n_kv_heads * d.k_head)) return rc;
+  if (int rc = pa_map(&mv, true, d.v_cache, d.v_head, d.n_kv_heads, d.v_head, d.ring_rows, (uint64_t)d.n_kv_heads * d.v_head)) return rc;
+  return pa_launch_inst<PA_WINDOW, KP, VP>(mk, mk, mv, p, stream);
+}
+
 template <typename KV, int RG> int wd_launch(const cutb_window_attn_desc &d, cudaStream_t stream) {
   const uint32_t rep = d.n_heads / d.n_kv_heads, keys = d.window < d.max_pos ? d.window : d.max_pos;
   uint32_t S = 1;
@@ -663,8 +681,12 @@ int window_kv_write_launch(const cutb_window_attn_desc &d, cudaStream_t stream) 
 
 int window_attention_launch(const cutb_window_attn_desc &d, cudaStream_t stream) {
   if (d.kv_dtype == CUTB_BF16 && d.dim <= 128 && d.vdim <= 128) {
-    if (d.dim <= 64) return d.vdim <= 64 ? wt_launch<64, 64>(d, stream) : wt_launch<64, 128>(d, stream);
-    return d.vdim <= 64 ? wt_launch<128, 64>(d, stream) : wt_launch<128, 128>(d, stream);
+    // Heads of 64 that see few keys: the smaller blocks start sooner (us, warp MMAs / tcgen05, 16 heads of 64: 100 tokens 8.3 / 9.2,
+    // 1000 in a window of 300 18.2 / 19.9, 600 in one of 2048 23.4 / 18.0, 1500 in one of 1000 49.5 / 43.5).  Heads of 96 and 128
+    // gain at every length (32 heads of 128: 16 tokens 15.3 / 11.3, 128 18.5 / 12.3, 512 36.7 / 20.4, 1501 154 / 69).
+    if (d.dim <= 64 && d.vdim <= 64) return d.n_tokens < 256 || d.window < 512 ? wt_launch<64, 64>(d, stream) : wp_launch<1, 1>(d, stream);
+    if (d.dim <= 64) return wp_launch<1, 2>(d, stream);
+    return d.vdim <= 64 ? wp_launch<2, 1>(d, stream) : wp_launch<2, 2>(d, stream);
   }
   const dim3 grid((d.n_tokens + WS_WARPS - 1) / WS_WARPS, d.n_heads);
   if (d.kv_dtype == CUTB_BF16) CUTB_CUDA_TRY(launch_pdl(window_attention_simt_kernel<__nv_bfloat16>, grid, dim3(32 * WS_WARPS), 0, stream, d));

@@ -531,6 +531,7 @@ class LayerListDecoder:
             (cache,) = seq.kv[i if m.kv_from is None else m.kv_from]
             exp = self._scratch("expand", n, pad(d["expand"].N, 8), torch.bfloat16)
             a = self._latent_desc(i, seq, T, q=q, k_exp=exp, v_exp=exp[:, m.heads * m.dim:], out=mid)
+            a.pos_ptr = None  # the position as the host knows it: the number of expanded rows that there are follows from it
             if L.lib().cutb_latent_prefill_supported(C.byref(a)):
                 self._dense(d["expand"], n, cache[:n], exp)
                 self._call("cutb_latent_prefill", a)

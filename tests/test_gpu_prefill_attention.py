@@ -1,0 +1,127 @@
+"""Prompt attention on the tensor cores at the edges of its tiles (128 tokens, 128 keys, boxes of 64 rows), against 64 bits.
+
+Without rotation the kernel's queries are the test's (rounded beforehand): what is left are fp32 scores and sums, exponentials of a
+few ulp and bf16 weights in two terms (2^-17) or fp16 weights (2^-11): rel-L2 1e-4 and 1e-3.  With rotation a query element may
+round the other way, one ulp (2^-8 in bf16) of a part of a score: 4e-3."""
+import numpy as np
+import pytest
+
+from cut_b200 import _lib as L
+from cut_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+
+def _rel(got, ref):
+    return float((got.double() - ref).norm() / ref.norm())
+
+
+def _reference(q, k, v, scale, pos, window, sink):
+    """q [T, H, d]; k, v [positions, G, .] in 64 bits; sink: a logit per head, or None."""
+    import torch
+
+    out = torch.empty((q.shape[0], q.shape[1], v.shape[2]), dtype=torch.float64, device=q.device)
+    keys, rep = torch.arange(k.shape[0], device=q.device), q.shape[1] // k.shape[1]
+    hidden = (keys[None, :] > pos[:, None]) | (pos[:, None] - keys[None, :] >= window)
+    for h in range(q.shape[1]):
+        s = (q[:, h] @ k[:, h // rep].T * scale).masked_fill(hidden, float("-inf"))
+        if sink is not None:
+            s = torch.cat([s, sink[h].expand(len(s), 1)], dim=1)
+        out[:, h] = s.softmax(-1)[:, : k.shape[0]] @ v[:, h // rep]
+    return out
+
+
+def _turned(x, cos, sin, neighbours):
+    import torch
+
+    n = cos.shape[1]
+    a, b = (x[..., 0: 2 * n: 2], x[..., 1: 2 * n: 2]) if neighbours else (x[..., :n], x[..., n: 2 * n])
+    c, s = cos[:, None], sin[:, None]
+    y = (a * c - b * s, b * c + a * s)
+    y = torch.stack(y, -1).flatten(-2) if neighbours else torch.cat(y, -1)
+    return torch.cat([y, x[..., 2 * n:]], -1)
+
+
+@pytest.mark.parametrize("T,pos,window,dim,vdim,rot,near,scale,sink", [
+    (16, 0, 1000, 128, 128, 0, True, 0.1, True), (127, 0, 64, 96, 128, 0, True, 0.1, False), (129, 63, 130, 128, 64, 128, True, 0.1, True),
+    (256, 1, 128, 128, 128, 128, False, -0.1, False), (257, 500, 333, 72, 40, 24, False, 0.1, True), (300, 0, 1, 128, 128, 0, True, 0.0, False),
+    (384, 200, 512, 64, 64, 64, True, 0.1, True), (2100, 0, 600, 128, 128, 32, True, 0.1, True)])
+def test_window(T, pos, window, dim, vdim, rot, near, scale, sink):
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(T + dim)
+    rand = lambda *s: torch.randn(s, device="cuda", generator=g)
+    H, G, end = 4, 2, pos + T
+    kh, vh = (dim + 7) // 8 * 8, (vdim + 7) // 8 * 8
+    ring = (min(window, end) + T + 63) // 64 * 64
+    k, v = rand(end, G, dim).bfloat16(), rand(end, G, vdim).bfloat16()
+    kc, vc = torch.full((ring, G, kh), float("nan"), device="cuda").bfloat16(), torch.full((ring, G, vh), float("nan"), device="cuda").bfloat16()
+    kept = torch.arange(max(0, pos + 1 - window), end, device="cuda")  # (everything else is NaN)
+    kc[kept % ring], vc[kept % ring] = 0, 0
+    kc[kept % ring, :, :dim], vc[kept % ring, :, :vdim] = k[kept], v[kept]
+    qkv = torch.empty((T, (H + G) * dim + G * vdim), device="cuda")
+    q = rand(T, H, dim).bfloat16().float()
+    qkv[:, : H * dim] = q.reshape(T, -1)
+    cos, sin = (torch.cos(rand(end, rot // 2)), torch.sin(rand(end, rot // 2))) if rot else (None, None)
+    at = torch.arange(pos, end, device="cuda")
+    if rot:
+        q = _turned(q, cos[at], sin[at], near).bfloat16()
+    out, status = torch.full((T, H * vdim), float("nan"), device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    d = ops.window_desc(qkv, H, G, dim, vdim, kc.view(ring, -1), vc.view(ring, -1), window=window, scale=scale, out=out, cos_t=cos, sin_t=sin, rot_dims=rot,
+                        pairing=L.ROT_NEIGHBOURS if near else L.ROT_HALVES, max_pos=end, sink=sink, pos=pos, status=status)
+    ops.window_attention(d)
+    zero = torch.zeros(H, dtype=torch.float64, device="cuda")
+    ref = _reference(q.double(), k.double(), v.double(), scale, at, window, zero if sink else None)
+    assert int(status.item()) == 0
+    assert _rel(out.view(T, H, vdim), ref) <= (4e-3 if rot else 1e-4)
+
+
+@pytest.mark.parametrize("T,pos,dim,rot,vdim,scale", [(40, 0, 128, 64, 128, 0.1), (128, 5, 64, 32, 64, 0.1), (257, 127, 128, 32, 128, -0.1),
+                                                     (300, 0, 24, 8, 40, 0.1), (1100, 64, 64, 64, 128, 0.1), (130, 0, 128, 0, 72, 0.1)])
+@pytest.mark.parametrize("on_device", [False, True])
+def test_latent(T, pos, dim, rot, vdim, scale, on_device):
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(T + dim + rot)
+    rand = lambda *s: torch.randn(s, device="cuda", generator=g)
+    H, end, rank = 3, pos + T, 64
+    k, v, r = rand(end, H, dim).bfloat16(), rand(end, H, vdim).bfloat16(), rand(end, max(rot, 1)).bfloat16()[:, :rot]
+    cache = torch.zeros((end + 50, rank + max(rot, 8)), device="cuda").bfloat16()
+    cache[:end, rank: rank + rot], cache[end:] = r, float("nan")
+    cos, sin = torch.cos(rand(end + 50, rot // 2)), torch.sin(rand(end + 50, rot // 2))
+    q = rand(T, H, dim + rot).bfloat16().float()
+    out, status = torch.full((T, H * vdim), float("nan"), device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    sink, where = rand(H), torch.tensor([pos], dtype=torch.int32, device="cuda")
+    d = ops.latent_desc(cache, H, dim, rot, vdim, rank, scale=scale, eps=1e-6, max_pos=end + 50, n_tokens=T, cos_t=cos, sin_t=sin, sink=sink,
+                        pos=0 if on_device else pos, pos_ptr=where.data_ptr() if on_device else None, q=q.view(T, -1), k_exp=k.view(end, -1),
+                        v_exp=v.view(end, -1), out=out, status=status)
+    import ctypes
+
+    L.check(L.lib().cutb_latent_prefill(ctypes.byref(d), torch.cuda.current_stream().cuda_stream))
+    at = torch.arange(pos, end, device="cuda")
+    qt = torch.cat([q[..., :dim], _turned(q[..., dim:], cos[at], sin[at], True)], -1).bfloat16() if rot else q
+    kk = torch.cat([k, r[:, None].expand(-1, H, -1)], -1)
+    ref = _reference(qt.double(), kk.double(), v.double(), scale, at, 1 << 30, sink.double())
+    assert int(status.item()) == 0
+    assert _rel(out.view(T, H, vdim), ref) <= (4e-3 if rot else 1e-4)
+
+
+@pytest.mark.parametrize("T,hd,order", [(16, 64, "up"), (129, 128, "up"), (256, 128, "down"), (300, 64, "mixed"), (1030, 128, "up")])
+def test_llama(T, hd, order):
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(T + hd)
+    rand = lambda *s: torch.randn(s, device="cuda", generator=g)
+    H, G, rows = 4, 2, T + 37
+    at = torch.arange(20, 20 + T, device="cuda")
+    at = at.flip(0) if order == "down" else at[torch.randperm(T, device="cuda", generator=g)] if order == "mixed" else at
+    kc, vc = rand(rows, G, hd).half(), rand(rows, G, hd).half()
+    kc[20 + T:], vc[20 + T:] = float("nan"), float("nan")
+    cos, sin = torch.cos(rand(rows, hd // 2)), torch.sin(rand(rows, hd // 2))
+    q = rand(T, H, hd)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = ops.batched_attention(q.view(T, -1), kc.view(rows, -1), vc.view(rows, -1), at.int(), cos, sin, H, G, hd, status=status)
+    seen = slice(0, 20 + T)
+    ref = _reference(_turned(q, cos[at], sin[at], False).half().double(), kc[seen].double(), vc[seen].double(), hd ** -0.5, at, 1 << 30, None)
+    assert int(status.item()) == 0
+    assert _rel(out.view(T, H, hd), ref) <= 1e-3
