@@ -72,7 +72,7 @@ enum { CUTB_FUSION_NONE = 0, CUTB_FUSION_UNARY = 1, CUTB_FUSION_BINARY = 2 };
 
 /* Kernel variants of cutb_qmatmul (variant = -1 lets the library choose). */
 enum {
-  CUTB_VARIANT_AUTO = -1,
+  CUTB_VARIANT_AUTO = -1, /* (9 to 32 rows over GGUF blocks may run as fp16 warp MMAs under either name below) */
   CUTB_VARIANT_GENERIC = 0, /* any shape, SIMT, exact fp32 dequant + FMA */
   CUTB_VARIANT_GEMV_MMA = 1, /* decode: bulk-copy ring + int8 warp MMA, M <= 16 (fp16 A) / 8 (fp32 A); when forced, up to
                                 four such row groups one after the other (M <= 64 / 32): faster than the GEMM on narrow

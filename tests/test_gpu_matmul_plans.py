@@ -47,3 +47,21 @@ def test_shares_of_k(fmt, M, K, N, act, op):
     cast = (M * K * 2 + 15) // 16 * 16 if act == np.float32 else 0
     for workspace in (None, cast):  # with and without room for partial sums
         assert rel_l2(_run(fmt, A, W, N, workspace, **fuse), ref) <= _tol(fmt), workspace
+
+
+@pytest.mark.parametrize("fmt", [synth.Q8_0, synth.Q4_0, synth.Q4_K])
+@pytest.mark.parametrize("M,K,N,act,op", [(9, 256, 1, np.float32, None), (16, 4096, 8600, np.float16, 0), (17, 8192, 2178, np.float16, None),
+                                          (32, 1024, 20000, np.float16, 2), (13, 512, 130, np.float16, None), (24, 4096, 4098, np.float32, 0)])
+def test_rows_as_fp16_mmas(fmt, M, K, N, act, op):
+    """9 to 32 rows: whole tiles and shares of tiles, ragged columns, the general path where the scratch is too small.  Up to 16 rows
+    weights are exact (fp32 sums of 24-bit products): 1e-5 with fp16 activations."""
+    from gpu_util import rel_l2
+
+    W, A = synth.make_weights(fmt, N, K, M), synth.make_activations(M, K, 7, act)
+    fuse = {} if op is None else {"fusion_type": L.FUSION_BINARY, "fusion_op": op, "D": np.random.default_rng(3).standard_normal((M, N)).astype(np.float32)}
+    ref = O.qmatmul_blocks(fmt, A.astype(np.float32), W, M, K, N, **fuse)
+    exact = act == np.float16 and M <= 16 and fmt != synth.Q4_K
+    got = _run(fmt, A, W, N, None, **fuse)
+    assert rel_l2(got, ref) <= (1e-5 if exact else _tol(fmt))
+    if act == np.float16:
+        assert rel_l2(_run(fmt, A, W, N, 16, **fuse) if M > 16 else got, ref) <= _tol(fmt)
