@@ -1,7 +1,9 @@
 // Prefill GEMM over dense bf16 weights, C[M, N] = unary(A[M, K] W[N, K]^T + bias), and its 32-bit companion.
 //
-// dense_gemm_tc_kernel: persistent, warp-specialised tcgen05 kernel.  A CTA tile is 128 tokens x BN weight rows (64 / 128 /
-// 256); tokens are the MMA's M operand (one per tensor-memory lane), weight rows its N operand.
+// dense_gemm_tc_kernel: persistent, warp-specialised tcgen05 kernel.  A CTA tile is 128 tokens x bn weight rows (up to 256);
+// tokens are the MMA's M operand (one per tensor-memory lane), weight rows its N operand.  PAIR: two CTAs of a cluster share a
+// tile of 256 tokens x bn rows (cta_group::2): each keeps its own 128 tokens' accumulators and copies its own tokens and half
+// of the weight rows, a third fewer bytes per product; the first CTA's MMA warp issues for both.
 //   warp 0      one lane copies the 64-k stages of both operands by TMA (128-byte swizzle; rows and k past the matrices read as
 //               zero) into a ring that fills shared memory;
 //   warp 1      allocates tensor memory (two accumulators of BN columns); one lane issues four K = 16 MMAs per stage and
@@ -28,11 +30,9 @@
 namespace cutb {
 namespace {
 
-constexpr int DG_BM = 128, DG_BK = 64, DG_THREADS = 192;
-constexpr uint32_t DG_A_BYTES = DG_BM * DG_BK * 2;
-__host__ __device__ constexpr int dg_stages(int bn) { return bn == 256 ? 4 : (bn == 128 ? 6 : 8); }
-__host__ __device__ constexpr uint32_t dg_stage_bytes(int bn) { return DG_A_BYTES + (uint32_t)bn * DG_BK * 2; }
-constexpr uint32_t dg_smem(int bn) { return 1024 + dg_stages(bn) * dg_stage_bytes(bn); }
+constexpr int DG_BM = 128, DG_BK = 64, DG_THREADS = 192, DG_MAX_STAGES = 8;
+constexpr uint32_t DG_A_BYTES = DG_BM * DG_BK * 2, DG_RING = 216 * 1024;
+__host__ __device__ constexpr uint32_t dg_stage_bytes(uint32_t rows) { return DG_A_BYTES + (rows + 7) / 8 * 8 * DG_BK * 2; }  // rows: those a CTA copies
 
 struct DgParams {
   const float *bias;
@@ -41,6 +41,7 @@ struct DgParams {
   int *status;
   uint32_t M, K, N, ldc;
   uint32_t tiles_m, tiles_n, ksplit, nk, nk_per, a_box_rows;
+  uint32_t bn, stages;  // weight rows of a tile (a multiple of 16, at most 256; pairs: of 32), 64-k stages in shared memory
   int c_bf16, unary;
   const uint32_t *offsets;  // grouped
   uint32_t experts;
@@ -52,14 +53,41 @@ struct DgJob {
   uint32_t m0, m_end, n0, w0, k0, nk, z;  // rows m0 .. m_end - 1 are stored; w0 = row of the stacked weight
 };
 
-template <int BN, bool GROUPED>
+// cta_group::2 forms: both CTAs' shared memory at the same offsets; completion is signalled to both
+__device__ __forceinline__ void umma_pair(uint32_t tmem_d, uint32_t adesc_lo, uint32_t bdesc_lo, uint32_t desc_hi, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+      "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %4, p;\n\t}" ::"r"(tmem_d),
+      "r"(adesc_lo), "r"(bdesc_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3)
+               : "memory");
+}
+// a tile into this CTA's shared memory, counted on the barrier of the pair's first CTA (`bar`: its cluster address)
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap *map, uint32_t x, uint32_t y, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+               "l"(map), "r"(x), "r"(y), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ uint32_t first_cta(uint32_t addr) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
+  return r;
+}
+
+template <bool GROUPED, bool PAIR>
 __global__ void __launch_bounds__(DG_THREADS, 1) dense_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a,
                                                                       const __grid_constant__ CUtensorMap map_w, const DgParams p) {
-  constexpr int S = dg_stages(BN);
-  constexpr uint32_t STAGE = dg_stage_bytes(BN), COLS = 2 * BN;
+  const uint32_t S = p.stages, BN = p.bn, rows = PAIR ? BN / 2 : BN, STAGE = dg_stage_bytes(rows);
+  constexpr uint32_t COLS = 512, TM = PAIR ? 2 * DG_BM : DG_BM;  // tokens of a tile
+  const uint32_t rank = PAIR ? blockIdx.x & 1u : 0u, first_job = PAIR ? blockIdx.x / 2 : blockIdx.x, workers = PAIR ? gridDim.x / 2 : gridDim.x;
   extern __shared__ __align__(1024) uint8_t dg_raw[];
   uint8_t *ring = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(dg_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ __align__(8) uint64_t bars[2 * S + 4];  // full[S], empty[S], accumulator full[2], accumulator empty[2]
+  __shared__ __align__(8) uint64_t bars[2 * DG_MAX_STAGES + 4];  // full[S], empty[S], accumulator full[2], accumulator empty[2]
   __shared__ uint32_t tmem_slot, abort_flag;
   __shared__ uint32_t offs[GROUPED ? DG_MAX_EXPERTS + 1 : 1], first_tile[GROUPED ? DG_MAX_EXPERTS + 1 : 1];
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -67,20 +95,25 @@ __global__ void __launch_bounds__(DG_THREADS, 1) dense_gemm_tc_kernel(const __gr
   const uint32_t ring_u = smem_u32(ring);
 
   if (tid == 0) {
-    for (int s = 0; s < S; ++s) mbar_init(full_u + s * 8, 1), mbar_init(empty_u + s * 8, 1);
-    for (int a = 0; a < 2; ++a) mbar_init(afull_u + a * 8, 1), mbar_init(aempty_u + a * 8, 4);
+    for (uint32_t s = 0; s < S; ++s) mbar_init(full_u + s * 8, 1), mbar_init(empty_u + s * 8, 1);
+    for (int a = 0; a < 2; ++a) mbar_init(afull_u + a * 8, 1), mbar_init(aempty_u + a * 8, PAIR ? 8 : 4);
     abort_flag = 0;
     fence_mbar_init();
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(COLS) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if constexpr (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(COLS) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(COLS) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   }
   if (GROUPED && warp == 2) {  // row tiles before each expert
     uint32_t before = 0;
     for (uint32_t e0 = 0; e0 < p.experts; e0 += 32) {
       const uint32_t e = e0 + lane, lo = min(p.offsets[min(e, p.experts)], p.M), hi = min(p.offsets[min(e + 1, p.experts)], p.M);
-      const uint32_t tiles = e < p.experts && hi > lo ? (hi - lo + DG_BM - 1) / DG_BM : 0;
+      const uint32_t tiles = e < p.experts && hi > lo ? (hi - lo + TM - 1) / TM : 0;
       uint32_t sum = tiles;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -95,6 +128,10 @@ __global__ void __launch_bounds__(DG_THREADS, 1) dense_gemm_tc_kernel(const __gr
   }
   tc_fence_before();
   __syncthreads();
+  if constexpr (PAIR) {  // the other CTA's barriers are there
+    asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+  }
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
   auto give_up = [&]() {
@@ -112,11 +149,11 @@ __global__ void __launch_bounds__(DG_THREADS, 1) dense_gemm_tc_kernel(const __gr
     if constexpr (GROUPED) {
       while (j >= first_tile[e + 1] * p.tiles_n) ++e;
       const uint32_t rel = j - first_tile[e] * p.tiles_n, tm = first_tile[e + 1] - first_tile[e];
-      b.m0 = offs[e] + rel % tm * DG_BM, b.m_end = offs[e + 1];
+      b.m0 = offs[e] + rel % tm * TM, b.m_end = offs[e + 1];
       b.n0 = rel / tm * BN, b.w0 = e * p.N + b.n0;
       b.z = b.k0 = 0, b.nk = p.nk;
     } else {
-      b.m0 = j % p.tiles_m * DG_BM, b.m_end = p.M;
+      b.m0 = j % p.tiles_m * TM, b.m_end = p.M;
       b.n0 = b.w0 = j / p.tiles_m % p.tiles_n * BN;
       b.z = j / (p.tiles_m * p.tiles_n);
       b.k0 = b.z * p.nk_per;
@@ -130,9 +167,9 @@ __global__ void __launch_bounds__(DG_THREADS, 1) dense_gemm_tc_kernel(const __gr
   if (warp == 0) {
     const bool leader = elect_one();
     uint32_t s = 0, ph = 1;  // (a fresh barrier lets a wait on the phase before its first pass)
-    const uint32_t bytes = p.a_box_rows * DG_BK * 2 + BN * DG_BK * 2;
+    const uint32_t bytes = (p.a_box_rows + rows) * DG_BK * 2 * (PAIR ? 2 : 1);
     bool dead = false;
-    for (uint32_t j = blockIdx.x; j < jobs; j += gridDim.x) {
+    for (uint32_t j = first_job; j < jobs; j += workers) {
       const DgJob b = job_of(j);
       for (uint32_t ks = 0; ks < b.nk; ++ks) {
         if (!dead && !mbar_spin_bounded(empty_u + s * 8, ph)) {
@@ -141,9 +178,16 @@ __global__ void __launch_bounds__(DG_THREADS, 1) dense_gemm_tc_kernel(const __gr
         }
         const uint32_t bar = full_u + s * 8, dst = ring_u + s * STAGE, x = (b.k0 + ks) * DG_BK;
         if (leader && !dead) {
-          mbar_arrive_expect_tx(bar, bytes);
-          tma_load_2d(dst, &map_a, x, b.m0, bar);
-          tma_load_2d(dst + DG_A_BYTES, &map_w, x, b.w0, bar);
+          if constexpr (PAIR) {
+            if (rank == 0) mbar_arrive_expect_tx(bar, bytes);  // both CTAs' copies
+            const uint32_t to = first_cta(bar);
+            tma_load_2d_pair(dst, &map_a, x, b.m0 + rank * DG_BM, to);
+            tma_load_2d_pair(dst + DG_A_BYTES, &map_w, x, b.w0 + rank * rows, to);
+          } else {
+            mbar_arrive_expect_tx(bar, bytes);
+            tma_load_2d(dst, &map_a, x, b.m0, bar);
+            tma_load_2d(dst + DG_A_BYTES, &map_w, x, b.w0, bar);
+          }
         }
         if (++s == S) s = 0, ph ^= 1u;
       }
@@ -158,15 +202,15 @@ __global__ void __launch_bounds__(DG_THREADS, 1) dense_gemm_tc_kernel(const __gr
       }
     }
     __syncwarp();
-  } else if (warp == 1) {
+  } else if (warp == 1 && rank == 0) {
     const bool leader = elect_one();
     const uint64_t proto = umma_desc_sw128(0);
     const uint32_t desc_hi = (uint32_t)(proto >> 32), base = (uint32_t)proto + ((ring_u & 0x3FFFFu) >> 4);
-    const uint32_t idesc = umma_idesc_bf16(DG_BM, BN);
+    const uint32_t idesc = umma_idesc_bf16(TM, BN);
     uint32_t s = 0, ph = 0, turn = 0;
     bool dead = false;
-    for (uint32_t j = blockIdx.x; j < jobs; j += gridDim.x, ++turn) {
-      const uint32_t nk = job_of(j).nk, a = turn & 1, d = tmem + a * BN;
+    for (uint32_t j = first_job; j < jobs; j += workers, ++turn) {
+      const uint32_t nk = job_of(j).nk, a = turn & 1, d = tmem + a * 256;
       if (turn >= 2 && !dead && !mbar_spin_bounded(aempty_u + a * 8, ((turn >> 1) - 1) & 1u)) {
         give_up();
         dead = true;
@@ -180,21 +224,32 @@ __global__ void __launch_bounds__(DG_THREADS, 1) dense_gemm_tc_kernel(const __gr
         tc_fence_after();
         const uint32_t at = base + s * (STAGE >> 4), wt = at + (DG_A_BYTES >> 4);
         if (leader) {
-          umma_f16(d, at, wt, desc_hi, idesc, ks != 0);
-          umma_f16(d, at + 2, wt + 2, desc_hi, idesc, 1);
-          umma_f16(d, at + 4, wt + 4, desc_hi, idesc, 1);
-          umma_f16(d, at + 6, wt + 6, desc_hi, idesc, 1);
-          umma_commit(empty_u + s * 8);
+          if constexpr (PAIR) {
+            umma_pair(d, at, wt, desc_hi, idesc, ks != 0);
+            umma_pair(d, at + 2, wt + 2, desc_hi, idesc, 1);
+            umma_pair(d, at + 4, wt + 4, desc_hi, idesc, 1);
+            umma_pair(d, at + 6, wt + 6, desc_hi, idesc, 1);
+            umma_commit_pair(empty_u + s * 8);
+          } else {
+            umma_f16(d, at, wt, desc_hi, idesc, ks != 0);
+            umma_f16(d, at + 2, wt + 2, desc_hi, idesc, 1);
+            umma_f16(d, at + 4, wt + 4, desc_hi, idesc, 1);
+            umma_f16(d, at + 6, wt + 6, desc_hi, idesc, 1);
+            umma_commit(empty_u + s * 8);
+          }
         }
         if (++s == S) s = 0, ph ^= 1u;
       }
-      if (leader) umma_commit(afull_u + a * 8);
+      if (leader) {
+        if constexpr (PAIR) umma_commit_pair(afull_u + a * 8);
+        else umma_commit(afull_u + a * 8);
+      }
     }
     __syncwarp();
-  } else {
+  } else if (warp >= 2) {
     const uint32_t quarter = warp & 3;  // tensor-memory lanes this warp may read
     uint32_t turn = 0;
-    for (uint32_t j = blockIdx.x; j < jobs; j += gridDim.x, ++turn) {
+    for (uint32_t j = first_job; j < jobs; j += workers, ++turn) {
       const DgJob b = job_of(j);
       const uint32_t a = turn & 1;
       uint32_t ok = 1;
@@ -205,15 +260,15 @@ __global__ void __launch_bounds__(DG_THREADS, 1) dense_gemm_tc_kernel(const __gr
         break;
       }
       tc_fence_after();
-      const uint32_t m = b.m0 + quarter * 32 + lane;
+      const uint32_t m = b.m0 + rank * DG_BM + quarter * 32 + lane, n_end = min(p.N, b.n0 + BN);
 #pragma unroll 1
       for (uint32_t c0 = 0; c0 < BN; c0 += 32) {
         const uint32_t n = b.n0 + c0;
         if (n >= p.N) break;
         uint32_t v[32];
-        tmem_ld32(tmem + ((quarter * 32) << 16) + a * BN + c0, v);
+        tmem_ld32(tmem + ((quarter * 32) << 16) + a * 256 + c0, v);  // (the last piece of an odd number of 16s runs past the tile)
         if (m >= b.m_end) continue;
-        const bool whole = n + 32 <= p.N;
+        const bool whole = n + 32 <= n_end;
         if constexpr (GROUPED) {
           if (p.glu.kind) {  // N is even: outputs 2 i and 2 i + 1 make one
             float y[16];
@@ -229,7 +284,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1) dense_gemm_tc_kernel(const __gr
             } else {
 #pragma unroll
               for (int i = 0; i < 16; ++i)
-                if (n + 2 * i < p.N) store_out(p.C, p.c_bf16, base + i, y[i]);
+                if (n + 2 * i < n_end) store_out(p.C, p.c_bf16, base + i, y[i]);
             }
             continue;
           }
@@ -241,13 +296,13 @@ __global__ void __launch_bounds__(DG_THREADS, 1) dense_gemm_tc_kernel(const __gr
           } else {
 #pragma unroll
             for (int i = 0; i < 32; ++i)
-              if (n + i < p.N) dst[i] = __uint_as_float(v[i]);
+              if (n + i < n_end) dst[i] = __uint_as_float(v[i]);
           }
           continue;
         }
         float x[32];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) x[i] = __uint_as_float(v[i]) + (p.bias && n + i < p.N ? __ldg(p.bias + n + i) : 0.f);
+        for (int i = 0; i < 32; ++i) x[i] = __uint_as_float(v[i]) + (p.bias && n + i < n_end ? __ldg(p.bias + n + i) : 0.f);
         if (p.unary == CUTB_UNARY_RELU_SQUARE) {
 #pragma unroll
           for (int i = 0; i < 32; ++i) x[i] = fmaxf(x[i], 0.f) * fmaxf(x[i], 0.f);
@@ -257,35 +312,48 @@ __global__ void __launch_bounds__(DG_THREADS, 1) dense_gemm_tc_kernel(const __gr
           apply_epilogue_n<32>(x8, none, CUTB_FUSION_UNARY, p.unary);
         }
         const size_t base = (size_t)m * p.ldc + n;
-        if (whole && p.ldc % 8 == 0) {
-          if (p.c_bf16) {
-            uint4 *dst = reinterpret_cast<uint4 *>(reinterpret_cast<__nv_bfloat16 *>(p.C) + base);
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-              dst[i] = make_uint4(pack_bf16(x[8 * i], x[8 * i + 1]), pack_bf16(x[8 * i + 2], x[8 * i + 3]),
-                                  pack_bf16(x[8 * i + 4], x[8 * i + 5]), pack_bf16(x[8 * i + 6], x[8 * i + 7]));
+        for (int h = 0; h < 32; h += 16) {
+          if (n + h + 16 <= n_end && p.ldc % 8 == 0) {
+            if (p.c_bf16) {
+              uint4 *dst = reinterpret_cast<uint4 *>(reinterpret_cast<__nv_bfloat16 *>(p.C) + base + h);
+#pragma unroll
+              for (int i = 0; i < 2; ++i)
+                dst[i] = make_uint4(pack_bf16(x[h + 8 * i], x[h + 8 * i + 1]), pack_bf16(x[h + 8 * i + 2], x[h + 8 * i + 3]),
+                                    pack_bf16(x[h + 8 * i + 4], x[h + 8 * i + 5]), pack_bf16(x[h + 8 * i + 6], x[h + 8 * i + 7]));
+            } else {
+              float4 *dst = reinterpret_cast<float4 *>(reinterpret_cast<float *>(p.C) + base + h);
+#pragma unroll
+              for (int i = 0; i < 4; ++i) dst[i] = make_float4(x[h + 4 * i], x[h + 4 * i + 1], x[h + 4 * i + 2], x[h + 4 * i + 3]);
+            }
           } else {
-            float4 *dst = reinterpret_cast<float4 *>(reinterpret_cast<float *>(p.C) + base);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) dst[i] = make_float4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
+            for (int i = h; i < h + 16; ++i)
+              if (n + i < n_end) store_out(p.C, p.c_bf16, base + i, x[i]);
           }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (n + i < p.N) store_out(p.C, p.c_bf16, base + i, x[i]);
         }
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(aempty_u + a * 8);
+      if (lane == 0) {
+        if constexpr (PAIR)
+          asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(first_cta(aempty_u + a * 8)) : "memory");
+        else
+          mbar_arrive(aempty_u + a * 8);
+      }
     }
   }
 
   tc_fence_before();
   __syncthreads();
+  if constexpr (PAIR) {  // nobody leaves while the other may still signal it or use its shared memory
+    asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+  }
   if (warp == 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(COLS) : "memory");
+    if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(COLS) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(COLS) : "memory");
   }
 }
 
@@ -375,25 +443,62 @@ template <typename TA> __global__ void __launch_bounds__(256) dense_gemm_simt_ke
 }
 
 struct DgPlan {
-  int bn;
-  uint32_t tiles_m, tiles_n, ksplit, nk, nk_per;
+  uint32_t bn, tiles_m, tiles_n, ksplit, nk, nk_per;
+  bool pair;
 };
-// Tile width by the time of its waves; K split when even narrow tiles leave most SMs idle.
+
+// Pairs of CTAs that run at once (0: none, or no device)
+uint32_t dg_pairs() {
+  static uint32_t known[64] = {};  // per device: pairs + 1
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  if (!known[dev]) {
+    const auto kernel = dense_gemm_tc_kernel<false, true>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2), cfg.blockDim = dim3(DG_THREADS), cfg.dynamicSmemBytes = 1024 + DG_RING;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr, cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(1024 + DG_RING)) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 0) {
+      (void)cudaGetLastError();
+      n = 0;
+    }
+    known[dev] = (uint32_t)n + 1;
+  }
+  return known[dev] - 1;
+}
+
+// The tile (width, one CTA's or a pair's) by the time of its waves.  Measured, relative: a 64-k stage of a wave of tiles; what a
+// pair's start costs more.  A pair copies two thirds of the bytes per product, so it wins wherever its 256 tokens are filled; 256
+// rows are slower than their share (six stages of copies in flight instead of seven, and a longer epilogue).  One CTA x 256 rows
+// (all there was) -> now, us: 2048 x 4096 x 14336 181 -> 156 (pairs x 224), x 12288 177 -> 138 (224), x 6144 111 -> 80 (192),
+// x 4096 65 -> 54 (256), 2048 x 14336 x 4096 186 -> 170 (256), 1501 x 4096 x 4096 59 -> 43 (192), 512 x 4096 x 14336 62 -> 50 (224);
+// 2048 x 1024 x 2048 stays (16.9 against 19.0: the pair's start).  `row_tiles`: row tiles of a given height, as they are likely to fall.
+template <class Tiles> void dg_width(uint32_t N, uint32_t nk, uint32_t sms, uint32_t pairs, Tiles row_tiles, DgPlan *pl) {
+  static const struct { uint32_t bn, cost; } one[] = {{256, 140}, {240, 138}, {224, 125}, {208, 122}, {192, 112}, {128, 97}, {64, 90}},
+                                             two[] = {{256, 120}, {224, 100}, {192, 92}, {160, 90}, {128, 86}};
+  constexpr uint64_t PAIR_START = 570;
+  uint64_t best = ~0ull;
+  auto consider = [&](uint32_t bn, uint32_t cost, bool pair) {
+    const uint32_t tm = row_tiles(pair ? 2 * DG_BM : DG_BM), tn = (N + bn - 1) / bn, workers = pair ? pairs : sms;
+    const uint64_t t = (((uint64_t)tm * tn + workers - 1) / workers) * nk * cost + (pair ? PAIR_START : 0);
+    if (t < best) best = t, pl->bn = bn, pl->tiles_m = tm, pl->tiles_n = tn, pl->pair = pair;
+  };
+  for (const auto &k : one) consider(k.bn, k.cost, false);
+  if (pairs)
+    for (const auto &k : two) consider(k.bn, k.cost, true);
+}
+// K split when even narrow tiles leave most SMs idle.
 DgPlan dg_plan(const cutb_dense_desc &d, uint32_t sms) {
   DgPlan b{};
-  uint64_t best = ~0ull;
   const uint32_t tm = (d.M + DG_BM - 1) / DG_BM;
-  // measured time of a wave of tiles, relative: a 64-k stage costs at least what its operands take to arrive
-  const struct { int bn; uint32_t cost; } kinds[] = {{256, 100}, {128, 66}, {64, 62}};
-  for (const auto &kind : kinds) {
-    const int bn = kind.bn;
-    const uint32_t tn = (d.N + bn - 1) / bn;
-    const uint64_t cost = (uint64_t)((tm * tn + sms - 1) / sms) * kind.cost;
-    if (cost < best) best = cost, b.bn = bn, b.tiles_m = tm, b.tiles_n = tn;
-  }
   b.nk = (d.K + DG_BK - 1) / DG_BK;
+  dg_width(d.N, b.nk, sms, d.M > DG_BM ? dg_pairs() : 0, [&](uint32_t rows) { return (d.M + rows - 1) / rows; }, &b);
   if (tm * ((d.N + 127) / 128) * 2 <= sms && b.nk >= 16) {
-    b.bn = 128;
+    b.bn = 128, b.pair = false, b.tiles_m = tm;
     b.tiles_n = (d.N + 127) / 128;
     uint32_t want = sms / (b.tiles_m * b.tiles_n);
     if (want > b.nk / 4) want = b.nk / 4;
@@ -407,18 +512,31 @@ DgPlan dg_plan(const cutb_dense_desc &d, uint32_t sms) {
   return b;
 }
 
-template <int BN, bool GROUPED> int dg_launch(const CUtensorMap &ma, const CUtensorMap &mw, const DgParams &p, uint32_t sms, cudaStream_t stream) {
+template <bool GROUPED, bool PAIR> int dg_launch_inst(const CUtensorMap &ma, const CUtensorMap &mw, const DgParams &p, uint32_t workers, cudaStream_t stream) {
   static bool configured[64] = {};
   int dev = 0;
   CUTB_CUDA_TRY(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64 || !configured[dev]) {
-    CUTB_CUDA_TRY(cudaFuncSetAttribute(dense_gemm_tc_kernel<BN, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dg_smem(BN)));
+    CUTB_CUDA_TRY(cudaFuncSetAttribute(dense_gemm_tc_kernel<GROUPED, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(1024 + DG_RING)));
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
   const uint32_t jobs = p.tiles_m * p.tiles_n * p.ksplit;  // (grouped: an upper bound)
-  dense_gemm_tc_kernel<BN, GROUPED><<<jobs < sms ? jobs : sms, DG_THREADS, dg_smem(BN), stream>>>(ma, mw, p);
-  CUTB_CUDA_TRY(cudaGetLastError());
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((jobs < workers ? jobs : workers) * (PAIR ? 2 : 1));
+  cfg.blockDim = dim3(DG_THREADS);
+  cfg.dynamicSmemBytes = 1024 + DG_RING;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr, cfg.numAttrs = PAIR ? 1 : 0;
+  CUTB_CUDA_TRY(cudaLaunchKernelEx(&cfg, dense_gemm_tc_kernel<GROUPED, PAIR>, ma, mw, p));
   return CUTB_OK;
+}
+template <bool GROUPED> int dg_launch(const CUtensorMap &ma, const CUtensorMap &mw, DgParams p, const DgPlan &pl, uint32_t sms, cudaStream_t stream) {
+  p.bn = pl.bn, p.stages = DG_RING / dg_stage_bytes(pl.pair ? pl.bn / 2 : pl.bn);
+  if (p.stages > DG_MAX_STAGES) p.stages = DG_MAX_STAGES;
+  return pl.pair ? dg_launch_inst<GROUPED, true>(ma, mw, p, dg_pairs(), stream) : dg_launch_inst<GROUPED, false>(ma, mw, p, sms, stream);
 }
 
 }  // namespace
@@ -449,10 +567,8 @@ int dense_gemm_tc_launch(const cutb_dense_desc &d, cudaStream_t stream) {
   p.c_bf16 = d.c_dtype == CUTB_BF16, p.unary = d.unary_op;
   CUtensorMap ma, mw;
   if (int rc = make_tmap_sw128(&ma, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, d.A, d.M, d.K, (uint64_t)d.lda * 2, p.a_box_rows)) return rc;
-  if (int rc = make_tmap_sw128(&mw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, d.W, d.N, d.K, (uint64_t)d.ldw * 2, (uint32_t)pl.bn)) return rc;
-  int rc = pl.bn == 256 ? dg_launch<256, false>(ma, mw, p, (uint32_t)di.sm_count, stream)
-         : pl.bn == 128 ? dg_launch<128, false>(ma, mw, p, (uint32_t)di.sm_count, stream)
-                        : dg_launch<64, false>(ma, mw, p, (uint32_t)di.sm_count, stream);
+  if (int rc = make_tmap_sw128(&mw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, d.W, d.N, d.K, (uint64_t)d.ldw * 2, pl.pair ? pl.bn / 2 : pl.bn)) return rc;
+  const int rc = dg_launch<false>(ma, mw, p, pl, (uint32_t)di.sm_count, stream);
   if (rc != CUTB_OK || pl.ksplit <= 1) return rc;
   dense_splitk_reduce_kernel<<<(unsigned)(((size_t)d.M * d.N + 255) / 256), 256, 0, stream>>>(p);
   CUTB_CUDA_TRY(cudaGetLastError());
@@ -469,22 +585,15 @@ int moe_gemm_tc_launch(const cutb_moe_desc &d, cudaStream_t stream) {
   p.c_bf16 = d.c_dtype == CUTB_BF16;
   p.nk = p.nk_per = (d.K + DG_BK - 1) / DG_BK, p.ksplit = 1;
   p.a_box_rows = rows >= DG_BM ? DG_BM : (rows + 7) / 8 * 8;
-  // row tiles: every expert in use ends in a part-filled one.  Widths by the time of their waves, as in dg_plan.
-  const uint32_t used = d.experts < rows ? d.experts : rows, likely = rows / DG_BM + (used + 1) / 2;
-  int bn = 256;
-  uint64_t best = ~0ull;
-  const struct { int bn; uint32_t cost; } kinds[] = {{256, 100}, {128, 66}, {64, 62}};
-  for (const auto &kind : kinds) {
-    const uint64_t cost = (uint64_t)((likely * ((d.N + kind.bn - 1) / kind.bn) + sms - 1) / sms) * kind.cost;
-    if (cost < best) best = cost, bn = kind.bn;
-  }
-  p.tiles_m = rows / DG_BM + used, p.tiles_n = (d.N + bn - 1) / bn;
+  // row tiles: every expert in use ends in a part-filled one
+  const uint32_t used = d.experts < rows ? d.experts : rows;
+  DgPlan pl{};
+  dg_width(d.N, p.nk, sms, rows > DG_BM ? dg_pairs() : 0, [&](uint32_t n) { return rows / n + (used + 1) / 2; }, &pl);
+  p.tiles_m = rows / (pl.pair ? 2 * DG_BM : DG_BM) + used, p.tiles_n = pl.tiles_n;
   CUtensorMap ma, mw;
   if (int rc = make_tmap_sw128(&ma, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, d.A, rows, d.K, d.lda * 2, p.a_box_rows)) return rc;
-  if (int rc = make_tmap_sw128(&mw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, d.W, d.experts * d.N, d.K, (uint64_t)d.ldw * 2, (uint32_t)bn)) return rc;
-  return bn == 256 ? dg_launch<256, true>(ma, mw, p, sms, stream)
-       : bn == 128 ? dg_launch<128, true>(ma, mw, p, sms, stream)
-                   : dg_launch<64, true>(ma, mw, p, sms, stream);
+  if (int rc = make_tmap_sw128(&mw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, d.W, d.experts * d.N, d.K, (uint64_t)d.ldw * 2, pl.pair ? pl.bn / 2 : pl.bn)) return rc;
+  return dg_launch<true>(ma, mw, p, pl, sms, stream);
 }
 
 namespace {

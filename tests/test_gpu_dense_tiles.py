@@ -1,0 +1,58 @@
+"""Tiles of the dense bf16 GEMM at their edges: widths of 64 to 256, single CTAs and pairs, ragged rows, columns and k.
+
+bf16 operands are exact; fp32 sums of at most 2100 products: 1e-5; a bf16 result: 2^-9 at most, 2.5e-3."""
+import ctypes
+
+import pytest
+
+from cut_b200 import _lib as L
+from cut_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+
+def _rel(got, ref):
+    return float((got.double() - ref).norm() / ref.norm())
+
+
+@pytest.mark.parametrize("M,K,N,bf16,unary", [(129, 1024, 20000, True, 0), (256, 2048, 16600, False, 0), (257, 1024, 9001, True, 133), (1000, 2056, 5136, False, L.UNARY_RELU_SQUARE),
+                                             (2048, 1024, 6144, True, 0), (2100, 136, 4104, False, 133), (511, 1200, 14337, True, 0), (3000, 64, 1000, False, 0)])
+def test_dense_widths(M, K, N, bf16, unary):
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    A = torch.randn((M, K), device="cuda", generator=g).bfloat16()
+    W = torch.randn((N, K), device="cuda", generator=g).mul_(K ** -0.5).bfloat16()
+    bias = torch.randn(N, device="cuda", generator=g)
+    ld = (N + 7) // 8 * 8
+    out = torch.full((M, ld), float("nan"), device="cuda", dtype=torch.bfloat16 if bf16 else torch.float32)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    d = ops.dense_desc(A, W, K, out, bias=bias, unary=unary, variant=L.DENSE_TC, status=status, N=N)
+    ops.dense_matmul(d)
+    ref = A.double() @ W.double().T + bias.double()
+    ref = torch.nn.functional.silu(ref) if unary == 133 else ref.clamp(min=0).square() if unary else ref
+    assert int(status.item()) == 0
+    assert _rel(out[:, :N], ref) <= (2.5e-3 if bf16 else 1e-5)
+    assert bool(out[:, N:].isnan().all())  # nothing past the last column
+
+
+@pytest.mark.parametrize("counts,K,N,glu", [((700, 0, 1, 255, 256, 257, 31, 500), 1024, 2048, 0), ((3, 900, 130), 2056, 4128, 1), ((2048, 2048), 512, 4096, 0)])
+def test_grouped_widths(counts, K, N, glu):
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(K + N)
+    E, R = len(counts), sum(counts)
+    A = torch.randn((R, K), device="cuda", generator=g).bfloat16()
+    W = torch.randn((E * N, K), device="cuda", generator=g).mul_(K ** -0.5).bfloat16()
+    ends = torch.tensor((0,) + counts, device="cuda").cumsum(0)
+    out = torch.full((R, N // 2 if glu else N), float("nan"), device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    d = ops.moe_matmul_desc(A, W, K, ends.int(), E, R, 1, out, glu=L.GLU_CLAMPED if glu else L.GLU_NONE, alpha=1.702, beta=1.0, limit=7.0,
+                            variant=L.DENSE_TC, status=status)
+    L.check(L.lib().cutb_moe_matmul(ctypes.byref(d), torch.cuda.current_stream().cuda_stream))
+    ref = torch.cat([A[ends[e]: ends[e + 1]].double() @ W[e * N: (e + 1) * N].double().T for e in range(E)])
+    if glu:
+        a, u = ref[:, 0::2].clamp(max=7.0), ref[:, 1::2].clamp(-7.0, 7.0)
+        ref = a * torch.sigmoid(1.702 * a) * (u + 1.0)
+    assert int(status.item()) == 0
+    assert _rel(out, ref) <= 1e-5
