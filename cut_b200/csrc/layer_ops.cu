@@ -217,12 +217,34 @@ __global__ void __launch_bounds__(256) glu_pairs_kernel(const float2 *__restrict
   }
 }
 
+// The same for 16-byte aligned rows of a multiple of four outputs: four per thread, a row per blockIdx.y (no divisions).  Bound by
+// L2 / DRAM bytes; 512 x 28672 -> 14336: 26.5 us one output at a time -> 12.1.
+__global__ void __launch_bounds__(256) glu_pairs_vec_kernel(const float4 *__restrict__ in, float4 *__restrict__ out, uint32_t rows, uint32_t quads,
+                                                            uint64_t ldi4, uint64_t ldo4, int op) {
+  pdl_enter();
+  const uint32_t c = blockIdx.x * 256 + threadIdx.x;
+  if (c >= quads) return;
+  for (uint32_t r = blockIdx.y; r < rows; r += gridDim.y) {
+    const float4 a = __ldg(in + r * ldi4 + 2 * c), b = __ldg(in + r * ldi4 + 2 * c + 1);
+    float g[4] = {a.x, a.z, b.x, b.z};
+    const float none[4] = {};
+    apply_epilogue_n<4>(g, none, CUTB_FUSION_UNARY, op);
+    out[r * ldo4 + c] = make_float4(g[0] * a.y, g[1] * a.w, g[2] * b.y, g[3] * b.w);
+  }
+}
+
 }  // namespace
 
 int glu_pairs_launch(const float *in, float *out, uint32_t rows, uint32_t cols_out, uint64_t ldi, uint64_t ldo, int unary_op,
                      cudaStream_t stream) {
   const uint64_t total = (uint64_t)rows * cols_out;
   if (total == 0) return CUTB_OK;
+  if (cols_out % 4 == 0 && ldi % 4 == 0 && ldo % 4 == 0 && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
+    const uint32_t quads = cols_out / 4;
+    CUTB_CUDA_TRY(launch_pdl(glu_pairs_vec_kernel, dim3((quads + 255) / 256, rows < 65535u ? rows : 65535u), dim3(256), 0, stream,
+                             reinterpret_cast<const float4 *>(in), reinterpret_cast<float4 *>(out), rows, quads, ldi / 4, ldo / 4, unary_op));
+    return CUTB_OK;
+  }
   uint64_t blocks = (total + 255) / 256;
   DeviceInfo di;
   const uint64_t sms = (get_device_info(&di) == CUTB_OK && di.sm_count > 0) ? (uint64_t)di.sm_count : 148u;

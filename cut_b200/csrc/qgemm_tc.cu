@@ -526,11 +526,7 @@ int qgemm_tc_launch(const cutb_qmatmul_desc &d, cudaStream_t stream) {
                      (unsigned long long)need, (unsigned long long)d.workspace_bytes);
       return CUTB_ERR_WORKSPACE;
     }
-    const size_t total = (size_t)d.M * (d.K / 4);
-    const unsigned blocks = (unsigned)((total + 255) / 256 < (size_t)di.sm_count * 8 ? (total + 255) / 256 : (size_t)di.sm_count * 8);
-    cast_f32_f16_kernel<<<blocks, 256, 0, stream>>>(reinterpret_cast<const float *>(d.A), d.lda,
-                                                    reinterpret_cast<__half *>(d.workspace), d.M, d.K, d.status);
-    CUTB_CUDA_TRY(cudaGetLastError());
+    if (int rc = cast_f32_f16_launch(d, stream)) return rc;
     a16 = d.workspace;
     stride = (uint64_t)d.K * sizeof(__half);
   }

@@ -294,19 +294,35 @@ template <int FMT> __device__ __forceinline__ void convert_window(const RawWindo
 
 // fp32 activations -> fp16 rows of K elements (the TMA source of the GEMM).  A finite value beyond the
 // fp16 range (it rounds to infinity) is reported through the caller's status word.
-__global__ void cast_f32_f16_kernel(const float *__restrict__ A, uint32_t lda, __half *__restrict__ out, uint32_t M, uint32_t K,
-                                    int *status) {
-  const size_t total = (size_t)M * (K / 4);
+// Eight elements per thread, rows over blockIdx.y (K is a multiple of 128).
+__global__ void __launch_bounds__(256) cast_f32_f16_kernel(const float *__restrict__ A, uint32_t lda, __half *__restrict__ out, uint32_t M, uint32_t K,
+                                                           int *status) {
+  const uint32_t k = (blockIdx.x * 256 + threadIdx.x) * 8;
   bool over = false;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-    const size_t m = i / (K / 4), k = (i % (K / 4)) * 4;
-    const float4 f = __ldg(reinterpret_cast<const float4 *>(A + m * lda + k));
-    const float big = fmaxf(fmaxf(fabsf(f.x), fabsf(f.y)), fmaxf(fabsf(f.z), fabsf(f.w)));  // NaN operands drop out of fmaxf
-    over |= big > 65504.0f && big < __int_as_float(0x7f800000);
-    *reinterpret_cast<uint2 *>(out + m * K + k) =
-        make_uint2(h2_as_u32(__floats2half2_rn(f.x, f.y)), h2_as_u32(__floats2half2_rn(f.z, f.w)));
+  if (k < K) {
+    for (uint32_t m = blockIdx.y; m < M; m += gridDim.y) {
+      const float4 *src = reinterpret_cast<const float4 *>(A + (size_t)m * lda + k);
+      const float4 f = __ldg(src), g = __ldg(src + 1);
+      const float big = fmaxf(fmaxf(fmaxf(fabsf(f.x), fabsf(f.y)), fmaxf(fabsf(f.z), fabsf(f.w))),
+                              fmaxf(fmaxf(fabsf(g.x), fabsf(g.y)), fmaxf(fabsf(g.z), fabsf(g.w))));  // NaN operands drop out of fmaxf
+      // (an infinity beside a finite value out of range: look at them one by one)
+      if (big > 65504.0f) {
+        const float v[8] = {f.x, f.y, f.z, f.w, g.x, g.y, g.z, g.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) over |= fabsf(v[i]) > 65504.0f && fabsf(v[i]) < __int_as_float(0x7f800000);
+      }
+      *reinterpret_cast<uint4 *>(out + (size_t)m * K + k) =
+          make_uint4(h2_as_u32(__floats2half2_rn(f.x, f.y)), h2_as_u32(__floats2half2_rn(f.z, f.w)), h2_as_u32(__floats2half2_rn(g.x, g.y)),
+                     h2_as_u32(__floats2half2_rn(g.z, g.w)));
+    }
   }
   if (status && __any_sync(0xffffffffu, over) && (threadIdx.x & 31) == 0) atomicExch(status, (int)CUTB_ERR_RANGE);
+}
+int cast_f32_f16_launch(const cutb_qmatmul_desc &d, cudaStream_t stream) {
+  cast_f32_f16_kernel<<<dim3((d.K / 8 + 255) / 256, d.M < 65535u ? d.M : 65535u), 256, 0, stream>>>(reinterpret_cast<const float *>(d.A), d.lda,
+                                                                                                   reinterpret_cast<__half *>(d.workspace), d.M, d.K, d.status);
+  CUTB_CUDA_TRY(cudaGetLastError());
+  return CUTB_OK;
 }
 
 int make_tmap_a(CUtensorMap *map, const void *a_f16, uint32_t M, uint32_t K, uint64_t row_stride_bytes, uint32_t box_rows = TC_BT) {
