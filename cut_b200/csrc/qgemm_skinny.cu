@@ -183,7 +183,8 @@ __global__ void __launch_bounds__(sk_threads(FMT), 1)
       uint32_t d = tmem_base, acc = 0;           // acc 0: the next MMA starts a tile's accumulator
       bool dead = false;
       for (uint32_t j = 0; j < nstages; ++j) {
-        const bool ok = mbar_spin_bounded(fullb_u + sb * 8, pb) && mbar_spin_bounded(fulla_u + sa * 8, pa);
+        // (the activations first: they are there long before the weights)
+        const bool ok = mbar_spin_bounded(fulla_u + sa * 8, pa) && mbar_spin_bounded(fullb_u + sb * 8, pb);
         if (!__all_sync(0xffffffffu, ok)) {
           if (leader) give_up();
           dead = true;

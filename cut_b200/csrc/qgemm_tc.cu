@@ -76,6 +76,18 @@ __global__ void __launch_bounds__(tc_max_threads(FMT), 1) qgemm_tc_kernel(const 
   const uint32_t fulla_u = smem_u32(bars), fullb_u = fulla_u + SA * 8, cons_u = fullb_u + NB * 8, accum_u = cons_u + NC * 8;
   const uint32_t tmem_cols = MB == 1 ? 128u : (MB == 2 ? 256u : 512u);
 
+  // converters: the raw bytes of the first stage are on their way while barriers and tensor memory are set up
+  const uint32_t G = (blockDim.x - TC_CTRL_THREADS) >> 7, ct = tid - TC_CTRL_THREADS, r = ct & 127u, g = ct >> 7, n = n0 + r;
+  const bool live = warp >= 4 && n < p.N;
+  const uint8_t *wrow = tc_is_plane(FMT) ? p.W : p.W + (size_t)(live ? n : 0) * p.row_bytes;
+  RawWindow<FMT> nxt;
+#pragma unroll
+  for (int i = 0; i < RawWindow<FMT>::NV; ++i) nxt.v[i] = make_uint4(0, 0, 0, 0);
+  if (live && g < nk) {
+    if constexpr (tc_is_plane(FMT)) load_window_plane<FMT>(p, n, (kc0 + g * KS) * TC_BK, nxt);
+    else load_window<FMT>(wrow, (kc0 + g * KS) * TC_BK, nxt);
+  }
+
   if (tid == 0) {
     for (uint32_t s = 0; s < SA; ++s) mbar_init(fulla_u + s * 8, 1);  // the TMA lane's arrive.expect_tx
     for (uint32_t s = 0; s < NB; ++s) mbar_init(fullb_u + s * 8, 4);  // one arrival per converter warp of the owning group
@@ -116,7 +128,9 @@ __global__ void __launch_bounds__(tc_max_threads(FMT), 1) qgemm_tc_kernel(const 
       uint32_t sa = 0, pa = 0, sb = 0, pb = 0, sc = 0;
       bool dead = false;
       for (uint32_t ks = 0; ks < nk; ++ks) {
-        const bool ok = mbar_spin_bounded(fullb_u + sb * 8, pb) && mbar_spin_bounded(fulla_u + sa * 8, pa);
+        // the activations first: they are there long before the weights, and a wait costs 160 cycles even then, which must not
+        // stand between the converters' hand-over and the MMAs
+        const bool ok = mbar_spin_bounded(fulla_u + sa * 8, pa) && mbar_spin_bounded(fullb_u + sb * 8, pb);
         if (!__all_sync(0xffffffffu, ok)) {
           if (leader) give_up();
           dead = true;
@@ -185,18 +199,7 @@ __global__ void __launch_bounds__(tc_max_threads(FMT), 1) qgemm_tc_kernel(const 
   } else if (warp >= 4) {
     // ---- converters: one weight row per thread; group g owns K stages g, g + G, ... and keeps
     // the raw bytes of its next stage in flight while it converts the current one (G <= NB) ----
-    const uint32_t G = (blockDim.x - TC_CTRL_THREADS) >> 7;
-    const uint32_t ct = tid - TC_CTRL_THREADS, r = ct & 127u, g = ct >> 7, n = n0 + r;
-    const bool live = n < p.N;
-    const uint8_t *wrow = tc_is_plane(FMT) ? p.W : p.W + (size_t)(live ? n : 0) * p.row_bytes;
     bool dead = false;
-    RawWindow<FMT> nxt;
-#pragma unroll
-    for (int i = 0; i < RawWindow<FMT>::NV; ++i) nxt.v[i] = make_uint4(0, 0, 0, 0);
-    if (live && g < nk) {
-      if constexpr (tc_is_plane(FMT)) load_window_plane<FMT>(p, n, (kc0 + g * KS) * TC_BK, nxt);
-      else load_window<FMT>(wrow, (kc0 + g * KS) * TC_BK, nxt);
-    }
     // this group's slot sequence: start at slot g, advance by G modulo NB
     uint32_t sb = g % NB;
     uint32_t sc = 0, pc = 0;  // consumed barrier of stage ks - NB, once ks >= NB
