@@ -16,7 +16,7 @@
 // Bound by the latency of a token tile's chain scores -> softmax -> weighted values (about 4500 cycles per 128 keys, of which the
 // tensor cores work 1500 and the exponentials 2000 for the two tiles together); the weights of 64 keys at a time are handed over,
 // so that the products of the first half run beside the exponentials of the second.  32 heads of 128, window 1024, 2048 tokens:
-// 207 us with warp MMAs -> 90 us.
+// 207 us with warp MMAs -> 74 us (88.6 while blocks ran head by head; by ncu the tensor pipe is busy a third of a block's cycles).
 // Every wait is bounded; on expiry the block records CUTB_ERR_TIMEOUT, waits (bounded) for its copies, frees its tensor memory
 // and returns.
 #pragma once
@@ -149,8 +149,8 @@ __global__ void __launch_bounds__(PA_THREADS, 1)
     abort_flag = 0, hi_s[0] = hi_s[1] = 0;
     fence_mbar_init();
   }
-  // later tokens (which see more keys) first
-  const uint32_t tok0 = (gridDim.x - 1 - blockIdx.x) * p.step, h = blockIdx.y, kvh = h / p.rep, ntok = min(p.step, p.n_tokens - tok0);
+  // the later tokens of every head (which see more keys) first: the short blocks fill what the long ones leave
+  const uint32_t tok0 = (gridDim.y - 1 - blockIdx.y) * p.step, h = blockIdx.x, kvh = h / p.rep, ntok = min(p.step, p.n_tokens - tok0);
   pdl_enter();
   uint32_t p0 = 0;
   if constexpr (MODE != PA_LLAMA) {
@@ -612,7 +612,7 @@ int pa_launch_inst(const CUtensorMap &mk, const CUtensorMap &mr, const CUtensorM
   PaParams p = params;
   pa_set_vec(&p, MODE);
   CUTB_CUDA_TRY(cudaFuncSetAttribute(prefill_attention_kernel<MODE, KP, VP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  CUTB_CUDA_TRY(launch_pdl(prefill_attention_kernel<MODE, KP, VP>, dim3((p.n_tokens + p.step - 1) / p.step, p.n_heads), dim3(PA_THREADS), smem, stream,
+  CUTB_CUDA_TRY(launch_pdl(prefill_attention_kernel<MODE, KP, VP>, dim3(p.n_heads, (p.n_tokens + p.step - 1) / p.step), dim3(PA_THREADS), smem, stream,
                            mk, mr, mv, p));
   return CUTB_OK;
 }
