@@ -413,7 +413,7 @@ class LayerListDecoder:
     # -- launches -----------------------------------------------------------------------------------------------------
     @staticmethod
     def _stream() -> int:
-        return torch.cuda.current_stream().cuda_stream
+        return ops._stream_ptr()
 
     def _call(self, name: str, d) -> None:
         self.launches += 1

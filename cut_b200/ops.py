@@ -15,7 +15,8 @@ from . import _lib as L
 
 
 def _stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream of the current device (torch.cuda.current_stream() builds an object for it, some 4 us per launch)."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _pad4(n: int) -> int:
