@@ -215,6 +215,11 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
 __device__ __forceinline__ bool mbar_wait_probe_first(uint32_t bar, uint32_t parity) {
   return mbar_test(bar, parity) || mbar_wait_bounded(bar, parity);
 }
+// The same for a whole warp, with one answer for all of its lanes.  A phase may complete between two lanes' probes, so lanes that
+// decide for themselves can part before warp-wide work (MMAs, shuffles, votes), which then waits without a limit for the others.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, mbar_wait_probe_first(bar, parity));
+}
 // Bounded polling wait without parking: for the single threads on a kernel's critical
 // path (an MMA issuer, a copy producer), where the wake-up delay of a parked wait would
 // be paid once per pipeline step.  About a second at ~30 cycles per probe.

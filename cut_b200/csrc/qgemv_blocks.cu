@@ -867,12 +867,9 @@ __global__ void __launch_bounds__(GV_THREADS, MINB) qgemv_blocks_kernel(const Gv
     for (int nt = 0; nt < NT; ++nt) tot[nt][0] = tot[nt][1] = 0.f;
 
     for (uint32_t c = 0; c < cpt; ++c) {
-      if (!dead && !mbar_test(full_u + (slot * HV + hv) * 8, parity)) {  // the vote only on the slow path
-        const bool ok = mbar_wait_bounded(full_u + (slot * HV + hv) * 8, parity);
-        if (!__all_sync(0xffffffffu, ok)) {
-          dead = true;
-          if (lane == 0 && p.status) atomicExch(p.status, (int)CUTB_ERR_TIMEOUT);
-        }
+      if (!dead && !warp_wait(full_u + (slot * HV + hv) * 8, parity)) {
+        dead = true;
+        if (lane == 0 && p.status) atomicExch(p.status, (int)CUTB_ERR_TIMEOUT);
       }
       const uint32_t gq = gs0 + c * GV_KC + warp;  // this warp's granule of the chunk
       if (!dead && gq < gs1) {

@@ -240,11 +240,9 @@ __global__ void __launch_bounds__(GR_THREADS, 1) qgemv_rows_kernel(const __grid_
   const uint32_t act0 = WB + kg * 2 * NT * 512 + lane * 16, sum0 = WB + 4096 * NT + kg * 2 * NT * 32 + t * 8;
 
   for (uint32_t j = 0; j < n; ++j) {
-    if (!dead && !mbar_test(full + slot * 8, ph)) {  // the vote only on the slow path
-      if (!__all_sync(0xffffffffu, mbar_wait_bounded(full + slot * 8, ph))) {
-        dead = true;
-        if (lane == 0 && p.status) atomicExch(p.status, (int)CUTB_ERR_TIMEOUT);
-      }
+    if (!dead && !warp_wait(full + slot * 8, ph)) {
+      dead = true;
+      if (lane == 0 && p.status) atomicExch(p.status, (int)CUTB_ERR_TIMEOUT);
     }
     const uint32_t st = ring + slot * STAGE;
     if (!dead) {

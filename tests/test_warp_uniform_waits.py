@@ -1,0 +1,84 @@
+"""A warp decides about a wait as one: shown from the kernels' text, since lanes that part cannot be shown by running them.
+
+A barrier's phase may complete between the probes of two lanes.  A branch on such a probe may therefore split the warp, and a vote, a
+shuffle, an MMA or a tensor-memory load behind it waits for all lanes without a limit.  So a condition that probes a barrier goes
+through a vote (warp_wait, __all_sync, __any_sync) wherever what it guards is warp-wide work, unless a single lane runs it."""
+import glob
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "cut_b200", "csrc")
+VOTES = re.compile(r"\b(__all_sync|__any_sync|warp_wait)\s*\(")
+PER_LANE = re.compile(r"\bmbar_(test|try_wait|wait_\w+|spin_\w+)\s*\(")
+WARP_WIDE = re.compile(r"_sync\(\s*0x|\b__syncwarp\b|\bwarp_wait\b|sync\.aligned|\btmem_(ld|st)|\bgr_mma\b|\b(break|return|continue)\b")
+ONE_LANE = re.compile(r"\blane == 0\b|\bleader\b|\btid == 0\b")
+
+
+def _match(text, at, left, right):
+    """Index behind the bracket that closes the one at `at`."""
+    depth = 0
+    for i in range(at, len(text)):
+        depth += (text[i] == left) - (text[i] == right)
+        if depth == 0:
+            return i + 1
+    raise ValueError("unbalanced")
+
+
+def _without_comments(text):
+    text = re.sub(r"/\*.*?\*/", " ", text, flags=re.S)
+    return re.sub(r"//[^\n]*", "", text)
+
+
+def _statement(text, at):
+    """End of the statement that starts at or behind `at`."""
+    at += len(text[at:]) - len(text[at:].lstrip())
+    if text[at] == "{":
+        return _match(text, at, "{", "}")
+    m = re.match(r"(if|for|while)\s*(constexpr\s*)?\(", text[at:])
+    if m:
+        return _statement(text, _match(text, at + m.end() - 1, "(", ")"))
+    return text.index(";", at) + 1
+
+
+def _ifs(text):
+    for m in re.finditer(r"\bif\s*\(", text):
+        end = _match(text, m.end() - 1, "(", ")")
+        yield text[m.end(): end - 1], end, _statement(text, end)
+
+
+def _unvoted(cond):
+    while m := VOTES.search(cond):
+        cond = cond[: m.start()] + cond[_match(cond, m.end() - 1, "(", ")"):]
+    return cond
+
+
+def split_warps(text):
+    """Conditions that lanes decide for themselves in front of warp-wide work."""
+    text, found = _without_comments(text), []
+    every = list(_ifs(text))
+    for cond, start, end in every:
+        if not PER_LANE.search(_unvoted(cond)):
+            continue
+        alone = any(ONE_LANE.search(c) for c, s, e in every if s <= start and end <= e)
+        if not alone and WARP_WIDE.search(text[start: end]):
+            found.append(cond)
+    return found
+
+
+KERNELS = sorted(p for p in glob.glob(os.path.join(CSRC, "*.cu*")) if os.path.basename(p) != "common.cuh")  # (which defines the waits)
+
+
+@pytest.mark.parametrize("path", KERNELS, ids=os.path.basename)
+def test_no_lane_waits_alone_before_warp_wide_work(path):
+    with open(path) as f:
+        assert split_warps(f.read()) == []
+
+
+def test_the_reading_finds_what_it_is_for():
+    assert split_warps("if (!mbar_test(b, p)) { if (!__all_sync(0xffffffffu, mbar_wait_bounded(b, p))) dead = true; }")
+    assert split_warps("if (!dead && !mbar_wait_probe_first(b, p)) break;")
+    assert not split_warps("if (!dead && !warp_wait(b, p)) { dead = true; break; }")
+    assert not split_warps("if (lane == 0) { if (!mbar_spin_bounded(b, p)) break; }")
+    assert not split_warps("if (!dead && !mbar_spin_bounded(b, p)) { give_up(); dead = true; }")
