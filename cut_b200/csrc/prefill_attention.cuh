@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(PA_THREADS, 1)
       uint32_t at[2];  // rows of the tile's halves
 #pragma unroll
       for (uint32_t j = 0; j < 2; ++j) at[j] = MODE == PA_WINDOW ? (t * PA_BN + 64 * j) % p.ring_rows : t * PA_BN + 64 * j;
-      if (!__all_sync(0xffffffffu, mbar_wait_probe_first(kempty + sk * 8, pk)) || aborted()) {
+      if (!__all_sync(0xffffffffu, mbar_wait_probe_first(kempty + sk * 8, pk) && !aborted())) {
         if (leader) give_up();
         break;
       }
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(PA_THREADS, 1)
           }
       }
       if (++sk == SK) sk = 0, pk ^= 1u;
-      if (!__all_sync(0xffffffffu, mbar_wait_probe_first(vempty + sv * 8, pv)) || aborted()) {
+      if (!__all_sync(0xffffffffu, mbar_wait_probe_first(vempty + sv * 8, pv) && !aborted())) {
         if (leader) give_up();
         break;
       }
@@ -430,12 +430,11 @@ __global__ void __launch_bounds__(PA_THREADS, 1)
     for (uint32_t t = t_first; t < t_end; ++t) {
       const uint32_t key0 = t * PA_BN;
       if (key0 < my_hi && key0 + PA_BN > my_lo) {
-        if (!dead && !__all_sync(0xffffffffu, mbar_wait_probe_first(sfull + grp * 8, ph))) dead = true;
-        ph ^= 1u;
-        if (dead || aborted()) {
+        if (!__all_sync(0xffffffffu, mbar_wait_probe_first(sfull + grp * 8, ph) && !aborted())) {
           dead = true;
           break;
         }
+        ph ^= 1u;
         tc_fence_after();
         uint32_t s[4][32];
 #pragma unroll
@@ -466,7 +465,7 @@ __global__ void __launch_bounds__(PA_THREADS, 1)
           const float mn = fmaxf(m, mx), f = mn == -INFINITY ? 1.f : pa_exp2(m - mn);
           m = mn, l *= f;
           if (done) {
-            if (!__all_sync(0xffffffffu, mbar_wait_probe_first(odone + grp * 8, (done - 1) & 1u))) {
+            if (!warp_wait(odone + grp * 8, (done - 1) & 1u)) {
               dead = true;
               break;
             }
@@ -488,7 +487,7 @@ __global__ void __launch_bounds__(PA_THREADS, 1)
         const float ms = m == -INFINITY ? 0.f : m;  // nothing attended yet: keep exponents finite
         // Keys nobody in the block sees carry no weight, but a weight of zero times a stray NaN would not be zero.
         if (key0 < key_lo || key0 + PA_BN > key_hi) {
-          if (!__all_sync(0xffffffffu, mbar_wait_probe_first(vfull + sv * 8, pv))) {
+          if (!warp_wait(vfull + sv * 8, pv)) {
             dead = true;
             break;
           }
@@ -528,7 +527,7 @@ __global__ void __launch_bounds__(PA_THREADS, 1)
       }
       if (++sv == SV) sv = 0, pv ^= 1u;
     }
-    if (!dead && done && !__all_sync(0xffffffffu, mbar_wait_probe_first(odone + grp * 8, (done - 1) & 1u))) dead = true;
+    if (!dead && done && !warp_wait(odone + grp * 8, (done - 1) & 1u)) dead = true;
     if (dead) {
       if (lane == 0) give_up();
     } else if (done) {

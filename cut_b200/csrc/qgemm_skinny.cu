@@ -350,12 +350,10 @@ __global__ void __launch_bounds__(sk_threads(FMT), 1)
           cidx += CG;
           if (cidx >= NC) cidx -= NC, cph ^= 1u;
         }
+        if (lane == 0 && aborted()) ok = 0;
         ok = __shfl_sync(0xffffffffu, ok, 0);
         if (!ok) {
           if (lane == 0) give_up();
-          dead = true;
-        }
-        if (dead || aborted()) {
           dead = true;
           break;
         }
@@ -383,8 +381,8 @@ __global__ void __launch_bounds__(sk_threads(FMT), 1)
     const uint32_t q = warp & 3, half = (warp - 4) >> 2;  // warps of one quarter share its items
     const uint32_t m = q * 32 + lane;
     asm volatile("griddepcontrol.wait;" ::: "memory");  // C, D and the workspace may still be in use by the kernel before
-    if (!dead && !aborted() && nunits && q * 32 < p.M) {
-      if (!mbar_wait_bounded(accum_u, 0)) {
+    if (!dead && nunits && q * 32 < p.M) {
+      if (!__all_sync(0xffffffffu, !aborted() && mbar_wait_bounded(accum_u, 0))) {
         give_up();
       } else {
         tc_fence_after();

@@ -231,12 +231,10 @@ __global__ void __launch_bounds__(tc_max_threads(FMT), 1) qgemm_tc_kernel(const 
             sc += G;
             if (sc >= NC) sc -= NC, pc ^= 1u;
           }
+          if (lane == 0 && aborted()) ok = 0;
           ok = __shfl_sync(0xffffffffu, ok, 0);
           if (!ok) {
             if (lane == 0) give_up();
-            dead = true;
-          }
-          if (dead || aborted()) {
             dead = true;
             break;
           }
@@ -255,8 +253,8 @@ __global__ void __launch_bounds__(tc_max_threads(FMT), 1) qgemm_tc_kernel(const 
 
     // ---- epilogue: one TMEM lane (= weight row) per thread, 32 token columns per item; the
     // groups share the items round-robin; a warp's stores of one token cover 32 consecutive n ----
-    if (!dead && !aborted()) {
-      if (!mbar_wait_bounded(accum_u, 0)) {
+    if (!dead) {
+      if (!__all_sync(0xffffffffu, !aborted() && mbar_wait_bounded(accum_u, 0))) {
         give_up();
       } else {
         tc_fence_after();

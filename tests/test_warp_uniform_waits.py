@@ -1,8 +1,9 @@
 """A warp decides about a wait as one: shown from the kernels' text, since lanes that part cannot be shown by running them.
 
-A barrier's phase may complete between the probes of two lanes.  A branch on such a probe may therefore split the warp, and a vote, a
-shuffle, an MMA or a tensor-memory load behind it waits for all lanes without a limit.  So a condition that probes a barrier goes
-through a vote (warp_wait, __all_sync, __any_sync) wherever what it guards is warp-wide work, unless a single lane runs it."""
+A barrier's phase may complete between the probes of two lanes, and another warp may raise a block's abort flag between two lanes'
+reads.  A branch on such a probe may therefore split the warp, and a vote, a shuffle, an MMA or a tensor-memory load behind it waits for
+all lanes without a limit.  So a condition that probes a barrier or reads the flag goes through a vote (warp_wait, __all_sync,
+__any_sync) wherever what it guards, or what it chooses instead, is warp-wide work, unless a single lane runs it."""
 import glob
 import os
 import re
@@ -11,7 +12,7 @@ import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "cut_b200", "csrc")
 VOTES = re.compile(r"\b(__all_sync|__any_sync|warp_wait)\s*\(")
-PER_LANE = re.compile(r"\bmbar_(test|try_wait|wait_\w+|spin_\w+)\s*\(")
+PER_LANE = re.compile(r"\bmbar_(test|try_wait|wait_\w+|spin_\w+)\s*\(|\baborted\(\)")
 WARP_WIDE = re.compile(r"_sync\(\s*0x|\b__syncwarp\b|\bwarp_wait\b|sync\.aligned|\btmem_(ld|st)|\bgr_mma\b|\b(break|return|continue)\b")
 ONE_LANE = re.compile(r"\blane == 0\b|\bleader\b|\btid == 0\b")
 
@@ -38,14 +39,16 @@ def _statement(text, at):
         return _match(text, at, "{", "}")
     m = re.match(r"(if|for|while)\s*(constexpr\s*)?\(", text[at:])
     if m:
-        return _statement(text, _match(text, at + m.end() - 1, "(", ")"))
+        end = _statement(text, _match(text, at + m.end() - 1, "(", ")"))
+        other = re.match(r"\s*else\b", text[end:])
+        return _statement(text, end + other.end()) if m.group(1) == "if" and other else end
     return text.index(";", at) + 1
 
 
 def _ifs(text):
     for m in re.finditer(r"\bif\s*\(", text):
         end = _match(text, m.end() - 1, "(", ")")
-        yield text[m.end(): end - 1], end, _statement(text, end)
+        yield text[m.end(): end - 1], end, _statement(text, m.start())  # (with its else)
 
 
 def _unvoted(cond):
@@ -79,6 +82,9 @@ def test_no_lane_waits_alone_before_warp_wide_work(path):
 def test_the_reading_finds_what_it_is_for():
     assert split_warps("if (!mbar_test(b, p)) { if (!__all_sync(0xffffffffu, mbar_wait_bounded(b, p))) dead = true; }")
     assert split_warps("if (!dead && !mbar_wait_probe_first(b, p)) break;")
+    assert split_warps("if (dead || aborted()) { dead = true; break; }")
+    assert split_warps("if (!mbar_wait_bounded(b, 0)) { give_up(); } else { tmem_ld32(t, v); }")
+    assert not split_warps("if (!__all_sync(0xffffffffu, !aborted() && mbar_wait_bounded(b, 0))) give_up(); else tmem_ld32(t, v);")
     assert not split_warps("if (!dead && !warp_wait(b, p)) { dead = true; break; }")
     assert not split_warps("if (lane == 0) { if (!mbar_spin_bounded(b, p)) break; }")
     assert not split_warps("if (!dead && !mbar_spin_bounded(b, p)) { give_up(); dead = true; }")
