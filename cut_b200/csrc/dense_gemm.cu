@@ -15,8 +15,8 @@
 // the next expert's rows, whose products are not stored.  Neighbouring outputs may pass through a gated unit (gate, up).
 // Few tiles and a long K: the K stages of a tile are shared out over CTAs, partial sums go to the workspace and a second
 // kernel adds them in a fixed order and applies the epilogue.
-// Every wait is bounded; on expiry the CTA records CUTB_ERR_TIMEOUT in the caller's status word, waits (bounded) for its own
-// copies in flight, frees its tensor memory and returns.
+// Every wait is bounded; on expiry the CTA records CUTB_ERR_TIMEOUT in the caller's status word and tells the other CTA of its pair.
+// Copies in flight are waited for (bounded; a pair's by its first CTA, before the two part), tensor memory is freed.
 //
 // dense_gemm_simt_kernel: fp32 fused multiply-adds (bf16 weights are exact in fp32), for the true 32-bit mode.
 #include <cuda.h>
@@ -136,7 +136,16 @@ __global__ void __launch_bounds__(DG_THREADS, 1) dense_gemm_tc_kernel(const __gr
   const uint32_t tmem = tmem_slot;
   auto give_up = [&]() {
     if (p.status) atomicExch(p.status, (int)CUTB_ERR_TIMEOUT);
-    atomicExch(&abort_flag, 1u);
+    if constexpr (PAIR) {  // both CTAs of the pair (each stays until the other has come to its end)
+#pragma unroll
+      for (uint32_t r = 0; r < 2; ++r) {
+        uint32_t at;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_u32(&abort_flag)), "r"(r));
+        asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(at), "r"(1u) : "memory");
+      }
+    } else {
+      atomicExch(&abort_flag, 1u);
+    }
   };
   auto aborted = [&]() { return *reinterpret_cast<volatile uint32_t *>(&abort_flag) != 0; };
 
@@ -192,9 +201,10 @@ __global__ void __launch_bounds__(DG_THREADS, 1) dense_gemm_tc_kernel(const __gr
         if (++s == S) s = 0, ph ^= 1u;
       }
     }
-    // do not retire with copies still landing in shared memory: every stage's last fill (bounded; a stage that was never
-    // filled, or whose fill the MMA warp has consumed, answers at once or runs into the small limit of an aborted launch)
-    if (aborted()) {
+    // do not retire with copies still landing in shared memory, whoever gives up and when: every stage's last fill (bounded; a stage
+    // that was never filled, or whose fill has landed, answers at once, a step that a dead warp left out runs into the small limit).
+    // Both CTAs of a pair count on the first one's barriers, which waits for both; the second stays for the cluster barrier below.
+    if (rank == 0) {
       for (uint32_t i = 0; i < S; ++i) {
         if (s == 0) s = S, ph ^= 1u;
         --s;

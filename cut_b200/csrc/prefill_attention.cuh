@@ -240,17 +240,17 @@ __global__ void __launch_bounds__(PA_THREADS, 1)
       }
       if (++sv == SV) sv = 0, pv ^= 1u;
     }
-    if (aborted()) {  // do not retire with copies still landing: every slot's last fill (bounded)
-      for (uint32_t i = 0; i < SK; ++i) {
-        if (sk == 0) sk = SK, pk ^= 1u;
-        --sk;
-        mbar_wait_bounded(kfull + sk * 8, pk ^ 1u, 1u << 8);
-      }
-      for (uint32_t i = 0; i < SV; ++i) {
-        if (sv == 0) sv = SV, pv ^= 1u;
-        --sv;
-        mbar_wait_bounded(vfull + sv * 8, pv ^ 1u, 1u << 8);
-      }
+    // do not retire with copies still landing, whoever gives up and when: every slot's last fill (bounded; a slot that was never
+    // filled answers at once)
+    for (uint32_t i = 0; i < SK; ++i) {
+      if (sk == 0) sk = SK, pk ^= 1u;
+      --sk;
+      mbar_wait_bounded(kfull + sk * 8, pk ^ 1u, 1u << 8);
+    }
+    for (uint32_t i = 0; i < SV; ++i) {
+      if (sv == 0) sv = SV, pv ^= 1u;
+      --sv;
+      mbar_wait_bounded(vfull + sv * 8, pv ^ 1u, 1u << 8);
     }
     __syncwarp();
   } else if (warp == 9) {

@@ -233,13 +233,12 @@ __global__ void __launch_bounds__(sk_threads(FMT), 1)
         if (++sa == SA) sa = 0, pa ^= 1u;
         if (++kc == nk * SK_SUBS) kc = 0;
       }
-      if (aborted()) {  // no copy may still be landing when the CTA retires
-        const uint32_t pending = issued < SA ? issued : SA;
-        for (uint32_t i = 0; i < pending; ++i) {
-          if (sa == 0) sa = SA, pa ^= 1u;
-          --sa;
-          mbar_wait_bounded(fulla_u + sa * 8, pa ^ 1u, 1u << 10);
-        }
+      // no copy may still be landing when the CTA retires, whoever gives up and when (bounded)
+      const uint32_t pending = issued < SA ? issued : SA;
+      for (uint32_t i = 0; i < pending; ++i) {
+        if (sa == 0) sa = SA, pa ^= 1u;
+        --sa;
+        mbar_wait_bounded(fulla_u + sa * 8, pa ^ 1u, 1u << 10);
       }
     }
     __syncwarp();
@@ -269,13 +268,11 @@ __global__ void __launch_bounds__(sk_threads(FMT), 1)
             if (++a == nk) a = 0, ++tile;
           }
         }
-        if (aborted()) {
-          // drain: every granule issued completes its "full" phase; wait (bounded) for the last ring turn
-          const uint32_t pending = issued < RS ? issued : RS;
-          for (uint32_t i = 0; i < pending; ++i) {
-            const uint32_t g = issued - 1 - i;
-            mbar_wait_bounded(rawfull_u + (g % RS) * 8, (g / RS) & 1u, 1u << 10);
-          }
+        // drain: every granule issued completes its "full" phase; wait (bounded) for the last ring turn
+        const uint32_t pending = issued < RS ? issued : RS;
+        for (uint32_t i = 0; i < pending; ++i) {
+          const uint32_t g = issued - 1 - i;
+          mbar_wait_bounded(rawfull_u + (g % RS) * 8, (g / RS) & 1u, 1u << 10);
         }
       }
       __syncwarp();

@@ -184,15 +184,13 @@ __global__ void __launch_bounds__(tc_max_threads(FMT), 1) qgemm_tc_kernel(const 
         ++issued;
         if (++sa == SA) sa = 0, pa ^= 1u;
       }
-      // an aborting CTA must not retire with copies still landing in its shared memory:
+      // a CTA that gives up, at whatever point, must not retire with copies still landing in its shared memory:
       // wait (bounded) for the last ring turn of copies it issued
-      if (aborted()) {
-        const uint32_t pending = issued < SA ? issued : SA;
-        for (uint32_t i = 0; i < pending; ++i) {
-          if (sa == 0) sa = SA, pa ^= 1u;
-          --sa;
-          mbar_wait_bounded(fulla_u + sa * 8, pa ^ 1u, 1u << 10);
-        }
+      const uint32_t pending = issued < SA ? issued : SA;
+      for (uint32_t i = 0; i < pending; ++i) {
+        if (sa == 0) sa = SA, pa ^= 1u;
+        --sa;
+        mbar_wait_bounded(fulla_u + sa * 8, pa ^ 1u, 1u << 10);
       }
     }
     __syncwarp();

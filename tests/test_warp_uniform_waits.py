@@ -1,4 +1,4 @@
-"""A warp decides about a wait as one: shown from the kernels' text, since lanes that part cannot be shown by running them.
+"""Waits of the kernels, read from their text: what goes wrong around them cannot be shown by running it.
 
 A barrier's phase may complete between the probes of two lanes, and another warp may raise a block's abort flag between two lanes'
 reads.  A branch on such a probe may therefore split the warp, and a vote, a shuffle, an MMA or a tensor-memory load behind it waits for
@@ -77,6 +77,14 @@ KERNELS = sorted(p for p in glob.glob(os.path.join(CSRC, "*.cu*")) if os.path.ba
 def test_no_lane_waits_alone_before_warp_wide_work(path):
     with open(path) as f:
         assert split_warps(f.read()) == []
+
+
+@pytest.mark.parametrize("path", KERNELS, ids=os.path.basename)
+def test_copies_in_flight_are_waited_for_whoever_gives_up_and_when(path):
+    """A copy warp that has issued everything may end before another warp gives up: its wait for copies does not hang on the flag."""
+    with open(path) as f:
+        text = _without_comments(f.read())
+    assert [c for c, start, end in _ifs(text) if "aborted()" in c and "mbar_wait_bounded" in text[start: end] and "tmem_ld" not in text[start: end]] == []
 
 
 def test_the_reading_finds_what_it_is_for():
