@@ -150,15 +150,17 @@ __global__ void __launch_bounds__(PA_THREADS, 1)
     fence_mbar_init();
   }
   // the later tokens of every head (which see more keys) first: the short blocks fill what the long ones leave
-  const uint32_t tok0 = (gridDim.y - 1 - blockIdx.y) * p.step, h = blockIdx.x, kvh = h / p.rep, ntok = min(p.step, p.n_tokens - tok0);
+  const uint32_t tok0 = (gridDim.y - 1 - blockIdx.y) * p.step, h = blockIdx.x, kvh = h / p.rep;
+  uint32_t p0 = 0, ntok = min(p.step, p.n_tokens - tok0);
   pdl_enter();
-  uint32_t p0 = 0;
   if constexpr (MODE != PA_LLAMA) {
-    p0 = (p.pos_ptr ? *p.pos_ptr : p.pos) + tok0;
-    if (p0 + ntok > p.max_pos) {  // no table rows: the cache write has done nothing for them either
+    const uint64_t first = (uint64_t)(p.pos_ptr ? *p.pos_ptr : p.pos) + tok0;
+    if (first + ntok > p.max_pos) {  // tokens without table rows are left out, as the cache write leaves them out
       if (p.status && tid == 0 && h == 0) atomicExch(p.status, (int)CUTB_ERR_INVALID);
-      return;
+      if (first >= p.max_pos) return;
+      ntok = (uint32_t)(p.max_pos - first);
     }
+    p0 = (uint32_t)first;
   }
   if (warp == 9) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(512u) : "memory");

@@ -76,6 +76,32 @@ def test_window(T, pos, window, dim, vdim, rot, near, scale, sink):
     assert _rel(out.view(T, H, vdim), ref) <= (4e-3 if rot else 1e-4)
 
 
+@pytest.mark.parametrize("T,heads,past,max_pos", [(300, 4, 1, 400), (300, 4, 150, 400), (500, 74, 90, 600), (130, 4, 129, 200)])
+def test_window_tokens_without_table_rows(T, heads, past, max_pos):
+    """The last `past` tokens lie beyond the tables: they stay unwritten and the status says so; every other token is served, wherever
+    the blocks of 128 and (500 tokens x 74 heads) 256 tokens end."""
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(T + past)
+    rand = lambda *s: torch.randn(s, device="cuda", generator=g)
+    pos, window, hd, n = max_pos - (T - past), 200, 128, T - past
+    ring = (window + T + 63) // 64 * 64
+    k, v, q = rand(max_pos, 2, hd).bfloat16(), rand(max_pos, 2, hd).bfloat16(), rand(T, heads, hd).bfloat16().float()
+    kc, vc = torch.full((ring, 2, hd), float("nan"), device="cuda").bfloat16(), torch.full((ring, 2, hd), float("nan"), device="cuda").bfloat16()
+    kept = torch.arange(max(0, pos + 1 - window), max_pos, device="cuda")
+    kc[kept % ring], vc[kept % ring] = k[kept], v[kept]
+    qkv = torch.zeros((T, (heads + 4) * hd), device="cuda")
+    qkv[:, : heads * hd] = q.reshape(T, -1)
+    out, status = torch.full((T, heads * hd), float("nan"), device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    ops.window_attention(ops.window_desc(qkv, heads, 2, hd, hd, kc.view(ring, -1), vc.view(ring, -1), window=window, scale=0.1, out=out, max_pos=max_pos,
+                                         sink=True, pos=pos, status=status))
+    zero = torch.zeros(heads, dtype=torch.float64, device="cuda")
+    ref = _reference(q[:n].double(), k.double(), v.double(), 0.1, torch.arange(pos, max_pos, device="cuda"), window, zero)
+    assert int(status.item()) == L.ERR_INVALID
+    assert bool(out[n:].isnan().all())
+    assert _rel(out[:n].view(n, heads, hd), ref) <= 1e-4
+
+
 @pytest.mark.parametrize("T,pos,dim,rot,vdim,scale", [(40, 0, 128, 64, 128, 0.1), (128, 5, 64, 32, 64, 0.1), (257, 127, 128, 32, 128, -0.1),
                                                      (300, 0, 24, 8, 40, 0.1), (1100, 64, 64, 64, 128, 0.1), (130, 0, 128, 0, 72, 0.1)])
 @pytest.mark.parametrize("on_device", [False, True])
