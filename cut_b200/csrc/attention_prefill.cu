@@ -50,6 +50,7 @@ int batched_attention_tc_launch(const float *q_in, uint32_t q_stride, const void
   a.rot = headDim, a.cos_t = cosT, a.sin_t = sinT, a.positions = positions, a.max_pos = max_seq;
   a.step = pa_step(n_tokens, nHeads, (uint32_t)di.sm_count), a.ksteps = headDim / 16, a.key_planes = headDim / 64;
   a.out = out, a.ldo = out_stride, a.vdim = headDim, a.status = status;
+  a.k = reinterpret_cast<const uint16_t *>(kC), a.v = reinterpret_cast<const uint16_t *>(vC), a.ld_k = a.ld_v = ld, a.k_head = a.v_head = headDim;
   pa_set_scale(&a, scale);
   return headDim == 128 ? ll_launch<2>(a, kC, vC, nKvHeads, ld, stream) : ll_launch<1>(a, kC, vC, nKvHeads, ld, stream);
 }

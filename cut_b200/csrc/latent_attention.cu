@@ -808,6 +808,9 @@ template <int KP, int VP> int lt_launch(const cutb_latent_attn_desc &d, cudaStre
   p.step = pa_step(d.n_tokens, d.n_heads, (uint32_t)di.sm_count);
   p.ksteps = d.rot_dim ? (p.rot_col + d.rot_dim + 15) / 16 : (d.dim + 15) / 16;
   p.sink = d.sink, p.out = d.out, p.ldo = d.ldo, p.vdim = d.vdim, p.out_bf16 = d.out_dtype == CUTB_BF16, p.status = d.status;
+  p.k = reinterpret_cast<const uint16_t *>(d.k_exp), p.k_head = d.dim, p.ld_k = d.ld_k;
+  p.v = reinterpret_cast<const uint16_t *>(d.v_exp), p.v_head = d.vdim, p.ld_v = d.ld_v;
+  p.r = reinterpret_cast<const uint16_t *>(d.cache) + d.rot_at, p.ld_r = d.ld_cache;
   pa_set_scale(&p, d.scale);
   // rows past the batch's last token may not exist: they are past the tensors and read as zero
   const uint64_t rows = (uint64_t)d.pos + d.n_tokens;
@@ -816,7 +819,7 @@ template <int KP, int VP> int lt_launch(const cutb_latent_attn_desc &d, cudaStre
   if (int rc = pa_map(&mv, true, d.v_exp, d.vdim, d.n_heads, d.vdim, rows, d.ld_v)) return rc;
   mr = mk;
   if (d.rot_dim)
-    if (int rc = pa_map(&mr, true, reinterpret_cast<const __nv_bfloat16 *>(d.cache) + d.rot_at, d.rot_dim, 1, d.ld_cache, rows, d.ld_cache)) return rc;
+    if (int rc = pa_map(&mr, true, p.r, d.rot_dim, 1, d.ld_cache, rows, d.ld_cache)) return rc;
   return pa_launch_inst<PA_LATENT, KP, VP>(mk, mr, mv, p, stream);
 }
 template <int VP> int lt_dispatch(const cutb_latent_attn_desc &d, uint32_t planes, cudaStream_t stream) {

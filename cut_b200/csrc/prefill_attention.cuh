@@ -17,6 +17,7 @@
 // tensor cores work 1500 and the exponentials 2000 for the two tiles together); the weights of 64 keys at a time are handed over,
 // so that the products of the first half run beside the exponentials of the second.  32 heads of 128, window 1024, 2048 tokens:
 // 207 us with warp MMAs -> 74 us (88.6 while blocks ran head by head; by ncu the tensor pipe is busy a third of a block's cycles).
+// A row that comes out non-finite is computed again from the keys it sees alone (pa_row_again).
 // Every wait is bounded; on expiry the block records CUTB_ERR_TIMEOUT, waits (bounded) for its copies, frees its tensor memory
 // and returns.
 #pragma once
@@ -48,6 +49,9 @@ struct PaParams {
   uint32_t step;              // tokens per block: 128 or 256
   uint32_t ksteps;            // 16-column steps of the score product
   uint32_t key_planes;        // 64-column planes that come from the heads' own keys (the others: the shared turned part)
+  const uint16_t *k, *r, *v;  // what the tensor maps cover, for pa_row_again: keys, the shared turned part, values; strides in elements
+  uint64_t ld_k, ld_r, ld_v;
+  uint32_t k_head, v_head;
   int q_vec;                  // queries and tables allow eight pairs at a time (pa_set_vec)
   float scale, q_mul;         // |scale| log2(e), and the scale's sign: the maxima are taken of raw scores
   const float *sink;          // PA_LATENT: a logit per head
@@ -125,10 +129,50 @@ template <int MODE> __device__ __forceinline__ uint16_t pa_bits(float v) {
   else return __bfloat16_as_ushort(__float2bfloat16_rn(v));
 }
 
+// One token's output again, by one warp in fp32: a key that the token does not see has a weight of zero in its tile, and zero times an
+// infinity or a NaN is not zero, so a row that came out non-finite may owe it to keys of other tokens.  `q`: the token tile's
+// queries in shared memory, `r` the row; ms, inv: the token's followed maximum and 1 / sum.
+template <int MODE>
+__device__ __noinline__ void pa_row_again(const PaParams &p, const uint8_t *q, uint32_t r, uint32_t h, uint32_t tok, uint32_t pos, float ms, float inv) {
+  const uint32_t lane = threadIdx.x & 31, kvh = h / p.rep, first = MODE == PA_WINDOW && pos + 1 > p.window ? pos + 1 - p.window : 0;
+  auto number = [](uint32_t bits) {
+    if constexpr (MODE == PA_LLAMA) return __half2float(__ushort_as_half((uint16_t)bits));
+    else return __uint_as_float(bits << 16);
+  };
+  auto row_of = [&](uint32_t key) { return (uint64_t)(MODE == PA_WINDOW ? key % p.ring_rows : key); };
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  for (uint32_t k0 = first; k0 <= pos; k0 += 32) {
+    const uint32_t key = k0 + lane;
+    float w = 0.f;
+    if (key <= pos) {
+      const uint64_t row = row_of(key);
+      float s = 0.f;
+      for (uint32_t c = 0; c < p.ksteps * 16; ++c) {
+        const bool turned = MODE == PA_LATENT && c >= p.rot_col;
+        const uint32_t e = turned ? c - p.rot_col : c, n = MODE == PA_LATENT ? (turned ? p.rot : p.dim) : p.q_head;
+        if (e >= n) continue;
+        const uint32_t x = *reinterpret_cast<const uint16_t *>(q + (c >> 6) * PA_PLANE + r * 128u + ((((c & 63u) >> 3) ^ (r & 7u)) << 4) + (c & 7u) * 2u);
+        s = fmaf(number(x), number(__ldg(turned ? p.r + row * p.ld_r + e : p.k + row * p.ld_k + (uint64_t)kvh * p.k_head + e)), s);
+      }
+      w = pa_exp2(fmaf(s, p.scale, -ms));
+    }
+    for (uint32_t j = 0; j < 32 && k0 + j <= pos; ++j) {
+      const float wj = __shfl_sync(0xffffffffu, w, j);
+      const uint16_t *src = p.v + row_of(k0 + j) * p.ld_v + (uint64_t)kvh * p.v_head;
+#pragma unroll
+      for (uint32_t i = 0; i < 4; ++i)
+        if (lane + 32 * i < p.vdim) acc[i] = fmaf(wj, number(__ldg(src + lane + 32 * i)), acc[i]);
+    }
+  }
+#pragma unroll
+  for (uint32_t i = 0; i < 4; ++i)
+    if (lane + 32 * i < p.vdim) store_out(p.out, p.out_bf16, (uint64_t)tok * p.ldo + (uint64_t)h * p.vdim + lane + 32 * i, acc[i] * inv);
+}
+
 template <int MODE, int KP, int VP>
 __global__ void __launch_bounds__(PA_THREADS, 1)
     prefill_attention_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_r,
-                             const __grid_constant__ CUtensorMap map_v, const PaParams p) {
+                             const __grid_constant__ CUtensorMap map_v, const __grid_constant__ PaParams p) {
   constexpr bool BF16 = MODE != PA_LLAMA;
   constexpr uint32_t SK = PaRings<KP>::K, SV = PaRings<KP>::V, QT = KP * PA_PLANE, KT = KP * PA_PLANE, VT = VP * PA_PLANE;
   extern __shared__ __align__(1024) uint8_t pa_raw[];
@@ -538,6 +582,7 @@ __global__ void __launch_bounds__(PA_THREADS, 1)
       const float inv = MODE == PA_LLAMA ? (l > 0.f ? 1.0f / l : 0.f) : 1.0f / l;
       const uint64_t base = (uint64_t)tok * p.ldo + (uint64_t)h * p.vdim;
       const bool quads = p.vdim % 8 == 0 && p.ldo % 8 == 0 && reinterpret_cast<uintptr_t>(p.out) % 16 == 0;
+      float stray = 0.f;  // becomes NaN with the first output that is not finite
 #pragma unroll 1
       for (uint32_t c = 0; c < VP * 64; c += 32) {
         if (c >= p.vdim) break;
@@ -547,7 +592,7 @@ __global__ void __launch_bounds__(PA_THREADS, 1)
         if (!live) continue;
         float y[32];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) y[i] = __uint_as_float(o[i]) * inv;
+        for (int i = 0; i < 32; ++i) y[i] = __uint_as_float(o[i]) * inv, stray = fmaf(y[i], 0.f, stray);
         if (quads) {
 #pragma unroll
           for (int i = 0; i < 32; i += 8) {
@@ -565,6 +610,12 @@ __global__ void __launch_bounds__(PA_THREADS, 1)
           for (int i = 0; i < 32; ++i)
             if (c + i < p.vdim) store_out(p.out, p.out_bf16, base + c + i, y[i]);
         }
+      }
+      __syncwarp();  // (rows stored above are stored again below, by other lanes)
+      for (uint32_t again = __ballot_sync(0xffffffffu, live && !(stray == 0.f)); again; again &= again - 1) {
+        const int src = __ffs(again) - 1;
+        pa_row_again<MODE>(p, smem + grp * QT, (warp & 3) * 32 + src, h, tok - lane + src, __shfl_sync(0xffffffffu, pos, src),
+                           __shfl_sync(0xffffffffu, m == -INFINITY ? 0.f : m, src), __shfl_sync(0xffffffffu, inv, src));
       }
     }
   }

@@ -632,10 +632,12 @@ template <int KP, int VP> int wp_launch(const cutb_window_attn_desc &d, cudaStre
   p.pos_ptr = d.pos_ptr, p.pos = d.pos, p.max_pos = d.max_pos, p.window = d.window, p.ring_rows = d.ring_rows;
   p.step = pa_step(d.n_tokens, d.n_heads, (uint32_t)di.sm_count), p.ksteps = (d.dim + 15) / 16, p.key_planes = KP;
   p.zero_sink = d.sink != 0, p.out = d.out, p.ldo = d.ldo, p.vdim = d.vdim, p.out_bf16 = d.out_dtype == CUTB_BF16, p.status = d.status;
+  p.k = reinterpret_cast<const uint16_t *>(d.k_cache), p.k_head = d.k_head, p.ld_k = (uint64_t)d.n_kv_heads * d.k_head;
+  p.v = reinterpret_cast<const uint16_t *>(d.v_cache), p.v_head = d.v_head, p.ld_v = (uint64_t)d.n_kv_heads * d.v_head;
   pa_set_scale(&p, d.scale);
   CUtensorMap mk, mv;
-  if (int rc = pa_map(&mk, true, d.k_cache, d.k_head, d.n_kv_heads, d.k_head, d.ring_rows, (uint64_t)d.n_kv_heads * d.k_head)) return rc;
-  if (int rc = pa_map(&mv, true, d.v_cache, d.v_head, d.n_kv_heads, d.v_head, d.ring_rows, (uint64_t)d.n_kv_heads * d.v_head)) return rc;
+  if (int rc = pa_map(&mk, true, d.k_cache, d.k_head, d.n_kv_heads, d.k_head, d.ring_rows, p.ld_k)) return rc;
+  if (int rc = pa_map(&mv, true, d.v_cache, d.v_head, d.n_kv_heads, d.v_head, d.ring_rows, p.ld_v)) return rc;
   return pa_launch_inst<PA_WINDOW, KP, VP>(mk, mk, mv, p, stream);
 }
 

@@ -151,3 +151,80 @@ def test_llama(T, hd, order):
     ref = _reference(_turned(q, cos[at], sin[at], False).half().double(), kc[seen].double(), vc[seen].double(), hd ** -0.5, at, 1 << 30, None)
     assert int(status.item()) == 0
     assert _rel(out.view(T, H, hd), ref) <= 1e-3
+
+
+def _attend(mode, q, k, v, pos, window, scale, status, sink=None, order=None):
+    """Unrotated attention of queries [T, H, d] at pos, pos + 1, ... (or at positions `order`) over k, v [positions, G, .], through the entry
+    point of `mode`; sink: a logit per head (llama: none, window: zeros)."""
+    import ctypes
+
+    import torch
+
+    T, H, hd = q.shape
+    end, G = k.shape[0], k.shape[1]
+    ones, zeros = torch.ones((end, hd // 2), device="cuda"), torch.zeros((end, hd // 2), device="cuda")
+    out = torch.full((T, H * hd), float("nan"), device="cuda")
+    if mode == "llama":
+        at = torch.arange(pos, end, device="cuda", dtype=torch.int32) if order is None else order.int()
+        ops.batched_attention(q.view(T, -1), k.view(end, -1), v.view(end, -1), at, ones, zeros, H, G, hd, out=out, scale=scale, status=status)
+    elif mode == "window":
+        ring = (min(window, end) + T + 63) // 64 * 64
+        kc, vc = torch.full((ring, G, hd), float("nan"), device="cuda").bfloat16(), torch.full((ring, G, hd), float("nan"), device="cuda").bfloat16()
+        kept = torch.arange(max(0, pos + 1 - window), end, device="cuda")
+        kc[kept % ring], vc[kept % ring] = k[kept], v[kept]
+        qkv = torch.zeros((T, (H + 2 * G) * hd), device="cuda")
+        qkv[:, : H * hd] = q.view(T, -1)
+        ops.window_attention(ops.window_desc(qkv, H, G, hd, hd, kc.view(ring, -1), vc.view(ring, -1), window=window, scale=scale, out=out, max_pos=end,
+                                             sink=sink is not None, pos=pos, status=status))
+    else:  # a third of the head as the shared turned part: equal in all heads
+        rot = 64
+        cache = torch.zeros((end, 64 + rot), device="cuda").bfloat16()
+        cache[:, 64:] = k[:, 0, hd - rot:]
+        d = ops.latent_desc(cache, H, hd - rot, rot, v.shape[2], 64, scale=scale, eps=1e-6, max_pos=end, n_tokens=T, cos_t=ones, sin_t=zeros, sink=sink, pos=pos,
+                            q=q.view(T, -1), k_exp=k[:, :, : hd - rot].reshape(end, -1), v_exp=v.reshape(end, -1), out=out[:, : H * v.shape[2]], status=status)
+        L.check(L.lib().cutb_latent_prefill(ctypes.byref(d), torch.cuda.current_stream().cuda_stream))
+        out = out[:, : H * v.shape[2]]
+    return out.view(T, H, -1)
+
+
+def _inputs(mode, T, pos, seed):
+    """q, k, v and a head count that gives blocks of 256 tokens (128 while the launch would leave multiprocessors idle) if T > 600."""
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    big = T > 600
+    H = 50 if big else 6
+    assert (-(-T // 256) * H >= torch.cuda.get_device_properties(0).multi_processor_count) == big
+    G, hd, vd = (H, 192, 128) if mode == "latent" else (10 if big else 2, 128, 128)
+    t = torch.float16 if mode == "llama" else torch.bfloat16
+    rand = lambda *s: torch.randn(s, device="cuda", generator=g).to(t)
+    q, k, v = rand(T, H, hd), rand(pos + T, G, hd), rand(pos + T, G, vd)
+    if mode == "latent":
+        k[:, :, 128:] = k[:, :1, 128:]
+    return q.float(), k, v
+
+
+@pytest.mark.parametrize("mode", ["llama", "window", "latent"])
+@pytest.mark.parametrize("T,pos,window", [(300, 0, 1 << 20), (300, 77, 90), (641, 0, 1 << 20), (700, 60, 200)])
+def test_values_that_are_not_finite(mode, T, pos, window):
+    """An infinity or a NaN among the values reaches the tokens that see its key, in its column, and no other."""
+    import torch
+
+    if mode != "window":
+        window = 1 << 20
+    q, k, v = _inputs(mode, T, pos, T + pos)
+    H, G, at = q.shape[1], k.shape[1], torch.arange(pos, pos + T, device="cuda")
+    strays = [(3, 0, 5, float("inf")), (pos + 130, G - 1, 0, float("nan")), (pos + 255, 0, 77, float("-inf")), (pos + T - 1, G - 1, 127, float("nan"))]
+    clean = v.clone()
+    for key, g, col, x in strays:
+        v[key, g, col], clean[key, g, col] = x, 0.0
+    ref = _reference(q.double(), k.double(), clean.double(), 0.1, at, window, None)
+    for key, g, col, x in strays:
+        seen = (at >= key) & (at - key < window)
+        ref[seen, g * (H // G): (g + 1) * (H // G), col] = x
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    got = _attend(mode, q, k, v, pos, window, 0.1, status)
+    finite = ref.isfinite()
+    assert int(status.item()) == 0
+    assert bool((got.isfinite() == finite).all()) and bool((got.isnan() == ref.isnan()).all()) and bool((got == ref)[ref.isinf()].all())
+    assert _rel(got[finite], ref[finite]) <= (1e-3 if mode == "llama" else 1e-4)
