@@ -19,7 +19,7 @@ DENSE_AUTO, DENSE_MATVEC, DENSE_TC, DENSE_SIMT = -1, 0, 1, 2
 ROT_HALVES, ROT_NEIGHBOURS = 0, 1
 LAYOUT_GGUF_BLOCKS, LAYOUT_KN_PLANES = 0, 1
 FUSION_NONE, FUSION_UNARY, FUSION_BINARY = 0, 1, 2
-VARIANT_AUTO, VARIANT_GENERIC, VARIANT_GEMV_MMA, VARIANT_GEMM_TC, VARIANT_GEMV_PLANES = -1, 0, 1, 2, 3
+VARIANT_AUTO, VARIANT_GENERIC, VARIANT_GEMV_MMA, VARIANT_GEMM_TC, VARIANT_GEMV_PLANES, VARIANT_ROWS_MMA = -1, 0, 1, 2, 3, 4
 FLAG_NO_OVERLAP = 1
 FLAG_ACT_16BIT = 2
 FLAG_A_RMSNORM = 4

@@ -94,7 +94,7 @@ int validate(const cutb_qmatmul_desc *d) {
       return CUTB_ERR_INVALID;
     }
   }
-  if (d->variant < CUTB_VARIANT_AUTO || d->variant > CUTB_VARIANT_GEMV_PLANES) {
+  if (d->variant < CUTB_VARIANT_AUTO || d->variant > CUTB_VARIANT_ROWS_MMA) {
     set_last_error("qmatmul: unknown variant %d", d->variant);
     return CUTB_ERR_INVALID;
   }
@@ -103,14 +103,16 @@ int validate(const cutb_qmatmul_desc *d) {
 
 // Decode shapes go to the bulk-copy MMA mat-vec, prefill shapes to the
 // tensor-core GEMM, everything else to the SIMT kernel.  The reference makes
-// the same split on M (operators/impl/matmul/MatMulOp.cpp:335-380).
+// the same split on M (operators/impl/matmul/MatMulOp.cpp:335-380).  This is the choice for a caller without scratch: with it, 9 to
+// 32 rows may run as fp16 MMAs instead (rows_instead).
 int select(const cutb_qmatmul_desc &d) {
   if (d.variant != CUTB_VARIANT_AUTO) return d.variant;
   if (d.layout == CUTB_LAYOUT_GGUF_BLOCKS) {
     if (qgemv_blocks_supported(d)) {
       // 13 to 16 fp16 rows need the mat-vec's fourth column tile; from 16 M weights up the tensor-core GEMM for few
       // tokens is faster there (16 rows: 4096 x 4096 15.0 against 11.2 us, 11008 x 4096 28.0 against 22.1 us; at
-      // 2048 x 2048 the mat-vec wins, 6.1 against 7.5 us).  The fused RMSNorm exists in the mat-vec only.
+      // 2048 x 2048 the mat-vec wins, 6.1 against 7.5 us).  Q8_0 and Q4_0 take this line without scratch only, Q4_K and
+      // paired rows always.  The fused RMSNorm exists in the mat-vec only.
       const bool matvec_only = d.flags & CUTB_FLAG_A_RMSNORM;
       if (d.a_dtype == CUTB_F16 && d.M >= 13 && (uint64_t)d.K * d.N >= (1ull << 24) && !matvec_only && qgemm_tc_supported(d))
         return CUTB_VARIANT_GEMM_TC;
@@ -123,6 +125,15 @@ int select(const cutb_qmatmul_desc &d) {
     return CUTB_VARIANT_GEMM_TC;  // prefill over the planes: the tensor-core GEMM with plane converters
   }
   return CUTB_VARIANT_GENERIC;
+}
+// fp32 rows that the mat-vec takes stay there (they keep their range in its digits)
+bool rows_instead(const cutb_qmatmul_desc &d, int v) {
+  return d.variant == CUTB_VARIANT_AUTO && (v == CUTB_VARIANT_GEMM_TC || (v == CUTB_VARIANT_GEMV_MMA && d.a_dtype == CUTB_F16)) &&
+         qgemv_rows_supported(d) && qgemv_rows_faster(d);
+}
+int chosen(const cutb_qmatmul_desc &d) {
+  const int v = select(d);
+  return rows_instead(d, v) && qgemv_rows_fits(d) ? CUTB_VARIANT_ROWS_MMA : v;
 }
 
 }  // namespace
@@ -141,28 +152,32 @@ const char *cutb_variant_name(int variant) {
     case CUTB_VARIANT_GEMV_MMA: return "QGemvBulkMma";
     case CUTB_VARIANT_GEMM_TC: return "QGemmTcgen05";
     case CUTB_VARIANT_GEMV_PLANES: return "QGemvPlanes";
+    case CUTB_VARIANT_ROWS_MMA: return "QGemvRowsMma";
     default: return "Unknown";
   }
 }
 
 int cutb_qmatmul_select_variant(const cutb_qmatmul_desc *desc) {
   if (validate(desc) != CUTB_OK) return -1;
-  return select(*desc);
+  return chosen(*desc);
 }
 
 uint64_t cutb_qmatmul_workspace_bytes(const cutb_qmatmul_desc *desc) {
   if (validate(desc) != CUTB_OK) return 0;
   const int v = select(*desc);
-  if (v == CUTB_VARIANT_GEMV_MMA) return qgemv_blocks_workspace(*desc);
-  if (v == CUTB_VARIANT_GEMM_TC) return qgemm_tc_workspace(*desc);
-  if (v == CUTB_VARIANT_GEMV_PLANES) return qgemv_planes_workspace(*desc);
-  return 0;
+  uint64_t need = 0;
+  if (v == CUTB_VARIANT_GEMV_MMA) need = qgemv_blocks_workspace(*desc);
+  if (v == CUTB_VARIANT_GEMM_TC) need = qgemm_tc_workspace(*desc);
+  if (v == CUTB_VARIANT_GEMV_PLANES) need = qgemv_planes_workspace(*desc);
+  const uint64_t rows = v == CUTB_VARIANT_ROWS_MMA ? (qgemv_rows_supported(*desc) ? qgemv_rows_workspace(*desc) : 0)
+                                                   : (rows_instead(*desc, v) ? qgemv_rows_workspace(*desc) : 0);
+  return need > rows ? need : rows;
 }
 
 int cutb_qmatmul(const cutb_qmatmul_desc *desc, void *stream) {
   if (int rc = validate(desc)) return rc;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  const int v = select(*desc);
+  const int v = chosen(*desc);
   if ((desc->flags & CUTB_FLAG_GLU_PAIRS) && v != CUTB_VARIANT_GEMV_MMA && v != CUTB_VARIANT_GEMM_TC) {
     // (the mat-vec launcher refuses shapes that split K; the tensor-core GEMMs take every shape they support)
     set_last_error("qmatmul: paired gate/up rows exist in the decode mat-vec and the tensor-core GEMM only");
@@ -199,6 +214,16 @@ int cutb_qmatmul(const cutb_qmatmul_desc *desc, void *stream) {
         return CUTB_ERR_UNSUPPORTED;
       }
       return qgemv_planes_launch(*desc, s);
+    case CUTB_VARIANT_ROWS_MMA:
+      if (!qgemv_rows_supported(*desc)) {
+        set_last_error("qmatmul: variant %s needs GGUF blocks, K %% 256 == 0, 16-byte aligned W and 9 to 32 rows, without paired rows", cutb_variant_name(v));
+        return CUTB_ERR_UNSUPPORTED;
+      }
+      if (!qgemv_rows_fits(*desc)) {
+        set_last_error("qmatmul: variant %s needs %llu bytes of 16-byte aligned scratch", cutb_variant_name(v), (unsigned long long)qgemv_rows_workspace(*desc));
+        return CUTB_ERR_WORKSPACE;
+      }
+      return qgemv_rows_launch(*desc, s);
     default:
       return qmatmul_generic_launch(*desc, s);
   }

@@ -20,9 +20,10 @@ int qgemv_blocks_launch(const cutb_qmatmul_desc &d, cudaStream_t stream, const c
 // Publishes this rank's peer stores of the step and waits (bounded) for every rank's.
 int peer_exchange_launch(const cutb_peer_scatter &peers, uint64_t *step_counter, int *status, cudaStream_t stream);
 
-// Matmul of 9 to 32 activation rows, as fp16 MMAs over GGUF blocks (qgemv_rows.cu); reached through qgemv_blocks_* and qgemm_tc_*
-// where the caller's workspace holds what it needs (qgemv_rows_fits).
-bool qgemv_rows_applies(const cutb_qmatmul_desc &d);
+// Matmul of 9 to 32 activation rows, as fp16 MMAs over GGUF blocks (qgemv_rows.cu).  qgemv_rows_faster: of the shapes that it takes,
+// those where it beats the other kernels.  It runs only where the caller's workspace holds what it needs (qgemv_rows_fits).
+bool qgemv_rows_supported(const cutb_qmatmul_desc &d);
+bool qgemv_rows_faster(const cutb_qmatmul_desc &d);
 uint64_t qgemv_rows_workspace(const cutb_qmatmul_desc &d);
 bool qgemv_rows_fits(const cutb_qmatmul_desc &d);
 int qgemv_rows_launch(const cutb_qmatmul_desc &d, cudaStream_t stream);

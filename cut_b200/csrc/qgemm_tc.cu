@@ -452,10 +452,7 @@ uint64_t tc_cast_bytes(const cutb_qmatmul_desc &d) {
 }  // namespace
 
 uint64_t qgemm_tc_workspace(const cutb_qmatmul_desc &d) {
-  if (qgemm_skinny_applies(d)) {
-    const uint64_t need = qgemm_skinny_workspace(d), rows = qgemv_rows_applies(d) ? qgemv_rows_workspace(d) : 0;
-    return need > rows ? need : rows;
-  }
+  if (qgemm_skinny_applies(d)) return qgemm_skinny_workspace(d);
   // fp32 activations are rounded to fp16 rows of K elements first; a K split adds its planes of partial sums
   DeviceInfo di;
   const uint32_t sms = get_device_info(&di) == CUTB_OK ? (uint32_t)di.sm_count : 148u;
@@ -465,7 +462,6 @@ uint64_t qgemm_tc_workspace(const cutb_qmatmul_desc &d) {
 }
 
 int qgemm_tc_launch(const cutb_qmatmul_desc &d, cudaStream_t stream) {
-  if (qgemv_rows_applies(d) && qgemv_rows_fits(d)) return qgemv_rows_launch(d, stream);
   if (qgemm_skinny_applies(d)) return qgemm_skinny_launch(d, stream);
   DeviceInfo di;
   if (int rc = get_device_info(&di)) return rc;

@@ -1214,9 +1214,6 @@ bool qgemv_blocks_supported_in_groups(const cutb_qmatmul_desc &d) {
   return d.M <= 4 * qgemv_rows_per_group(d) && qgemv_blocks_supported(one) && !(d.flags & CUTB_FLAG_GLU_PAIRS);
 }
 
-// nine fp16 rows and more: as fp16 MMAs (the same exact weights and more of the activations' bits than the digits hold)
-static bool gv_as_rows(const cutb_qmatmul_desc &d) { return d.a_dtype == CUTB_F16 && d.M <= 16 && qgemv_rows_applies(d); }
-
 uint64_t qgemv_blocks_workspace(const cutb_qmatmul_desc &d) {
   const uint32_t per = qgemv_rows_per_group(d);
   if (d.M > per && qgemv_blocks_supported_in_groups(d)) {  // the groups run one after the other on one scratch block
@@ -1232,8 +1229,7 @@ uint64_t qgemv_blocks_workspace(const cutb_qmatmul_desc &d) {
   }
   GvPlan pl;
   if (!qgemv_blocks_supported(d) || !gv_plan(d, di, &pl)) return 0;
-  const uint64_t need = gv_workspace_need(pl), rows = gv_as_rows(d) ? qgemv_rows_workspace(d) : 0;
-  return need > rows ? need : rows;
+  return gv_workspace_need(pl);
 }
 
 int qgemv_blocks_launch(const cutb_qmatmul_desc &d, cudaStream_t stream, const cutb_peer_scatter *sc) {
@@ -1250,7 +1246,6 @@ int qgemv_blocks_launch(const cutb_qmatmul_desc &d, cudaStream_t stream, const c
     }
     return CUTB_OK;
   }
-  if (!sc && gv_as_rows(d) && qgemv_rows_fits(d)) return qgemv_rows_launch(d, stream);
   DeviceInfo di;
   if (int rc = get_device_info(&di)) return rc;
   GvPlan pl;

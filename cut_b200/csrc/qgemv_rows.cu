@@ -499,6 +499,12 @@ template <int FMT> int gr_dispatch(const cutb_qmatmul_desc &d, const GrParams &p
 
 }  // namespace
 
+bool qgemv_rows_supported(const cutb_qmatmul_desc &d) {
+  if (d.layout != CUTB_LAYOUT_GGUF_BLOCKS || d.K == 0 || d.K % 256 != 0 || d.N == 0 || reinterpret_cast<uintptr_t>(d.W) % 16 != 0) return false;
+  if (d.flags & (CUTB_FLAG_A_RMSNORM | CUTB_FLAG_GLU_PAIRS | CUTB_FLAG_STAGE_PER_CTA)) return false;
+  return d.M >= 9 && d.M <= 32;
+}
+
 // Where this kernel is the faster one, us per call in a chain (int8 mat-vec or tcgen05 GEMM for few tokens -> this):
 //   9 to 16 rows   fp16, 12 rows, 4096 x 4096 / 4096 x 11008 / 8192 x 8192 / 1024 x 1000: Q4_0 11.8 -> 10.1 / 19.7 -> 16.8 / 26.3 -> 21.8 /
 //                  7.2 -> 6.4, Q8_0 14.3 -> 10.3 / 26.0 -> 16.5 / 33.6 -> 21.8 / 7.0 -> 6.4; Q4_K the same within 4 % either way (its
@@ -507,10 +513,7 @@ template <int FMT> int gr_dispatch(const cutb_qmatmul_desc &d, const GrParams &p
 //                  7.6 -> 8.5, 14336 x 4096 25.5 -> 26.3; Q4_K 13.8 -> 14.3 / 23.4 -> 23.7: stays
 //   fp32 rows      (rounded to fp16 above eight rows by either kernel; here in the same pass that orders them) 9 rows: Q4_0 17.2 -> 10.0 /
 //                  25.5 -> 16.7 / 31.4 -> 21.6 / 11.2 -> 6.5; 32 rows: Q4_K 19.6 -> 14.4 / 27.4 -> 23.8 / 33.3 -> 32 / 12.0 -> 8.6
-bool qgemv_rows_applies(const cutb_qmatmul_desc &d) {
-  if (d.layout != CUTB_LAYOUT_GGUF_BLOCKS || d.K == 0 || d.K % 256 != 0 || d.N == 0 || reinterpret_cast<uintptr_t>(d.W) % 16 != 0) return false;
-  if (d.flags & (CUTB_FLAG_A_RMSNORM | CUTB_FLAG_GLU_PAIRS | CUTB_FLAG_STAGE_PER_CTA)) return false;
-  if (d.M < 9 || d.M > 32 || d.variant != CUTB_VARIANT_AUTO) return false;  // (a caller that names a kernel gets that one)
+bool qgemv_rows_faster(const cutb_qmatmul_desc &d) {
   if (d.a_dtype == CUTB_F32 || (d.M <= 16 && d.format != CUTB_Q4_K)) return true;
   const uint64_t weights = (uint64_t)d.K * d.N;
   return d.M > 16 && ((d.format == CUTB_Q8_0 && weights >= (1ull << 23)) || (d.format == CUTB_Q4_0 && weights >= (1ull << 24) && d.K <= 8192));

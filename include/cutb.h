@@ -72,7 +72,7 @@ enum { CUTB_FUSION_NONE = 0, CUTB_FUSION_UNARY = 1, CUTB_FUSION_BINARY = 2 };
 
 /* Kernel variants of cutb_qmatmul (variant = -1 lets the library choose). */
 enum {
-  CUTB_VARIANT_AUTO = -1, /* (9 to 32 rows over GGUF blocks may run as fp16 warp MMAs under either name below) */
+  CUTB_VARIANT_AUTO = -1,
   CUTB_VARIANT_GENERIC = 0, /* any shape, SIMT, exact fp32 dequant + FMA */
   CUTB_VARIANT_GEMV_MMA = 1, /* decode: bulk-copy ring + int8 warp MMA, M <= 16 (fp16 A) / 8 (fp32 A); when forced, up to
                                 four such row groups one after the other (M <= 64 / 32): faster than the GEMM on narrow
@@ -80,8 +80,11 @@ enum {
   CUTB_VARIANT_GEMM_TC = 2, /* prefill: tcgen05 tensor-core GEMM, accumulators in tensor memory; its operands are fp16
                                (see the operand-range note at cutb_qmatmul_desc).  GGUF blocks (K % 256 == 0) and
                                CUTB_LAYOUT_KN_PLANES (K % 128 == 0; above four rows what CUTB_VARIANT_AUTO picks there) */
-  CUTB_VARIANT_GEMV_PLANES = 3 /* decode over CUTB_LAYOUT_KN_PLANES (the reference's run-time layout), M <= 4: coalesced
-                                  column groups, K split over warps and blocks */
+  CUTB_VARIANT_GEMV_PLANES = 3, /* decode over CUTB_LAYOUT_KN_PLANES (the reference's run-time layout), M <= 4: coalesced
+                                   column groups, K split over warps and blocks */
+  CUTB_VARIANT_ROWS_MMA = 4 /* batched decode: fp16 warp MMAs on the quants of GGUF blocks (K % 256 == 0), 9 <= M <= 32, operands as
+                               CUTB_VARIANT_GEMM_TC rounds them (up to 16 rows the weights are exact); needs the scratch of
+                               cutb_qmatmul_workspace_bytes.  What CUTB_VARIANT_AUTO picks where it measured faster */
 };
 
 /* Descriptor flags.
@@ -176,8 +179,8 @@ typedef struct cutb_qmatmul_desc {
  * planes of partial sums of a K split (same rule: optional, faster with them). */
 CUTB_API uint64_t cutb_qmatmul_workspace_bytes(const cutb_qmatmul_desc *desc);
 
-/* Variant the library would run for this descriptor (resolves CUTB_VARIANT_AUTO);
- * negative on an invalid descriptor.  Mirrors the variant choice made in the
+/* Variant the library would run for this descriptor (resolves CUTB_VARIANT_AUTO, which may pick another kernel without scratch than
+ * with it); negative on an invalid descriptor.  Mirrors the variant choice made in the
  * MatMulOpNode constructor (operators/impl/matmul/MatMulOp.cpp:335-380). */
 CUTB_API int cutb_qmatmul_select_variant(const cutb_qmatmul_desc *desc);
 

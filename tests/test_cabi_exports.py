@@ -122,3 +122,36 @@ def test_select_variant_and_workspace_plan_without_device():
     d.flags = 0
     assert lib.cutb_qmatmul_workspace_bytes(C.byref(d)) > ws
     assert lib.cutb_qmatmul_workspace_bytes(C.byref(desc(L.Q4_0, 2, 4096, 11008))) == 0
+
+
+def test_rows_kernel_has_a_name_and_is_named_where_it_runs():
+    """9 to 32 rows over blocks: with the scratch that the query asks for the choice is QGemvRowsMma, without it the former kernel, and a
+    caller may name any of them; shapes that the kernel does not take are refused."""
+    lib = L.lib()
+
+    def desc(M, variant=L.VARIANT_AUTO, flags=0, fmt=L.Q4_0, dtype=L.F16, scratch=True):
+        d = L.QMatmulDesc()
+        d.format, d.layout, d.a_dtype, d.variant, d.flags = fmt, L.LAYOUT_GGUF_BLOCKS, dtype, variant, flags
+        d.M, d.K, d.N, d.lda, d.ldc = M, 4096, 11008, 4096, 11008
+        d.A = d.W = d.C = 256  # never dereferenced here
+        d.W_bytes = 1 << 40
+        if scratch:
+            d.workspace, d.workspace_bytes = 256, lib.cutb_qmatmul_workspace_bytes(C.byref(d))
+        return d
+
+    chosen = lambda d: lib.cutb_qmatmul_select_variant(C.byref(d))
+    assert lib.cutb_variant_name(L.VARIANT_ROWS_MMA) == b"QGemvRowsMma"
+    for M, dtype, former in ((9, L.F16, L.VARIANT_GEMV_MMA), (16, L.F16, L.VARIANT_GEMM_TC), (32, L.F16, L.VARIANT_GEMM_TC), (9, L.F32, L.VARIANT_GEMM_TC)):
+        assert chosen(desc(M, dtype=dtype)) == L.VARIANT_ROWS_MMA
+        assert chosen(desc(M, dtype=dtype, scratch=False)) == former
+        assert chosen(desc(M, former, dtype=dtype)) == former
+        d = desc(M, dtype=dtype)
+        d.workspace_bytes -= 1
+        assert chosen(d) in (former, L.VARIANT_ROWS_MMA) and chosen(d) == (former if lib.cutb_qmatmul_workspace_bytes(C.byref(desc(M, L.VARIANT_ROWS_MMA, dtype=dtype))) > d.workspace_bytes else L.VARIANT_ROWS_MMA)
+    assert chosen(desc(8)) == L.VARIANT_GEMV_MMA and chosen(desc(33)) == L.VARIANT_GEMM_TC and chosen(desc(12, fmt=L.Q4_K)) == L.VARIANT_GEMV_MMA
+    assert chosen(desc(12, dtype=L.F32, flags=L.FLAG_ACT_16BIT)) == L.VARIANT_GEMV_MMA  # (the mat-vec keeps their range)
+    assert chosen(desc(12, L.VARIANT_ROWS_MMA)) == L.VARIANT_ROWS_MMA
+    for d in (desc(8, L.VARIANT_ROWS_MMA), desc(33, L.VARIANT_ROWS_MMA), desc(12, L.VARIANT_ROWS_MMA, L.FLAG_STAGE_PER_CTA)):
+        assert lib.cutb_qmatmul(C.byref(d), None) == L.ERR_UNSUPPORTED
+    assert lib.cutb_qmatmul(C.byref(desc(12, L.VARIANT_ROWS_MMA, scratch=False)), None) == L.ERR_WORKSPACE
+    assert chosen(desc(12, L.VARIANT_ROWS_MMA + 1)) < 0
