@@ -5,8 +5,10 @@
 //   warps 0-3, 4-7  softmax of the first and of the second token tile, one token per thread (= tensor-memory lane).  Scores come
 //                   by tcgen05.ld, the weights go back by tcgen05.st in the place of the scores: bf16 weights as the sum of two
 //                   terms (16 significant bits), high parts in the first 64 columns and low parts in the other 64; fp16 weights as
-//                   one term.  The running maximum is only followed when a score exceeds it by more than 2^8 (weights stay
-//                   below 2^8, sums are fp32): the weighted values are rescaled in tensor memory then, a rare event.
+//                   one term.  The running maximum is followed tile by tile, and the weighted values are rescaled in tensor memory
+//                   when it rises: the largest weight is an exact 1 then.  Following it only past 2^8 was 2 to 9 % faster (32 heads,
+//                   1500 tokens 46.9 against 47.7 us; 8 heads, 256 tokens behind 4000 82 against 91), but the error against 64 bits
+//                   was up to 3.4 times (fp16) and 1.3 times (bf16) that of the kernels before; now 1.00 to 1.07 times.
 //   warp 8          one lane copies the key and value tiles by TMA (boxes of 64 columns x 64 rows, 128-byte swizzle); columns past
 //                   a head's elements and rows past the tensor read as zero.
 //   warp 9          one lane issues the products: scores = Q K^T from shared memory, then weights (tensor memory, the A operand)
@@ -507,27 +509,27 @@ __global__ void __launch_bounds__(PA_THREADS, 1)
             }
         }
         const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale;
-        if (__any_sync(0xffffffffu, mx > m + 8.f)) {  // (also the first keys seen: m is -infinity then)
+        if (done == 0) {  // nothing is summed yet
+          m = fmaxf(m, mx);
+        } else if (__any_sync(0xffffffffu, mx > m)) {
           const float mn = fmaxf(m, mx), f = mn == -INFINITY ? 1.f : pa_exp2(m - mn);
           m = mn, l *= f;
-          if (done) {
-            if (!warp_wait(odone + grp * 8, (done - 1) & 1u)) {
-              dead = true;
-              break;
-            }
-            tc_fence_after();
+          if (!warp_wait(odone + grp * 8, (done - 1) & 1u)) {
+            dead = true;
+            break;
+          }
+          tc_fence_after();
 #pragma unroll 1
-            for (uint32_t c = 0; c < VP * 64; c += 32) {
-              uint32_t o[32];
-              tmem_ld32_async(o_t + c, o);
-              tmem_wait32(o);
-              uint32_t a[16], b[16];
+          for (uint32_t c = 0; c < VP * 64; c += 32) {
+            uint32_t o[32];
+            tmem_ld32_async(o_t + c, o);
+            tmem_wait32(o);
+            uint32_t a[16], b[16];
 #pragma unroll
-              for (int i = 0; i < 16; ++i)
-                a[i] = __float_as_uint(__uint_as_float(o[i]) * f), b[i] = __float_as_uint(__uint_as_float(o[16 + i]) * f);
-              tmem_st16(o_t + c, a);
-              tmem_st16(o_t + c + 16, b);
-            }
+            for (int i = 0; i < 16; ++i)
+              a[i] = __float_as_uint(__uint_as_float(o[i]) * f), b[i] = __float_as_uint(__uint_as_float(o[16 + i]) * f);
+            tmem_st16(o_t + c, a);
+            tmem_st16(o_t + c + 16, b);
           }
         }
         const float ms = m == -INFINITY ? 0.f : m;  // nothing attended yet: keep exponents finite

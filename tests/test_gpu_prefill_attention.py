@@ -228,3 +228,33 @@ def test_values_that_are_not_finite(mode, T, pos, window):
     assert int(status.item()) == 0
     assert bool((got.isfinite() == finite).all()) and bool((got.isnan() == ref.isnan()).all()) and bool((got == ref)[ref.isinf()].all())
     assert _rel(got[finite], ref[finite]) <= (1e-3 if mode == "llama" else 1e-4)
+
+
+@pytest.mark.parametrize("mode", ["llama", "window", "latent"])
+@pytest.mark.parametrize("T,pos,sink", [(140, 200, None), (700, 130, None), (140, 200, 0.0)])
+def test_the_largest_weight_is_exact(mode, T, pos, sink):
+    """One key, behind the first key tile, has a value; its logit stands 0.5 to 8 (in powers of two) above the others', another height for
+    every token.  Its weight is 1 relative to the maximum, without rounding to 16 bits, so the output is that value times a quotient of
+    fp32 sums: exponentials to 2^-22 and their arguments (up to 8) to 2^-21, 1e-6 in all.  (Weights relative to an older maximum carry
+    2^-12 in fp16 and 2^-18 in two bf16 terms.)"""
+    import torch
+
+    if mode == "llama" and sink is not None:
+        pytest.skip("no sink on the llama path")
+    q, k, v = _inputs(mode, T, pos, T)
+    H, at, d = q.shape[1], torch.arange(pos, pos + T, device="cuda"), q.shape[2] - (64 if mode == "latent" else 0)
+    key = pos - 1
+    height = torch.linspace(0.5, 8.0, T, device="cuda").to(k.dtype).float()
+    q.zero_()
+    q[:, :, 0] = height[:, None]
+    k.zero_()
+    k[key, :, 0] = 1.0
+    v[:key], v[key + 1:] = 0.0, 0.0
+    scale = 0.6931472
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    sinks = None if sink is None else torch.full((H,), sink, device="cuda")
+    got = _attend(mode, q, k, v, pos, 1 << 20, scale, status, sinks)
+    ref = _reference(q.double(), k.double(), v.double(), float(torch.tensor(scale)), at, 1 << 30, None if sink is None else sinks.double())
+    assert int(status.item()) == 0
+    worst = ((got.double() - ref).norm(dim=2) / ref.norm(dim=2)).max()
+    assert float(worst) <= 1e-6
