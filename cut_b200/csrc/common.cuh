@@ -215,6 +215,10 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
 __device__ __forceinline__ bool mbar_wait_probe_first(uint32_t bar, uint32_t parity) {
   return mbar_test(bar, parity) || mbar_wait_bounded(bar, parity);
 }
+// A copy warp's last look at a stage before its block may end: short, since copies land in microseconds unless a launch has failed.
+__device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
+  if (!mbar_test(bar, parity)) (void)mbar_wait_bounded(bar, parity, 1u << 8);
+}
 // The same for a whole warp, with one answer for all of its lanes.  A phase may complete between two lanes' probes, so lanes that
 // decide for themselves can part before warp-wide work (MMAs, shuffles, votes), which then waits without a limit for the others.
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity) {

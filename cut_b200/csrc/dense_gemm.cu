@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1) dense_gemm_tc_kernel(const __gr
       for (uint32_t i = 0; i < S; ++i) {
         if (s == 0) s = S, ph ^= 1u;
         --s;
-        mbar_wait_bounded(full_u + s * 8, ph ^ 1u, 1u << 8);
+        mbar_drain(full_u + s * 8, ph ^ 1u);
       }
     }
     __syncwarp();

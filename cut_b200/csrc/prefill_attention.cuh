@@ -293,12 +293,12 @@ __global__ void __launch_bounds__(PA_THREADS, 1)
     for (uint32_t i = 0; i < SK; ++i) {
       if (sk == 0) sk = SK, pk ^= 1u;
       --sk;
-      mbar_wait_bounded(kfull + sk * 8, pk ^ 1u, 1u << 8);
+      mbar_drain(kfull + sk * 8, pk ^ 1u);
     }
     for (uint32_t i = 0; i < SV; ++i) {
       if (sv == 0) sv = SV, pv ^= 1u;
       --sv;
-      mbar_wait_bounded(vfull + sv * 8, pv ^ 1u, 1u << 8);
+      mbar_drain(vfull + sv * 8, pv ^ 1u);
     }
     __syncwarp();
   } else if (warp == 9) {

@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(sk_threads(FMT), 1)
       for (uint32_t i = 0; i < pending; ++i) {
         if (sa == 0) sa = SA, pa ^= 1u;
         --sa;
-        mbar_wait_bounded(fulla_u + sa * 8, pa ^ 1u, 1u << 10);
+        mbar_drain(fulla_u + sa * 8, pa ^ 1u);
       }
     }
     __syncwarp();
@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(sk_threads(FMT), 1)
         const uint32_t pending = issued < RS ? issued : RS;
         for (uint32_t i = 0; i < pending; ++i) {
           const uint32_t g = issued - 1 - i;
-          mbar_wait_bounded(rawfull_u + (g % RS) * 8, (g / RS) & 1u, 1u << 10);
+          mbar_drain(rawfull_u + (g % RS) * 8, (g / RS) & 1u);
         }
       }
       __syncwarp();

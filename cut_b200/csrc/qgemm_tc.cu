@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(tc_max_threads(FMT), 1) qgemm_tc_kernel(const 
       for (uint32_t i = 0; i < pending; ++i) {
         if (sa == 0) sa = SA, pa ^= 1u;
         --sa;
-        mbar_wait_bounded(fulla_u + sa * 8, pa ^ 1u, 1u << 10);
+        mbar_drain(fulla_u + sa * 8, pa ^ 1u);
       }
     }
     __syncwarp();

@@ -84,7 +84,7 @@ def test_copies_in_flight_are_waited_for_whoever_gives_up_and_when(path):
     """A copy warp that has issued everything may end before another warp gives up: its wait for copies does not hang on the flag."""
     with open(path) as f:
         text = _without_comments(f.read())
-    assert [c for c, start, end in _ifs(text) if "aborted()" in c and "mbar_wait_bounded" in text[start: end] and "tmem_ld" not in text[start: end]] == []
+    assert [c for c, start, end in _ifs(text) if "aborted()" in c and ("mbar_drain" in text[start: end] or "mbar_wait_bounded" in text[start: end]) and "tmem_ld" not in text[start: end]] == []
 
 
 def test_the_reading_finds_what_it_is_for():
