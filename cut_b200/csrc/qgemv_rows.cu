@@ -505,18 +505,31 @@ bool qgemv_rows_supported(const cutb_qmatmul_desc &d) {
   return d.M >= 9 && d.M <= 32;
 }
 
-// Where this kernel is the faster one, us per call in a chain (int8 mat-vec or tcgen05 GEMM for few tokens -> this):
-//   9 to 16 rows   fp16, 12 rows, 4096 x 4096 / 4096 x 11008 / 8192 x 8192 / 1024 x 1000: Q4_0 11.8 -> 10.1 / 19.7 -> 16.8 / 26.3 -> 21.8 /
-//                  7.2 -> 6.4, Q8_0 14.3 -> 10.3 / 26.0 -> 16.5 / 33.6 -> 21.8 / 7.0 -> 6.4; Q4_K the same within 4 % either way (its
-//                  minima cost a second product): stays.  Eight rows, which fill the int8 kernel's columns: 12.8 -> 14.3: stays.
-//   17 to 32 rows  fp16, 32 rows: Q8_0 16.5 -> 13.8 / 32.0 -> 22.1 / 42.1 -> 26.9 / 7.6 -> 8.4, Q4_0 13.9 -> 13.4 / 23.4 -> 21.5 / 28.9 -> 26.3 /
-//                  7.6 -> 8.5, 14336 x 4096 25.5 -> 26.3; Q4_K 13.8 -> 14.3 / 23.4 -> 23.7: stays
-//   fp32 rows      (rounded to fp16 above eight rows by either kernel; here in the same pass that orders them) 9 rows: Q4_0 17.2 -> 10.0 /
-//                  25.5 -> 16.7 / 31.4 -> 21.6 / 11.2 -> 6.5; 32 rows: Q4_K 19.6 -> 14.4 / 27.4 -> 23.8 / 33.3 -> 32 / 12.0 -> 8.6
+// Where this kernel is the faster one.  us per call in a chain, the kernel that runs otherwise (int8 mat-vec, or tcgen05 GEMM for few
+// tokens) -> this one; tiles: 128 weight rows each, units: tiles x K / 256.
+//   9 to 16 fp16 rows   From 20 tiles up always: 12 rows, 256 x 8192 10.5 -> 4.2, 2560 x 2560 Q4_0 x 0.79, 4096 x 4096 Q8_0 14.3 -> 10.3,
+//                  8192 x 8192 Q4_0 26.3 -> 21.8.  Fewer tiles are shared by many CTAs, whose meeting costs more than it gives until the
+//                  int8 kernel has to split K as well: 9 rows, 2048 x 2048 Q8_0 6.1 -> 7.7, 4608 x 2048 Q4_0 8.1 -> 10.3 and Q8_0 11.7 ->
+//                  10.4, 8192 x 512 8.3 -> 12.2, so from 8 tiles of 192 (Q8_0: 3072 x 2048 x 0.75) or 384 units (Q4_0: 6144 x 2048 12.1 ->
+//                  10.2; 16384 x 1024 alone loses 3 % up to 12 rows, and wins 25 % from 13); and where both are small, 1024 x 1000
+//                  7.2 -> 6.2, 2048 x 768 8.1 -> 7.1.  Q4_K the same within 4 % either way (its minima cost a second product): stays.
+//                  Eight rows, which fill the int8 kernel's columns: 12.8 -> 14.3: stays.
+//   17 to 32 fp16 rows  Q8_0 from 8 M weights on 24 tiles (3072 x 4096 x 0.84 to 0.88, 4096 x 3072 x 1.01) and 14 M weights on any (8192 x
+//                  1536 15.9 -> 17.0, 4096 x 2048 x 1.03; 14336 x 1024 x 0.85 to 0.92, 8192 x 8192 42 -> 27).  Q4_0 from 16 M weights on
+//                  48 tiles (4096 x 6144 x 0.93 to 0.98, 8192 x 8192 x 0.86, 28672 x 8192 72 -> 63), or 32 with K up to 4096 (4096 x 4096
+//                  x 0.92 to 0.97, but 6144 x 4096 x 0.99 to 1.04, 8192 x 4096 18.5 -> 20.3, 14336 x 4096 x 0.99 to 1.01, 16384 x 2048
+//                  19.4 -> 21.9).  Q4_K 4096 x 4096 x 1.03, 11008 x 4096 x 1.06: stays.
+//   fp32 rows      Rounded to fp16 by either kernel; here in the same pass that orders them.  All three formats gain on all of 35 weights
+//                  from 512 x 512 to 28672 x 8192: x 0.44 to 0.94 (9 and 16 rows), x 0.48 to 0.98 (17 to 32 rows, 8192 x 512 x 1.01).
 bool qgemv_rows_faster(const cutb_qmatmul_desc &d) {
-  if (d.a_dtype == CUTB_F32 || (d.M <= 16 && d.format != CUTB_Q4_K)) return true;
-  const uint64_t weights = (uint64_t)d.K * d.N;
-  return d.M > 16 && ((d.format == CUTB_Q8_0 && weights >= (1ull << 23)) || (d.format == CUTB_Q4_0 && weights >= (1ull << 24) && d.K <= 8192));
+  if (d.a_dtype == CUTB_F32) return true;
+  if (d.format == CUTB_Q4_K) return false;
+  const uint32_t tiles = (d.N + GR_ROWS - 1) / GR_ROWS;
+  const uint64_t weights = (uint64_t)d.K * d.N, units = (uint64_t)tiles * (d.K / 256);
+  const bool q8 = d.format == CUTB_Q8_0;
+  if (d.M <= 16) return tiles >= 20 || (tiles >= 8 && units >= (q8 ? 192u : 384u)) || (tiles <= 8 && d.K <= 2048);
+  if (q8) return weights >= (14ull << 20) || (weights >= (8ull << 20) && tiles >= 24);
+  return weights >= (16ull << 20) && (tiles >= 48 || (tiles >= 32 && d.K <= 4096));
 }
 
 uint64_t qgemv_rows_workspace(const cutb_qmatmul_desc &d) {

@@ -155,3 +155,28 @@ def test_rows_kernel_has_a_name_and_is_named_where_it_runs():
         assert lib.cutb_qmatmul(C.byref(d), None) == L.ERR_UNSUPPORTED
     assert lib.cutb_qmatmul(C.byref(desc(12, L.VARIANT_ROWS_MMA, scratch=False)), None) == L.ERR_WORKSPACE
     assert chosen(desc(12, L.VARIANT_ROWS_MMA + 1)) < 0
+
+
+def test_rows_kernel_runs_where_it_measured_faster():
+    """The line between the row kernel and the former ones, at shapes on both of its sides."""
+    lib = L.lib()
+
+    def rows(fmt, M, K, N, dtype=L.F16):
+        d = L.QMatmulDesc()
+        d.format, d.layout, d.a_dtype, d.variant = fmt, L.LAYOUT_GGUF_BLOCKS, dtype, L.VARIANT_AUTO
+        d.M, d.K, d.N, d.lda, d.ldc = M, K, N, K, N
+        d.A = d.W = d.C = d.workspace = 256  # never dereferenced here
+        d.W_bytes, d.workspace_bytes = 1 << 40, 1 << 40
+        return lib.cutb_qmatmul_select_variant(C.byref(d)) == L.VARIANT_ROWS_MMA
+
+    for M in (9, 16):  # the int8 mat-vec was up to 1.5 times as fast on these
+        assert not any(rows(f, M, K, N) for f in (L.Q8_0, L.Q4_0) for K, N in ((2048, 2048), (512, 2048), (1536, 1536), (8192, 512), (4096, 1024), (28672, 512)))
+        assert all(rows(f, M, K, N) for f in (L.Q8_0, L.Q4_0) for K, N in ((1024, 1000), (512, 8192), (2560, 2560), (6144, 2048), (8192, 8192), (28672, 1024)))
+        assert rows(L.Q8_0, M, 3072, 2048) and not rows(L.Q4_0, M, 3072, 2048) and not rows(L.Q4_0, M, 4608, 2048)
+    for M in (17, 32):
+        assert not any(rows(L.Q8_0, M, K, N) for K, N in ((4096, 2048), (8192, 1536), (2048, 2048)))
+        assert all(rows(L.Q8_0, M, K, N) for K, N in ((3072, 4096), (14336, 1024), (8192, 8192)))
+        assert not any(rows(L.Q4_0, M, K, N) for K, N in ((8192, 4096), (8192, 2048), (14336, 4096), (16384, 2048), (2048, 4096)))
+        assert all(rows(L.Q4_0, M, K, N) for K, N in ((4096, 4096), (4096, 6144), (8192, 8192), (14336, 8192)))
+    assert not any(rows(L.Q4_K, M, 8192, 8192) for M in (9, 16, 17, 32))
+    assert all(rows(f, M, K, N, L.F32) for f in (L.Q8_0, L.Q4_0, L.Q4_K) for M in (9, 32) for K, N in ((512, 512), (2048, 2048), (14336, 4096)))
