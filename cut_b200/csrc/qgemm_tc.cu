@@ -35,7 +35,7 @@
 //               = token), fused op, stores to C coalesced along n.
 // fp32 activations are first rounded to fp16 into the caller's workspace by a
 // small cast kernel (the copy engine cannot convert).  Shared memory holds a ring
-// of activation stages (three at 512 tokens) and a ring of two weight tiles (three up to 256 tokens per CTA).
+// of activation stages (three at 512 tokens) and a ring of two or three weight tiles.
 //
 // Every wait is bounded; on expiry the CTA records CUTB_ERR_TIMEOUT in the
 // caller's status word, skips its remaining work, frees its tensor memory and
@@ -49,7 +49,7 @@ namespace cutb {
 namespace {
 
 template <int FMT>
-__global__ void __launch_bounds__(tc_max_threads(FMT), 1) qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmapA, const TcParams p) {
+__global__ void __launch_bounds__(TC_MAX_THREADS, 1) qgemm_tc_kernel(const __grid_constant__ CUtensorMap tmapA, const TcParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // tiles must start on a 1024-byte boundary (the 128-byte swizzle repeats every 8 rows)
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -422,16 +422,18 @@ namespace {
 // to eight MMA issues take the issuer: stages of 128 k halve the waits per k, and shared memory has room for them there.
 uint32_t tc_ksub(uint32_t mb) { return mb <= 2 ? 2u : 1u; }
 
-// Token blocks per CTA and K split, by an estimate of the time (us) that follows measurements on all the shapes below within
-// a tenth: a 64-k stage of a CTA, the CTA's start and epilogue, and for a split the planes of partial sums through L2 and a second
-// launch.  A stage costs almost the same for one to three token blocks (dequantising 128 weight rows sets the pace; with four it is
-// the activations through L2), so few large CTAs with their K shared out beat many small ones.  Rule before (token blocks only,
-// K split only for 512 tokens and K >= 8192) -> now, us:  333 x 11008 x 4096 Q8_0 111 -> 50 (3 blocks, 4 shares);
-// 512 x 4096 x 4096 Q4_K 37.9 -> 29.2 (4, 4);  512 x 4096 x 6144 42.5 -> 37.4 (4, 3);  200 x 4096 x 4096 Q4_0 36.4 -> 21.0 (2, 4);
-// 256 x 8192 x 8192 68.6 -> 52.2 (2, 2);  400 x 2048 x 2048 21.5 -> 15.9 (2, 4);  1500 x 4096 x 4096 Q8_0 63.0 -> 55.3 (3, 1);
-// unchanged: 512 x 14336 x 4096 (4, 4), 512 x 4096 x 14336 and x 28672 (4, 1), 2048 x 4096 x 11008 (4, 1).
+// Token blocks per CTA and K split, by an estimate of the time (us): a 64-k stage of a CTA, the CTA's start and epilogue, and for a
+// split the planes of partial sums through L2 and a second launch.  A stage of Q8_0 costs almost the same for one to three token blocks
+// (its bytes set the pace), one of the 4-bit formats more with three, and with four it is the activations through L2; so few large CTAs
+// with their K shared out beat many small ones.  On 22 shapes of the three formats with every plan of each timed (fp16 activations: the
+// cast of fp32 ones costs the same in all) the estimate of the chosen plan is within 11 %, and the chosen plan is the fastest of all
+// with partial sums and of those without, but for one (Q4_K 527 x 8192 x 2048 32.5, best 31.1).  us, one block and K whole as plans for
+// few rows were -> now: Q8_0 333 x 11008 x 4096 94 -> 40 (3 blocks, 4 shares), 256 x 8192 x 8192 82 -> 54 (2, 2), 150 x 4096 x 4096 42 ->
+// 20 (2, 4); Q4_K 512 x 4096 x 4096 34 -> 28 (2, 2), 1500 x 4096 x 4096 92 -> 48 (3, 1); Q4_0 200 x 4096 x 4096 33 -> 19 (2, 4).
 void tc_shape_plan(const cutb_qmatmul_desc &d, uint32_t sm_count, bool split, uint32_t *mb_out, uint32_t *ksplit_out) {
-  static const float stage[TC_MAX_MB] = {0.58f, 0.56f, 0.65f, 0.71f}, fixed[TC_MAX_MB] = {6.f, 8.f, 9.f, 11.f};
+  static const struct { float stage[TC_MAX_MB], fixed[TC_MAX_MB]; } q8 = {{0.555f, 0.57f, 0.63f, 0.71f}, {6.f, 8.f, 9.f, 10.f}},
+      q4 = {{0.41f, 0.45f, 0.59f, 0.69f}, {6.f, 8.f, 9.f, 10.f}}, planes = {{0.58f, 0.56f, 0.65f, 0.71f}, {6.f, 8.f, 9.f, 11.f}};
+  const auto &cost = d.layout == CUTB_LAYOUT_KN_PLANES ? planes : (d.format == CUTB_Q8_0 ? q8 : q4);
   const uint32_t mblocks = (d.M + TC_BT - 1) / TC_BT, ctiles = (d.N + TC_BW - 1) / TC_BW;
   float best = 1e30f;
   for (uint32_t mb = mblocks < TC_MAX_MB ? mblocks : TC_MAX_MB; mb >= 1; --mb) {
@@ -440,7 +442,7 @@ void tc_shape_plan(const cutb_qmatmul_desc &d, uint32_t sm_count, bool split, ui
       const uint32_t per = (nk + want - 1) / want, ks = (nk + per - 1) / per;  // no empty share
       const uint64_t ctas = (uint64_t)ctiles * ((mblocks + mb - 1) / mb) * ks;
       const float waves = (float)((ctas + sm_count - 1) / sm_count);
-      float t = waves * (fixed[mb - 1] + (float)(per * ksub) * stage[mb - 1]);
+      float t = waves * (cost.fixed[mb - 1] + (float)(per * ksub) * cost.stage[mb - 1]);
       if (ks > 1) t += 2.f + (float)ks * (float)d.M * (float)d.N * (4.f / 6.6e6f);
       if (t < best) best = t, *mb_out = mb, *ksplit_out = ks;
     }
@@ -494,14 +496,17 @@ int qgemm_tc_launch(const cutb_qmatmul_desc &d, cudaStream_t stream) {
       p.partial = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(d.workspace) + cast_bytes);
     }
   }
-  // Weight slots, one per converter group: three where a stage's weights set the pace and shared memory has room (128 tokens:
-  // stages of 128 k; 384 tokens: 333 x 11008 x 4096 56 -> 50 us), two at 256 and 512 tokens (a third one costs an activation
-  // stage there: 512 x 4096 x 14336 62 -> 70 us); the rest of shared memory holds activation stages in flight.
-  p.nb = p.mb == 1 || p.mb == 3 ? 3 : 2;
-  p.groups = d.layout == CUTB_LAYOUT_KN_PLANES ? 2 : p.nb;
+  // Weight slots, the rest of shared memory holding activation stages in flight.  A third one loosens the hand-over converter -> issuer ->
+  // tensor core -> converter (us, two / three: one block, Q8_0 297 x 14336 x 4096 141 / 130, Q4_K 111 / 99; two blocks, Q4_0 235 x 5120 x
+  // 11008 48.9 / 43.4, Q8_0 180 x 14336 x 8192 in two shares 86.6 / 81.4), but costs activation stages, which short shares of two
+  // blocks feel (Q8_0 129 x 11008 x 4096 in four shares, 22 stages: 36.1 / 37.2, 150 x 4096 x 4096, 8 stages: 19.7 / 20.7; Q4_K 147 x
+  // 8192 x 11008 in three, 22 stages: 60.7 / 58.5), and with four blocks the third of three (512 x 4096 x 14336 62 / 70).
+  p.ksub = tc_ksub(p.mb);
+  const uint32_t nk = d.K / (TC_BK * p.ksub), stages = (nk + p.ksplit - 1) / p.ksplit;
+  p.nb = p.mb == 4 || (p.mb == 2 && stages < (d.format == CUTB_Q8_0 ? 28u : 16u)) ? 2 : 3;
+  p.groups = TC_MAX_GROUPS;
   p.issuers = 2;
   if (p.issuers > (p.mb + 1) / 2) p.issuers = (p.mb + 1) / 2;
-  p.ksub = tc_ksub(p.mb);
   p.sa = 0;
   for (uint32_t sa = 6; sa >= 2; --sa)
     if (tc_smem_bytes(p.mb, sa, p.nb, p.ksub) <= di.smem_optin) {

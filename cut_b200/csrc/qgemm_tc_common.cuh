@@ -50,10 +50,11 @@ struct TcParams {
 // and the same with per-block mins behind the scales (the runner's affine re-encode of Q4_K).
 constexpr int TC_PLANE_Q8 = 100, TC_PLANE_Q4 = 101, TC_PLANE_Q4A = 102;
 __host__ __device__ constexpr bool tc_is_plane(int fmt) { return fmt >= TC_PLANE_Q8; }
-// Converter groups of 128 threads; group g dequantises K stages g, g + G, ...  More than three groups slow one another down
-// (333 x 11008 x 4096 Q8_0: 50 us with three, 61 with four).  The plane formats' converters need the register file of two.
-__host__ __device__ constexpr int tc_max_groups(int fmt) { return tc_is_plane(fmt) ? 2 : 3; }
-__host__ __device__ constexpr int tc_max_threads(int fmt) { return TC_CTRL_THREADS + 128 * tc_max_groups(fmt); }
+// Converter groups of 128 threads; group g dequantises K stages g, g + G, ...  More groups slow one another down, two against three
+// in us: Q8_0 297 x 14336 x 4096 with one token block 129 / 138, 333 x 11008 x 4096 with three and four shares of K 40.5 / 41.2,
+// 150 x 4096 x 4096 42 / 45; Q4_0 96 / 98, 38.4 / 39.4, 33.0 / 34.4; Q4_K 99 / 102, 38.9 / 39.4, 34.1 / 35.6.
+constexpr int TC_MAX_GROUPS = 2;
+constexpr int TC_MAX_THREADS = TC_CTRL_THREADS + 128 * TC_MAX_GROUPS;
 
 // Byte offset of 16-byte chunk `c` (0..7) of row `r` inside a swizzled tile.
 __device__ __forceinline__ uint32_t sw128(uint32_t r, uint32_t c) { return r * 128u + ((c ^ (r & 7u)) << 4); }
