@@ -19,6 +19,8 @@
 // Copies in flight are waited for (bounded; a pair's by its first CTA, before the two part), tensor memory is freed.
 //
 // dense_gemm_simt_kernel: fp32 fused multiply-adds (bf16 weights are exact in fp32), for the true 32-bit mode.
+#include <algorithm>
+
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -487,9 +489,10 @@ uint32_t dg_pairs() {
 // (all there was) -> now, us: 2048 x 4096 x 14336 181 -> 156 (pairs x 224), x 12288 177 -> 138 (224), x 6144 111 -> 80 (192),
 // x 4096 65 -> 54 (256), 2048 x 14336 x 4096 186 -> 170 (256), 1501 x 4096 x 4096 59 -> 43 (192), 512 x 4096 x 14336 62 -> 50 (224);
 // 2048 x 1024 x 2048 stays (16.9 against 19.0: the pair's start).  `row_tiles`: row tiles of a given height, as they are likely to fall.
-template <class Tiles> void dg_width(uint32_t N, uint32_t nk, uint32_t sms, uint32_t pairs, Tiles row_tiles, DgPlan *pl) {
+// Grouped: 240 rows gain nothing over 256 (16 experts of 200 tokens x 4: 98 against 97 us).
+template <class Tiles> void dg_width(uint32_t N, uint32_t nk, uint32_t sms, uint32_t pairs, bool grouped, Tiles row_tiles, DgPlan *pl) {
   static const struct { uint32_t bn, cost; } one[] = {{256, 140}, {240, 138}, {224, 125}, {208, 122}, {192, 112}, {128, 97}, {64, 90}},
-                                             two[] = {{256, 120}, {224, 100}, {192, 92}, {160, 90}, {128, 86}};
+                                             two[] = {{256, 116}, {224, 100}, {192, 92}, {160, 90}, {128, 86}};
   constexpr uint64_t PAIR_START = 570;
   uint64_t best = ~0ull;
   auto consider = [&](uint32_t bn, uint32_t cost, bool pair) {
@@ -497,7 +500,8 @@ template <class Tiles> void dg_width(uint32_t N, uint32_t nk, uint32_t sms, uint
     const uint64_t t = (((uint64_t)tm * tn + workers - 1) / workers) * nk * cost + (pair ? PAIR_START : 0);
     if (t < best) best = t, pl->bn = bn, pl->tiles_m = tm, pl->tiles_n = tn, pl->pair = pair;
   };
-  for (const auto &k : one) consider(k.bn, k.cost, false);
+  for (const auto &k : one)
+    if (!grouped || k.bn != 240) consider(k.bn, k.cost, false);
   if (pairs)
     for (const auto &k : two) consider(k.bn, k.cost, true);
 }
@@ -506,7 +510,7 @@ DgPlan dg_plan(const cutb_dense_desc &d, uint32_t sms) {
   DgPlan b{};
   const uint32_t tm = (d.M + DG_BM - 1) / DG_BM;
   b.nk = (d.K + DG_BK - 1) / DG_BK;
-  dg_width(d.N, b.nk, sms, d.M > DG_BM ? dg_pairs() : 0, [&](uint32_t rows) { return (d.M + rows - 1) / rows; }, &b);
+  dg_width(d.N, b.nk, sms, d.M > DG_BM ? dg_pairs() : 0, false, [&](uint32_t rows) { return (d.M + rows - 1) / rows; }, &b);
   if (tm * ((d.N + 127) / 128) * 2 <= sms && b.nk >= 16) {
     b.bn = 128, b.pair = false, b.tiles_m = tm;
     b.tiles_n = (d.N + 127) / 128;
@@ -595,10 +599,13 @@ int moe_gemm_tc_launch(const cutb_moe_desc &d, cudaStream_t stream) {
   p.c_bf16 = d.c_dtype == CUTB_BF16;
   p.nk = p.nk_per = (d.K + DG_BK - 1) / DG_BK, p.ksplit = 1;
   p.a_box_rows = rows >= DG_BM ? DG_BM : (rows + 7) / 8 * 8;
-  // row tiles: every expert in use ends in a part-filled one
+  // Row tiles: an expert in use has one at least, and ends in a part-filled one, half of a tile on average.  (Counted as rows / n +
+  // used / 2, pairs seemed to halve the tiles of experts with less than a tile each, and the last wave went uncounted.)  us, counted so
+  // -> now, beside single CTAs x 256 rows: 16 experts, 1501 tokens x 4, 4096 -> 2 x 2048 gated 215 -> 189 (189), 200 tokens x 4 110 -> 97
+  // (97), 8 experts, 700 tokens x 2, 1024 -> 2 x 1024 21.5 -> 14.8 (14.8), 2000 tokens x 4, 2560 -> 2 x 2048 130 -> 126 (138).
   const uint32_t used = d.experts < rows ? d.experts : rows;
   DgPlan pl{};
-  dg_width(d.N, p.nk, sms, rows > DG_BM ? dg_pairs() : 0, [&](uint32_t n) { return rows / n + (used + 1) / 2; }, &pl);
+  dg_width(d.N, p.nk, sms, rows > DG_BM ? dg_pairs() : 0, true, [&](uint32_t n) { return std::max(used, (2 * rows + used * n + 2 * n - 1) / (2 * n)); }, &pl);
   p.tiles_m = rows / (pl.pair ? 2 * DG_BM : DG_BM) + used, p.tiles_n = pl.tiles_n;
   CUtensorMap ma, mw;
   if (int rc = make_tmap_sw128(&ma, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, d.A, rows, d.K, d.lda * 2, p.a_box_rows)) return rc;
