@@ -180,3 +180,18 @@ def test_rows_kernel_runs_where_it_measured_faster():
         assert all(rows(L.Q4_0, M, K, N) for K, N in ((4096, 4096), (4096, 6144), (8192, 8192), (14336, 8192)))
     assert not any(rows(L.Q4_K, M, 8192, 8192) for M in (9, 16, 17, 32))
     assert all(rows(f, M, K, N, L.F32) for f in (L.Q8_0, L.Q4_0, L.Q4_K) for M in (9, 32) for K, N in ((512, 512), (2048, 2048), (14336, 4096)))
+
+
+def test_prompt_gemm_shares_k_where_it_measured_faster():
+    """Planes of partial sums that the prompt GEMM asks for: the shares of K of the plan that was the fastest of all on 148
+    multiprocessors."""
+    lib = L.lib()
+    for fmt, M, K, N, shares in ((L.Q8_0, 333, 11008, 4096, 4), (L.Q8_0, 256, 8192, 8192, 2), (L.Q8_0, 150, 4096, 4096, 4), (L.Q8_0, 700, 2048, 6144, 1),
+                                 (L.Q4_K, 512, 4096, 4096, 2), (L.Q4_K, 512, 14336, 4096, 4), (L.Q4_K, 1500, 4096, 4096, 1), (L.Q4_0, 200, 4096, 4096, 4),
+                                 (L.Q4_0, 1092, 11008, 1024, 6), (L.Q4_0, 235, 5120, 11008, 1), (L.Q4_0, 400, 4096, 11008, 1)):
+        d = L.QMatmulDesc()
+        d.format, d.layout, d.a_dtype, d.variant = fmt, L.LAYOUT_GGUF_BLOCKS, L.F16, L.VARIANT_AUTO
+        d.M, d.K, d.N, d.lda, d.ldc = M, K, N, K, N
+        d.A = d.W = d.C = 256  # never dereferenced here
+        d.W_bytes = 1 << 40
+        assert lib.cutb_qmatmul_workspace_bytes(C.byref(d)) == (shares * M * N * 4 if shares > 1 else 0), (fmt, M, K, N)
