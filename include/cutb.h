@@ -128,16 +128,16 @@ enum { CUTB_FLAG_NO_OVERLAP = 1, CUTB_FLAG_ACT_16BIT = 2, CUTB_FLAG_A_RMSNORM = 
  * Strides are in elements (bytes for W planes), as in the reference.
  *
  * Operand range.  The generic and the decode variants dequantise exactly and take fp32
- * activations at full range.  CUTB_VARIANT_GEMM_TC (what CUTB_VARIANT_AUTO picks above 8 fp32 /
- * 16 fp16 activation rows over GGUF blocks, and from 13 fp16 rows on weights of 16 M elements
- * and more) feeds the tensor cores fp16 operands, as the
+ * activations at full range.  CUTB_VARIANT_GEMM_TC and CUTB_VARIANT_ROWS_MMA (one of which
+ * CUTB_VARIANT_AUTO picks above 8 fp32 / 16 fp16 activation rows over GGUF blocks, and for some
+ * weights from 9 fp16 rows) feed the tensor cores fp16 operands, as the
  * reference's tensor-core variants do (MatMulQ4CoopMatTiled.cu:37-75): fp32 activations are
  * rounded to fp16 first, and a dequantised weight d * q (d * sc * q - dmin * m for Q4_K) is
- * rounded to fp16 too.  |A| above 65504 therefore becomes infinity, and the launch records
+ * rounded to fp16 too (CUTB_VARIANT_ROWS_MMA: above 16 rows).  |A| above 65504 therefore becomes infinity, and the launch records
  * CUTB_ERR_RANGE in *status (the output then holds inf / NaN where such a value took part);
  * weight products below 6e-8 flush to zero.  Callers whose activations can exceed the fp16
  * range select CUTB_VARIANT_GENERIC, or scale A down and C up.  Accumulation and C are fp32.
- * Up to 128 activation rows the same variant runs a kernel of its own (tokens as the MMA's M
+ * Up to 128 activation rows CUTB_VARIANT_GEMM_TC runs a kernel of its own (tokens as the MMA's M
  * operand, K shared out over all SMs); it is launched with programmatic stream serialization
  * like the decode mat-vec (it waits for the previous kernel only before it reads A and before it
  * stores), which CUTB_FLAG_NO_OVERLAP switches off.
@@ -175,8 +175,9 @@ typedef struct cutb_qmatmul_desc {
  * decode mat-vec its staged activations (three rows and up) and split-K partial sums; the tensor-core GEMM the
  * fp16 copy of fp32 activations and, up to 128 activation rows, the partial tiles of weight tiles whose K is shared
  * by several blocks (summed in a fixed order by a second small kernel; without that room every weight tile goes
- * whole to one block, which is slower but needs nothing); with 512 rows and more on few weight rows and K >= 8192,
- * planes of partial sums of a K split (same rule: optional, faster with them). */
+ * whole to one block, which is slower but needs nothing); above 128 rows, where few blocks have work, planes of
+ * M x N partial sums, one for each share of K (same rule: optional, faster with them; up to eight).
+ * CUTB_VARIANT_ROWS_MMA its reordered activations and the shares of weight tiles that several blocks work on. */
 CUTB_API uint64_t cutb_qmatmul_workspace_bytes(const cutb_qmatmul_desc *desc);
 
 /* Variant the library would run for this descriptor (resolves CUTB_VARIANT_AUTO, which may pick another kernel without scratch than
@@ -216,7 +217,8 @@ CUTB_API int cutb_qmatmul_decode_noalloc(const cutb_qmatmul_desc *desc, void *st
  *   flag_peers[q] rank q's arrival counter (one uint64, zero at the start, never reset)
  *   ldc_total     row stride of the full outputs (elements); n_offset: first column of the slice
  *
- * cutb_qmatmul_scatter: desc->C is not written.  The shape must take the mat-vec variant
+ * cutb_qmatmul_scatter: desc->C is not written.  A slice holds what CUTB_VARIANT_GEMV_MMA gives for these weight
+ * rows, bit for bit (CUTB_VARIANT_AUTO may pick another kernel from 9 fp16 rows up).  The shape must take the mat-vec variant
  * (M <= 16 fp16 / 8 fp32 rows, K % 256 == 0), else CUTB_ERR_UNSUPPORTED; shapes that split K need
  * the workspace of cutb_qmatmul_workspace_bytes(desc) as usual (their reduction kernel scatters).
  * The stores are not yet published when it returns or when its kernel ends.
