@@ -278,6 +278,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1) dense_gemm_tc_kernel(const __gr
         const uint32_t n = b.n0 + c0;
         if (n >= p.N) break;
         uint32_t v[32];
+        __syncwarp();  // (lanes without a row have gone ahead)
         tmem_ld32(tmem + ((quarter * 32) << 16) + a * 256 + c0, v);  // (the last piece of an odd number of 16s runs past the tile)
         if (m >= b.m_end) continue;
         const bool whole = n + 32 <= n_end;

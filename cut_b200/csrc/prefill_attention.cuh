@@ -589,6 +589,7 @@ __global__ void __launch_bounds__(PA_THREADS, 1)
       for (uint32_t c = 0; c < VP * 64; c += 32) {
         if (c >= p.vdim) break;
         uint32_t o[32];
+        __syncwarp();  // (lanes without a token have gone ahead)
         tmem_ld32_async(o_t + c, o);
         tmem_wait32(o);
         if (!live) continue;

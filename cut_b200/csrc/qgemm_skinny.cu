@@ -391,6 +391,7 @@ __global__ void __launch_bounds__(sk_threads(FMT), 1)
           const uint32_t k_hi = seg + 1 == nsegs ? (k_first + nunits - 1) % nk + 1 : nk;
           const bool whole = k_lo == 0 && k_hi == nk;
           uint32_t v[32];
+          __syncwarp();  // (lanes without a token have gone ahead)
           tmem_ld32(tmem_base + ((q * 32) << 16) + seg * SK_BW + c0, v);
           if (m >= p.M) continue;
           if (!whole) {

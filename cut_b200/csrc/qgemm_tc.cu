@@ -263,6 +263,7 @@ __global__ void __launch_bounds__(TC_MAX_THREADS, 1) qgemm_tc_kernel(const __gri
         for (uint32_t item = g; item < MB * (TC_BT / 32); item += G) {
           const uint32_t c0 = item * 32;  // token offset = accumulator column
           uint32_t v[32];
+          __syncwarp();
           tmem_ld32(tmem_base + ((q * 32) << 16) + c0, v);
           const uint32_t mbase = m0 + c0;
           if (mbase >= p.M) continue;

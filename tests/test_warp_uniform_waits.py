@@ -79,6 +79,25 @@ def test_no_lane_waits_alone_before_warp_wide_work(path):
         assert split_warps(f.read()) == []
 
 
+def split_loads(text):
+    """Loops that some lanes go round ahead of the others, into a tensor-memory load that wants the whole warp."""
+    text, found = _without_comments(text), []
+    for m in re.finditer(r"\bfor\s*\(", text):
+        start = _match(text, m.end() - 1, "(", ")")
+        body = text[start: _statement(text, start)]
+        load = re.search(r"\btmem_ld\w*\(", body)
+        inner = any(re.search(r"\btmem_ld\w*\(", body[f.end():]) for f in re.finditer(r"\bfor\s*\(", body[: load.start()])) if load else False
+        if load and not inner and re.search(r"\bcontinue;", body[load.end():]) and "__syncwarp()" not in body[: load.start()]:
+            found.append(text[m.start(): start])
+    return found
+
+
+@pytest.mark.parametrize("path", KERNELS, ids=os.path.basename)
+def test_a_warp_meets_before_it_loads_tensor_memory(path):
+    with open(path) as f:
+        assert split_loads(f.read()) == []
+
+
 @pytest.mark.parametrize("path", KERNELS, ids=os.path.basename)
 def test_copies_in_flight_are_waited_for_whoever_gives_up_and_when(path):
     """A copy warp that has issued everything may end before another warp gives up: its wait for copies does not hang on the flag."""
