@@ -493,7 +493,7 @@ uint32_t dg_pairs() {
 // Grouped: 240 rows gain nothing over 256 (16 experts of 200 tokens x 4: 98 against 97 us).
 template <class Tiles> void dg_width(uint32_t N, uint32_t nk, uint32_t sms, uint32_t pairs, bool grouped, Tiles row_tiles, DgPlan *pl) {
   static const struct { uint32_t bn, cost; } one[] = {{256, 140}, {240, 138}, {224, 125}, {208, 122}, {192, 112}, {128, 97}, {64, 90}},
-                                             two[] = {{256, 116}, {224, 100}, {192, 92}, {160, 90}, {128, 86}};
+                                             two[] = {{256, 115}, {224, 100}, {192, 92}, {160, 90}, {128, 86}};
   constexpr uint64_t PAIR_START = 570;
   uint64_t best = ~0ull;
   auto consider = [&](uint32_t bn, uint32_t cost, bool pair) {
@@ -601,13 +601,16 @@ int moe_gemm_tc_launch(const cutb_moe_desc &d, cudaStream_t stream) {
   p.c_bf16 = d.c_dtype == CUTB_BF16;
   p.nk = p.nk_per = (d.K + DG_BK - 1) / DG_BK, p.ksplit = 1;
   p.a_box_rows = rows >= DG_BM ? DG_BM : (rows + 7) / 8 * 8;
-  // Row tiles: an expert in use has one at least, and ends in a part-filled one, half of a tile on average.  (Counted as rows / n +
-  // used / 2, pairs seemed to halve the tiles of experts with less than a tile each, and the last wave went uncounted.)  us, counted so
-  // -> now, beside single CTAs x 256 rows: 16 experts, 1501 tokens x 4, 4096 -> 2 x 2048 gated 215 -> 193 (188), 200 tokens x 4 110 -> 97
-  // (97), 8 experts, 700 tokens x 2, 1024 -> 2 x 1024 21.5 -> 14.8 (14.8), 2000 tokens x 4, 2560 -> 2 x 2048 130 -> 126 (138).
-  const uint32_t used = d.experts < rows ? d.experts : rows;
+  // Row tiles: an expert in use has one at least; of two guesses, that experts are evenly used and that the last tile of each is half
+  // full on average, the one with fewer tiles.  (Counted as rows / n + used / 2, pairs seemed to halve the tiles of experts with less than
+  // a tile each, and the last wave went uncounted.)  us, counted so -> now, beside single CTAs x 256 rows: 16 experts, 200 tokens x 4,
+  // 4096 -> 2 x 2048 gated 110 -> 97 (97), 1501 tokens x 4 215 -> 194 (189; its down projection 109 -> 102 (111)), 8 experts, 700 tokens x 2,
+  // 1024 -> 2 x 1024 21.5 -> 14.8 (14.8), 2000 tokens x 4, 2560 -> 2 x 2048 130 -> 126 (138), 1500 tokens x 2, 4096 -> 2 x 2048 103 -> 94 (94).
+  const uint32_t used = d.experts < rows ? d.experts : rows, each = (rows + used - 1) / used;
   DgPlan pl{};
-  dg_width(d.N, p.nk, sms, rows > DG_BM ? dg_pairs() : 0, true, [&](uint32_t n) { return std::max(used, (2 * rows + used * n + 2 * n - 1) / (2 * n)); }, &pl);
+  dg_width(d.N, p.nk, sms, rows > DG_BM ? dg_pairs() : 0, true, [&](uint32_t n) {
+    return std::max(used, std::min(used * ((each + n - 1) / n), (2 * rows + used * n + 2 * n - 1) / (2 * n)));
+  }, &pl);
   p.tiles_m = rows / (pl.pair ? 2 * DG_BM : DG_BM) + used, p.tiles_n = pl.tiles_n;
   CUtensorMap ma, mw;
   if (int rc = make_tmap_sw128(&ma, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, d.A, rows, d.K, d.lda * 2, p.a_box_rows)) return rc;
