@@ -293,7 +293,7 @@ MatMulOpNode::MatMulOpNode(TensorStore &store, const Tensor &a, const Tensor &ra
   if (K_ % 256 == 0 && vrows <= 16) builtin = 1;
   else if (K_ % 256 == 0 && M_ > 1 && store.caps().cooperativeMatrix) builtin = 2;
   // 13 to 16 fp16 rows on 16 M weights or more: the tensor-core GEMM for few tokens beats the mat-vec's fourth
-  // column tile (the library's own automatic choice makes the same cut)
+  // column tile (the library makes the same cut for a caller without scratch)
   if (builtin == 1 && dtypeA_ == DataType::Float16 && M_ >= 13 && (uint64_t)K_ * N_ >= (1ull << 24) &&
       store.caps().cooperativeMatrix)
     builtin = 2;

@@ -73,7 +73,6 @@ template <int KP, int VP> constexpr uint32_t pa_smem() {
 }
 
 // A rows by tensor memory, B rows by descriptor
-template <bool BF16>
 __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t bdesc_lo, uint32_t desc_hi, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
@@ -336,7 +335,7 @@ __global__ void __launch_bounds__(PA_THREADS, 1)
           for (uint32_t term = 0; term < (BF16 ? 2u : 1u); ++term)
 #pragma unroll
             for (uint32_t ks = 4 * half; ks < 4 * half + 4; ++ks)
-              umma_ts<BF16>(tmem + 256 + x * 128, tmem + x * 128 + term * 64 + ks * 8, v_lo + sv * (VT >> 4) + ks * (2048 >> 4), v_hi, id_o,
+              umma_ts(tmem + 256 + x * 128, tmem + x * 128 + term * 64 + ks * 8, v_lo + sv * (VT >> 4) + ks * (2048 >> 4), v_hi, id_o,
                             term | ks ? 1u : acc[x]);
         }
       }

@@ -85,10 +85,10 @@ template <typename KV> __global__ void __launch_bounds__(256) window_kv_write_ke
 }
 
 // ---- prefill on the tensor cores -----------------------------------------------------------------------------------
-constexpr int WT_BM = 64, WT_BN = 64, WT_THREADS = 128, WT_PAD = 8;
+constexpr int WT_BM = 64, WT_BN = 64, WT_HEAD = 64, WT_THREADS = 128, WT_PAD = 8;
 
-template <int DK, int DV> __global__ void __launch_bounds__(WT_THREADS) window_attention_tc_kernel(const cutb_window_attn_desc d) {
-  constexpr int LK = DK + WT_PAD, LV = DV + WT_PAD, KS = DK / 16;
+__global__ void __launch_bounds__(WT_THREADS) window_attention_tc_kernel(const cutb_window_attn_desc d) {
+  constexpr int DK = WT_HEAD, DV = WT_HEAD, LK = DK + WT_PAD, LV = DV + WT_PAD, KS = DK / 16;
   constexpr uint32_t KT = WT_BN * LK * 2, VT = WT_BN * LV * 2;
   extern __shared__ __align__(16) uint8_t wt_smem[];
   __nv_bfloat16 *Qs = reinterpret_cast<__nv_bfloat16 *>(wt_smem);
@@ -615,10 +615,10 @@ template <typename KV, int RG> __global__ void __launch_bounds__(WD_THREADS) win
   cluster.sync();  // nobody leaves while its shared memory may still be read
 }
 
-template <int DK, int DV> int wt_launch(const cutb_window_attn_desc &d, cudaStream_t stream) {
-  constexpr size_t smem = ((size_t)(WT_BM + 2 * WT_BN) * (DK + WT_PAD) + (size_t)2 * WT_BN * (DV + WT_PAD)) * 2;
-  CUTB_CUDA_TRY(cudaFuncSetAttribute(window_attention_tc_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  CUTB_CUDA_TRY(launch_pdl(window_attention_tc_kernel<DK, DV>, dim3((d.n_tokens + WT_BM - 1) / WT_BM, d.n_heads), dim3(WT_THREADS), smem,
+int wt_launch(const cutb_window_attn_desc &d, cudaStream_t stream) {
+  constexpr size_t smem = ((size_t)(WT_BM + 4 * WT_BN) * (WT_HEAD + WT_PAD)) * 2;
+  CUTB_CUDA_TRY(cudaFuncSetAttribute(window_attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CUTB_CUDA_TRY(launch_pdl(window_attention_tc_kernel, dim3((d.n_tokens + WT_BM - 1) / WT_BM, d.n_heads), dim3(WT_THREADS), smem,
                            stream, d));
   return CUTB_OK;
 }
@@ -686,7 +686,7 @@ int window_attention_launch(const cutb_window_attn_desc &d, cudaStream_t stream)
     // Heads of 64 that see few keys: the smaller blocks start sooner (us, warp MMAs / tcgen05, 16 heads of 64: 100 tokens 8.3 / 9.2,
     // 1000 in a window of 300 18.2 / 19.9, 600 in one of 2048 23.4 / 18.0, 1500 in one of 1000 49.5 / 43.5).  Heads of 96 and 128
     // gain at every length (32 heads of 128: 16 tokens 15.3 / 11.3, 128 18.5 / 12.3, 512 36.7 / 20.4, 1501 154 / 69).
-    if (d.dim <= 64 && d.vdim <= 64) return d.n_tokens < 256 || d.window < 512 ? wt_launch<64, 64>(d, stream) : wp_launch<1, 1>(d, stream);
+    if (d.dim <= 64 && d.vdim <= 64) return d.n_tokens < 256 || d.window < 512 ? wt_launch(d, stream) : wp_launch<1, 1>(d, stream);
     if (d.dim <= 64) return wp_launch<1, 2>(d, stream);
     return d.vdim <= 64 ? wp_launch<2, 1>(d, stream) : wp_launch<2, 2>(d, stream);
   }
