@@ -258,3 +258,63 @@ def test_the_largest_weight_is_exact(mode, T, pos, sink):
     assert int(status.item()) == 0
     worst = ((got.double() - ref).norm(dim=2) / ref.norm(dim=2)).max()
     assert float(worst) <= 1e-6
+
+
+@pytest.mark.parametrize("mode", ["llama", "window", "latent"])
+@pytest.mark.parametrize("T,pos,window", [(128, 600, 1 << 20), (257, 511, 700), (700, 60, 1 << 20), (897, 0, 640)])
+def test_scores_that_jump(mode, T, pos, window):
+    """Every third token meets keys whose logits stand 20 and then 40 (in powers of two) above the others', in later key tiles: the maximum
+    is followed and what was summed is scaled down, several times in a row, while the other tokens of the warp stay as they are.  (700 and
+    897 tokens: two token tiles to a block, the second of the last block ragged, and of one token.)"""
+    import torch
+
+    if mode != "window":
+        window = 1 << 20
+    q, k, v = _inputs(mode, T, pos, T + pos)
+    H, at = q.shape[1], torch.arange(pos, pos + T, device="cuda")
+    d = q.shape[2] - (64 if mode == "latent" else 0)
+    scale = 0.1
+    unit = torch.zeros(d, device="cuda")
+    unit[: d // 2] = 1.0  # (exact in 16 bits)
+    q[::3, :, :d] += 4.0 * unit
+    for key, jump in ((140, 20.0), (139, 21.0), (300, 30.0), (420, 40.0), (421, 40.5), (pos + T - 2, 50.0)):
+        k[key, :, :d] = (jump / (4.0 * (d // 2) * scale * 1.4427) * unit).to(k.dtype)
+    sink = None if mode == "llama" else torch.zeros(H, device="cuda") if mode == "window" else torch.full((H,), 15.0, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    got = _attend(mode, q.to(k.dtype).float(), k, v, pos, window, scale, status, sink)
+    ref = _reference(q.to(k.dtype).double(), k.double(), v.double(), scale, at, window, None if sink is None else sink.double())
+    assert int(status.item()) == 0
+    assert _rel(got, ref) <= (1e-3 if mode == "llama" else 1e-4)
+    worst = (got.double() - ref).norm(dim=2) / ref.norm(dim=2)
+    assert float(worst.max()) <= (4e-3 if mode == "llama" else 4e-4)  # (a token: rounding of few weights, not averaged over many)
+
+
+@pytest.mark.parametrize("mode", ["llama", "window", "latent"])
+@pytest.mark.parametrize("T,pos,window", [(769, 0, 300), (640, 33, 257), (1153, 100, 640)])
+def test_two_token_tiles_to_a_block(mode, T, pos, window):
+    """Blocks of 256 tokens: both tiles over shared key and value slots, a last block of one tile, of one token, and of 129 tokens; windows
+    that begin and end inside a key tile; positions in no order on the llama path."""
+    import torch
+
+    if mode != "window":
+        window = 1 << 20
+    q, k, v = _inputs(mode, T, pos, T + pos)
+    at = torch.arange(pos, pos + T, device="cuda")
+    if mode == "llama":
+        at = at[torch.randperm(T, device="cuda", generator=torch.Generator(device="cuda").manual_seed(T))]
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    got = _attend(mode, q, k, v, pos, window, 0.1, status, order=at)
+    ref = _reference(q.double(), k.double(), v.double(), 0.1, at, window, None)
+    assert int(status.item()) == 0
+    assert _rel(got, ref) <= (1e-3 if mode == "llama" else 1e-4)
+
+
+@pytest.mark.parametrize("T,pos", [(300, 0), (700, 60)])
+def test_a_sink_of_minus_infinity_is_none(T, pos):
+    import torch
+
+    q, k, v = _inputs("latent", T, pos, T)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    one = _attend("latent", q, k, v, pos, 1 << 20, 0.1, status, torch.full((q.shape[1],), float("-inf"), device="cuda"))
+    assert torch.equal(one, _attend("latent", q, k, v, pos, 1 << 20, 0.1, status)) and bool(one.isfinite().all())
+    assert int(status.item()) == 0
