@@ -829,7 +829,7 @@ template <int VP> int lt_dispatch(const cutb_latent_attn_desc &d, uint32_t plane
 
 int latent_prefill_launch(const cutb_latent_attn_desc &d, cudaStream_t stream) {
   // tcgen05 where the number of expanded rows is known here (a position on the host) and the block's queries, keys and values
-  // fit shared memory: 32 heads of 128 + 64 / 128, us before / after: 40 tokens 21.4 / 11.8, 333 38.8 / 18.2, 1501 199 / 54
+  // fit shared memory: 32 heads of 128 + 64 / 128, us before / after: 40 tokens 21.4 / 11.8, 333 38.8 / 18.2, 1501 199 / 59
   const uint32_t planes = (d.dim + 63) / 64 + (d.rot_dim + 63) / 64;
   if (!d.pos_ptr && d.dim > 0 && planes <= 3 && d.vdim <= 128 && (d.n_tokens + 127) / 128 <= 65535 && (uint64_t)d.pos + d.n_tokens <= d.max_pos)
     return d.vdim <= 64 ? lt_dispatch<1>(d, planes, stream) : lt_dispatch<2>(d, planes, stream);

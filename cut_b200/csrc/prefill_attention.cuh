@@ -15,10 +15,10 @@
 //                   times values (shared memory, read along the keys).  The two token tiles alternate, so that the tensor cores
 //                   work for one while the other is in its softmax.
 // Tensor memory: 2 x 128 columns of scores / weights, 2 x 128 of weighted values.
-// Bound by the latency of a token tile's chain scores -> softmax -> weighted values (about 4500 cycles per 128 keys, of which the
-// tensor cores work 1500 and the exponentials 2000 for the two tiles together); the weights of 64 keys at a time are handed over,
-// so that the products of the first half run beside the exponentials of the second.  32 heads of 128, window 1024, 2048 tokens:
-// 207 us with warp MMAs -> 74 us (88.6 while blocks ran head by head; by ncu the tensor pipe is busy a third of a block's cycles).
+// Bound by the latency of a token tile's chain scores -> softmax -> weighted values (about 4500 cycles per 128 keys without rescaling,
+// of which the tensor cores work 3000, in fp16 2000, and the exponentials 2000 for the two tiles together); the weights of 64 keys at a
+// time are handed over, so that the products of the first half run beside the exponentials of the second.  32 heads of 128, window 1024,
+// 2048 tokens: 207 us with warp MMAs -> 78 us (by ncu the tensor pipe is busy 30 % of a block's cycles).
 // A row that comes out non-finite is computed again from the keys it sees alone (pa_row_again).
 // Every wait is bounded; on expiry the block records CUTB_ERR_TIMEOUT, waits (bounded) for its copies, frees its tensor memory
 // and returns.
