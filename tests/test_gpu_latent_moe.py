@@ -229,6 +229,34 @@ def test_expert_matvecs(T, E, top, width, ff, dense):
             assert rel(y[:width], want) < 3e-6 and float(y[width]) == 7.0
 
 
+@pytest.mark.parametrize("T,E,top,width,ff", [(2, 6, 6, 64, 40), (1, 64, 8, 256, 136), (1, 4, 2, 1028, 520)])
+@pytest.mark.parametrize("late", ["x", "act", "xd", "all"])
+def test_expert_matvecs_read_inputs_at_any_float(T, E, top, width, ff, late):
+    """Inputs that start between two 16-byte pieces are staged one element at a time: the same numbers, hence the same bits."""
+    m, rng, Kd = Moe(T, E, top, width, ff, limit=0.8), np.random.default_rng(7), 72
+    Wd, xd = bf16(rng.standard_normal((width, Kd)) / np.sqrt(Kd)), rng.standard_normal(Kd).astype(np.float32)
+    dense, z = dev(padded(Wd), torch.bfloat16), dev(m.z[0])
+
+    def place(name, a, shifted):
+        buf = torch.full((a.size + 8,), float("nan"), device="cuda")
+        at = 1 if shifted and late in (name, "all") else 0
+        buf[at : at + a.size] = dev(a)
+        assert (buf[at:].data_ptr() % 16 == 0) == (at == 0)
+        return buf[at : at + a.size]
+
+    outs = []
+    for shifted in (False, True):
+        x, xq, act = place("x", m.h[0], shifted), place("xd", xd, shifted), place("act", np.zeros(top * ff, np.float32), shifted)
+        ids, q, y = torch.full((top,), -1, dtype=torch.int32, device="cuda"), torch.zeros(width, device="cuda"), torch.zeros(width, device="cuda")
+        more = dict(dense=dense, dense_K=Kd, xd=xq)
+        ops.launch_layer_op("cutb_expert_up", ops.expert_desc(E, top, width, ff, m.gu, ids, act, logits=z, x=x, **m.glu, **more, out=q))
+        ops.launch_layer_op("cutb_expert_down", ops.expert_desc(E, top, width, ff, m.dn, ids, act, **more, out=y))
+        outs.append((act.clone(), q, y))
+    assert rel(outs[0][2], m.want(0)[0] + Wd.astype(np.float64) @ xd.astype(np.float64)) < 3e-6
+    for got, want in zip(outs[1], outs[0]):
+        assert torch.equal(got, want)
+
+
 # ---- latent attention ------------------------------------------------------------------------------------------------------
 class Latent:
     """Random queries and latents of one layer, its oracle, and the device side over a cache."""
