@@ -1,4 +1,5 @@
-// Decode mat-vec (a few activation rows) over native GGUF blocks for sm_100a.
+// Decode mat-vec of 2 to 16 activation rows over native GGUF blocks (qgemv_row.cu: one row, two at 16 bits), and the plan and
+// launch of both.
 //
 // C[m, n] = sum_k A[m, k] * dequant(W)[n, k], W = N rows of Q8_0 / Q4_0 / Q4_K
 // blocks.  Replaces the reference's M = 1 variants MatMulQ4GemvKPar8 /
@@ -48,8 +49,7 @@
 // CUTB_ERR_TIMEOUT in the caller's status word and leaves without spinning.
 #include <stdlib.h>
 
-#include "common.cuh"
-#include "kernels.h"
+#include "matvec_common.cuh"
 
 namespace cutb {
 
@@ -59,8 +59,6 @@ constexpr int GV_ROWS = 16;
 
 constexpr int GV_WARPS = 16;                      // consumer warps; one more warp issues the copies
 constexpr int GV_THREADS = (GV_WARPS + 1) * 32;
-// how the activations are read and staged
-constexpr int GV_A_HALF = 0, GV_A_F32_TWO = 1, GV_A_F32_ONE = 2;
 
 constexpr int GV_KC = GV_WARPS;                   // granules (256 weights) per row and stage, one per consumer warp
 
@@ -69,56 +67,12 @@ constexpr int GV_KC = GV_WARPS;                   // granules (256 weights) per 
 // MMA row g reads tile row 2g and MMA row g + 8 reads tile row 2g + 1 -- in different load
 // instructions, so the two rows of a pair may share banks, while the padding of the pair stride
 // keeps the 8 pairs of one instruction on disjoint banks (4 consecutive words per row for Q8_0 /
-// Q4_0 and the Q4_K diagonal variant, 8 for Q4_K shared-k).  Two rows that are adjacent in global
+// Q4_0, 8 for Q4_K).  Two rows that are adjacent in global
 // memory thus land adjacent in shared memory: when a stage holds whole rows, one bulk copy moves
 // a pair (the copy engine takes about as long to accept a copy whatever its size).
 __host__ __device__ constexpr int gv_raw_row(int fmt) { return GV_KC * (fmt == CUTB_Q8_0 ? 272 : 144); }
-__host__ __device__ constexpr int gv_pair_stride(int fmt, bool diag) {
-  return 2 * gv_raw_row(fmt) + ((fmt == CUTB_Q4_K && !diag) ? 32 : 16);  // = 4 or 8 words (mod 32)
-}
-
-struct GvParams {
-  const uint8_t *W;
-  uint64_t row_bytes;
-  const void *A;
-  uint32_t lda;
-  float *C;
-  uint32_t ldc;
-  const float *D;
-  uint32_t ldd;
-  float *partial;  // [ksplit][M][N] when ksplit > 1
-  uint32_t M, K, N;
-  uint32_t gran_per_split;
-  uint32_t ksplit;
-  uint32_t stages;
-  int fusion_type, fusion_op;
-  int a_f32;
-  int glu;              // rows in (gate, up) pairs: C[m, i] = unary(acc[2i]) * acc[2i + 1]
-  const float *norm_w;  // fused RMSNorm of the activation rows (nullptr: none)
-  float norm_eps;
-  int *status;
-  // Activations staged once for all CTAs by stage_acts_kernel (nullptr: every CTA stages its own):
-  // one blob per K split in the shared-memory layout [act | esc | sx], staged_bytes each.
-  uint8_t *staged;
-  uint32_t staged_bytes;
-  // Row-sharded scatter epilogue (world > 1): instead of C, the output slice is stored into
-  // every rank's full output at column n_off.  Peer-mapped pointers; plain stores, no
-  // multicast, no fence here: the step's exchange kernel publishes them.
-  uint32_t world, n_off, ldc_total;
-  float *peer_C[CUTB_MAX_PEERS];
-};
-
-// Shared-memory loads by 32-bit shared address.  Plain loads through an
-// address-space-qualified pointer rather than inline asm, so the compiler can
-// schedule them freely between the (memory-clobbering) barrier waits.
-__device__ __forceinline__ uint32_t lds_u32(uint32_t addr) {
-  return *reinterpret_cast<const uint32_t *>(__cvta_shared_to_generic(addr));
-}
-__device__ __forceinline__ uint2 lds_u64(uint32_t addr) {
-  return *reinterpret_cast<const uint2 *>(__cvta_shared_to_generic(addr));
-}
-__device__ __forceinline__ uint4 lds_u128(uint32_t addr) {
-  return *reinterpret_cast<const uint4 *>(__cvta_shared_to_generic(addr));
+__host__ __device__ constexpr int gv_pair_stride(int fmt) {
+  return 2 * gv_raw_row(fmt) + (fmt == CUTB_Q4_K ? 32 : 16);  // = 4 or 8 words (mod 32)
 }
 
 // int8 MMA, D = A * B with a zero accumulator.  UA: the A operand holds unsigned bytes.
@@ -148,12 +102,6 @@ __device__ __forceinline__ void mma_i8_acc(int (&d)[4], uint32_t a0, uint32_t a1
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// Low / high nibbles of four bytes -> four unsigned bytes 16 * q.  The Q4_0
-// offset (q - 8) is applied after the MMA through the staged sum of the
-// activations of the block: sum((q - 8) x) = sum(q x) - 8 sum(x).
-__device__ __forceinline__ uint32_t nib_lo_s(uint32_t x) { return (x << 4) & 0xF0F0F0F0u; }
-__device__ __forceinline__ uint32_t nib_hi_s(uint32_t x) { return x & 0xF0F0F0F0u; }
-
 // Element (0..31) of a 32-weight block that sits in byte i (0..7) of lane t's
 // MMA fragment pair {b0, b1}; the weight side reads its bytes in the same
 // order.  `even` = the block starts on a 4-byte boundary of the row.
@@ -174,177 +122,6 @@ template <int FMT> __device__ __forceinline__ uint32_t frag_elem(bool even, uint
     if (i < 4) return 2 + 4 * t + j;
     if (t < 3) return 18 + 4 * t + j;
     return (j < 2) ? 30 + j : j - 2;  // {30, 31, 0, 1}
-  }
-}
-
-// "Diagonal" variant used for one or two activation rows.  Lane t of a quad owns
-// whole blocks (2t and 2t+1 of each 8-block granule) instead of a quarter of
-// every block; its activation column pair is non-zero only in its own k slots,
-// so MMA column pair t ends up holding the dot product of the lane's own block:
-// the block scale is then applied once per block by the lane that loaded it.
-// Element of a 32-weight block in byte b (0..7) of the fragment of MMA i (0..3).
-template <int FMT> __device__ __forceinline__ uint32_t diag_elem(bool even, uint32_t i, uint32_t b) {
-  const uint32_t j = b & 3;
-  if constexpr (FMT == CUTB_Q4_K) {
-    return 8 * i + b;
-  } else if constexpr (FMT == CUTB_Q4_0) {
-    uint32_t byte;
-    if (!even) byte = 4 * i + j;
-    else if (i < 3) byte = 2 + 4 * i + j;
-    else byte = (j < 2) ? j : 12 + j;  // {0, 1, 14, 15}
-    return byte + ((b >> 2) << 4);
-  } else {
-    const uint32_t w = 2 * i + (b >> 2);
-    if (!even) return 4 * w + j;
-    if (w < 7) return 2 + 4 * w + j;
-    return (j < 2) ? j : 28 + j;  // {0, 1, 30, 31}
-  }
-}
-
-// The four MMAs of one block in two independent accumulation chains.  r0* / r1*:
-// first and second A register of MMA i for rows g (a) and g + 8 (b); act: shared
-// address of the lane's 32 staged activation bytes of the block.
-template <bool UA>
-__device__ __forceinline__ void block_mmas(int (&c)[4], int (&c2)[4], const uint32_t (&r0a)[4], const uint32_t (&r0b)[4],
-                                           const uint32_t (&r1a)[4], const uint32_t (&r1b)[4], uint32_t act) {
-  const uint4 x0 = lds_u128(act), x1 = lds_u128(act + 16);
-  mma_i8<UA>(c, r0a[0], r0b[0], r1a[0], r1b[0], x0.x, x0.y);
-  mma_i8<UA>(c2, r0a[1], r0b[1], r1a[1], r1b[1], x0.z, x0.w);
-  mma_i8_acc<UA>(c, r0a[2], r0b[2], r1a[2], r1b[2], x1.x, x1.y);
-  mma_i8_acc<UA>(c2, r0a[3], r0b[3], r1a[3], r1b[3], x1.z, x1.w);
-}
-
-// One granule (8 blocks of 32 weights, or one Q4_K super-block) x 16 rows for
-// the diagonal variant.  `rowA`: shared address of row g's granule; actp/escp/sxp:
-// per-lane shared addresses of the lane's even block (see the kernel), pass_a /
-// pass_e: byte distance to its odd block (0 for lanes whose columns are idle).
-template <int FMT, int NVR>
-__device__ __forceinline__ void compute_granule_diag(uint32_t rowA, const uint32_t (&actp)[NVR], uint32_t pass_a,
-                                                     const uint32_t (&escp)[NVR], const uint32_t (&sxp)[NVR],
-                                                     uint32_t pass_e, uint32_t t, float (&tot)[NVR][2]) {
-  const uint32_t rowB = rowA + gv_raw_row(FMT);  // the pair's second row: MMA row g + 8
-  // c / c2: two independent accumulation chains of the block's four MMAs
-  auto finish = [&](int nt, const int (&c)[4], const int (&c2)[4], float sA, float sB, uint32_t eoff) {
-    const float e = __uint_as_float(lds_u32(escp[nt] + eoff));
-    const float fg = (float)((c[0] + c2[0]) * 256 + (c[1] + c2[1])), fh = (float)((c[2] + c2[2]) * 256 + (c[3] + c2[3]));
-    if constexpr (FMT == CUTB_Q4_0) {
-      // d * (e/16 * sum(16 q x^) - 8 e sum(x^)) = d e sum((q - 8) x^)
-      const float off = __uint_as_float(lds_u32(sxp[nt] + eoff));
-      tot[nt][0] = fmaf(sA, fmaf(e, fg, -off), tot[nt][0]);
-      tot[nt][1] = fmaf(sB, fmaf(e, fh, -off), tot[nt][1]);
-    } else {
-      tot[nt][0] = fmaf(sA * e, fg, tot[nt][0]);
-      tot[nt][1] = fmaf(sB * e, fh, tot[nt][1]);
-    }
-  };
-  if constexpr (FMT == CUTB_Q4_0) {
-    const uint32_t pa = rowA + 36 * t, pb = rowB + 36 * t;
-    uint32_t la[9], lb[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) {
-      la[k] = lds_u32(pa + 4 * k);
-      lb[k] = lds_u32(pb + 4 * k);
-    }
-#pragma unroll
-    for (int pass = 0; pass < 2; ++pass) {
-      uint32_t wa[4], wb[4];
-      float dA, dB;
-      if (pass == 0) {
-        wa[0] = la[1]; wa[1] = la[2]; wa[2] = la[3]; wa[3] = __byte_perm(la[0], la[4], 0x5432);
-        wb[0] = lb[1]; wb[1] = lb[2]; wb[2] = lb[3]; wb[3] = __byte_perm(lb[0], lb[4], 0x5432);
-        dA = h2f_bits(la[0] & 0xFFFFu); dB = h2f_bits(lb[0] & 0xFFFFu);
-      } else {
-        wa[0] = la[5]; wa[1] = la[6]; wa[2] = la[7]; wa[3] = la[8];
-        wb[0] = lb[5]; wb[1] = lb[6]; wb[2] = lb[7]; wb[3] = lb[8];
-        dA = h2f_bits(la[4] >> 16); dB = h2f_bits(lb[4] >> 16);
-      }
-      uint32_t al[4], ah[4], bl[4], bh[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        al[i] = nib_lo_s(wa[i]); ah[i] = nib_hi_s(wa[i]);
-        bl[i] = nib_lo_s(wb[i]); bh[i] = nib_hi_s(wb[i]);
-      }
-#pragma unroll
-      for (int nt = 0; nt < NVR; ++nt) {
-        int c[4], c2[4];
-        block_mmas<true>(c, c2, al, bl, ah, bh, actp[nt] + pass * pass_a);
-        finish(nt, c, c2, dA, dB, pass * pass_e);
-      }
-    }
-  } else if constexpr (FMT == CUTB_Q8_0) {
-    const uint32_t pa = rowA + 68 * t, pb = rowB + 68 * t;
-#pragma unroll
-    for (int pass = 0; pass < 2; ++pass) {
-      uint32_t wa[8], wb[8];
-      float dA, dB;
-      if (pass == 0) {
-        const uint32_t a0 = lds_u32(pa), b0 = lds_u32(pb), a8 = lds_u32(pa + 32), b8 = lds_u32(pb + 32);
-#pragma unroll
-        for (int k = 0; k < 7; ++k) {
-          wa[k] = lds_u32(pa + 4 + 4 * k);
-          wb[k] = lds_u32(pb + 4 + 4 * k);
-        }
-        wa[7] = __byte_perm(a0, a8, 0x5432);
-        wb[7] = __byte_perm(b0, b8, 0x5432);
-        dA = h2f_bits(a0 & 0xFFFFu); dB = h2f_bits(b0 & 0xFFFFu);
-      } else {
-        dA = h2f_bits(lds_u32(pa + 32) >> 16); dB = h2f_bits(lds_u32(pb + 32) >> 16);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          wa[k] = lds_u32(pa + 36 + 4 * k);
-          wb[k] = lds_u32(pb + 36 + 4 * k);
-        }
-      }
-#pragma unroll
-      for (int nt = 0; nt < NVR; ++nt) {
-        const uint32_t r0a[4] = {wa[0], wa[2], wa[4], wa[6]}, r1a[4] = {wa[1], wa[3], wa[5], wa[7]};
-        const uint32_t r0b[4] = {wb[0], wb[2], wb[4], wb[6]}, r1b[4] = {wb[1], wb[3], wb[5], wb[7]};
-        int c[4], c2[4];
-        block_mmas<false>(c, c2, r0a, r0b, r1a, r1b, actp[nt] + pass * pass_a);
-        finish(nt, c, c2, dA, dB, pass * pass_e);
-      }
-    }
-  } else {  // Q4_K: lane t owns the 64-weight group t = sub-blocks 2t (low nibbles) and 2t+1 (high nibbles)
-    const uint4 hA = lds_u128(rowA), hB = lds_u128(rowB);
-    const uint4 qa0 = lds_u128(rowA + 16 + 32 * t), qa1 = lds_u128(rowA + 32 + 32 * t);
-    const uint4 qb0 = lds_u128(rowB + 16 + 32 * t), qb1 = lds_u128(rowB + 32 + 32 * t);
-    const uint32_t wa[8] = {qa0.x, qa0.y, qa0.z, qa0.w, qa1.x, qa1.y, qa1.z, qa1.w};
-    const uint32_t wb[8] = {qb0.x, qb0.y, qb0.z, qb0.w, qb1.x, qb1.y, qb1.z, qb1.w};
-    const float dA = h2f_bits(hA.x & 0xFFFFu), mA = h2f_bits(hA.x >> 16);
-    const float dB = h2f_bits(hB.x & 0xFFFFu), mB = h2f_bits(hB.x >> 16);
-    // 6-bit (scale, min) fields of this lane's two sub-blocks (gguf_reader.cpp:668-676)
-    const bool upper = t >= 2;  // sub-blocks 4..7 keep their high bits elsewhere
-    const uint32_t scA = upper ? (hA.w & 0x0F0F0F0Fu) | ((hA.y >> 2) & 0x30303030u) : hA.y & 0x3F3F3F3Fu;
-    const uint32_t mnA = upper ? ((hA.w >> 4) & 0x0F0F0F0Fu) | ((hA.z >> 2) & 0x30303030u) : hA.z & 0x3F3F3F3Fu;
-    const uint32_t scB = upper ? (hB.w & 0x0F0F0F0Fu) | ((hB.y >> 2) & 0x30303030u) : hB.y & 0x3F3F3F3Fu;
-    const uint32_t mnB = upper ? ((hB.w >> 4) & 0x0F0F0F0Fu) | ((hB.z >> 2) & 0x30303030u) : hB.z & 0x3F3F3F3Fu;
-    const float ndA = -dA * 8388608.f, nmA = -mA * 8388608.f, ndB = -dB * 8388608.f, nmB = -mB * 8388608.f;
-#pragma unroll
-    for (int pass = 0; pass < 2; ++pass) {
-      const uint32_t sel = 0x7540u | (((2 * t) & 3) + pass);
-      // d * (2^23 + sc) - d * 2^23 == d * sc exactly
-      const float dsA = fmaf(dA, __uint_as_float(__byte_perm(scA, 0x4B000000u, sel)), ndA);
-      const float dmA = fmaf(mA, __uint_as_float(__byte_perm(mnA, 0x4B000000u, sel)), nmA);
-      const float dsB = fmaf(dB, __uint_as_float(__byte_perm(scB, 0x4B000000u, sel)), ndB);
-      const float dmB = fmaf(mB, __uint_as_float(__byte_perm(mnB, 0x4B000000u, sel)), nmB);
-      uint32_t fa[8], fb[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        fa[k] = (pass ? (wa[k] >> 4) : wa[k]) & 0x0F0F0F0Fu;
-        fb[k] = (pass ? (wb[k] >> 4) : wb[k]) & 0x0F0F0F0Fu;
-      }
-#pragma unroll
-      for (int nt = 0; nt < NVR; ++nt) {
-        const uint32_t r0a[4] = {fa[0], fa[2], fa[4], fa[6]}, r1a[4] = {fa[1], fa[3], fa[5], fa[7]};
-        const uint32_t r0b[4] = {fb[0], fb[2], fb[4], fb[6]}, r1b[4] = {fb[1], fb[3], fb[5], fb[7]};
-        int c[4], c2[4];
-        block_mmas<true>(c, c2, r0a, r0b, r1a, r1b, actp[nt] + pass * pass_a);
-        finish(nt, c, c2, dsA, dsB, pass * pass_e);
-        const float sxv = __uint_as_float(lds_u32(sxp[nt] + pass * pass_e));
-        tot[nt][0] = fmaf(-dmA, sxv, tot[nt][0]);
-        tot[nt][1] = fmaf(-dmB, sxv, tot[nt][1]);
-      }
-    }
   }
 }
 
@@ -466,37 +243,16 @@ __device__ __forceinline__ void compute_stage(uint32_t st, uint32_t ngr, uint32_
   }
 }
 
-template <bool AF32> __device__ __forceinline__ float load_act(const void *A, uint64_t idx) {
-  if constexpr (AF32) return __ldg(reinterpret_cast<const float *>(A) + idx);
-  return __half2float(__ldg(reinterpret_cast<const __half *>(A) + idx));
-}
-
-// Balanced int8 digits of |v| <= 32639: v = 256 * hi + lo, both in [-128, 127].  Eight values
-// packed four to a word: the low digit is the value's low byte as it stands (read as int8),
-// the high digit is byte 1 of value + 128.
-__device__ __forceinline__ void pack_digits(const int (&v)[8], uint32_t (&hi)[2], uint32_t (&lo)[2]) {
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const uint32_t a = (uint32_t)v[4 * h], b = (uint32_t)v[4 * h + 1], c = (uint32_t)v[4 * h + 2], d = (uint32_t)v[4 * h + 3];
-    lo[h] = __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
-    hi[h] = __byte_perm(__byte_perm(a + 128u, b + 128u, 0x0051), __byte_perm(c + 128u, d + 128u, 0x0051), 0x5410);
-  }
-}
-
-constexpr float GV_QMAX = 32512.f;
-
 // Stages the activations of blocks [0, nblk) of this K split (starting at k0)
 // as two-digit block floating point in MMA fragment order.
 //   act  : [blk][col][lane t][8 bytes]; col = 2 * vrow + digit (0 = high digit)
 //   esc  : [blk][NV] fp32 scale of the integer dot product (includes the 1/16 of the Q4_0 nibble encoding)
 //   sx   : [blk][NV] fp32 e * sum(x^) (Q4_K), 8 e * sum(x^) (Q4_0: the q - 8 offset)
 //
-// Diagonal variant (DIAG): act is [blk][vrow][digit][MMA i][8 bytes] followed by
-// 32 zero bytes, esc / sx are [blk][NT] (NT = number of virtual rows).
-template <int FMT, int AMODE, int NT, bool DIAG, int THREADS>
+template <int FMT, int AMODE, int NT, int THREADS>
 __device__ __forceinline__ void stage_activations(const GvParams &p, uint8_t *act, float *esc, float *sx, uint32_t k0,
                                                   uint32_t nblk, uint32_t ncp, uint32_t tid, const float *nscale) {
-  constexpr uint32_t NV = DIAG ? NT : NT * 4;
+  constexpr uint32_t NV = NT * 4;
   const uint32_t nrows = p.M;
   constexpr bool AF32 = AMODE != GV_A_HALF;      // fp32 loads
   constexpr bool TWO = AMODE == GV_A_F32_TWO;     // two 16-bit levels per fp32 value
@@ -526,7 +282,7 @@ __device__ __forceinline__ void stage_activations(const GvParams &p, uint8_t *ac
         float2 v[4];
 #pragma unroll
         for (uint32_t i = 0; i < 4; ++i) {
-          const uint32_t el = DIAG ? diag_elem<FMT>(even, ct, 2 * i) : frag_elem<FMT>(even, ct, 2 * i);
+          const uint32_t el = frag_elem<FMT>(even, ct, 2 * i);
           v[i] = __ldg(reinterpret_cast<const float2 *>(reinterpret_cast<const float *>(p.A) + rb + el));
         }
 #pragma unroll
@@ -535,7 +291,7 @@ __device__ __forceinline__ void stage_activations(const GvParams &p, uint8_t *ac
         __half2 v[4];
 #pragma unroll
         for (uint32_t i = 0; i < 4; ++i) {
-          const uint32_t el = DIAG ? diag_elem<FMT>(even, ct, 2 * i) : frag_elem<FMT>(even, ct, 2 * i);
+          const uint32_t el = frag_elem<FMT>(even, ct, 2 * i);
           v[i] = __ldg(reinterpret_cast<const __half2 *>(reinterpret_cast<const __half *>(p.A) + rb + el));
         }
 #pragma unroll
@@ -547,7 +303,7 @@ __device__ __forceinline__ void stage_activations(const GvParams &p, uint8_t *ac
     } else {
 #pragma unroll
       for (uint32_t i = 0; i < 8; ++i) {
-        const uint32_t el = DIAG ? diag_elem<FMT>(even, ct, i) : frag_elem<FMT>(even, ct, i);
+        const uint32_t el = frag_elem<FMT>(even, ct, i);
         x[i] = load_act<AF32>(p.A, rb + el);
       }
     }
@@ -555,7 +311,7 @@ __device__ __forceinline__ void stage_activations(const GvParams &p, uint8_t *ac
     for (uint32_t i = 0; i < 8; ++i) {
       if (!live) x[i] = 0.f;
       if (nscale && live) {  // RMSNorm fused into the staging
-        const uint32_t el = DIAG ? diag_elem<FMT>(even, ct, i) : frag_elem<FMT>(even, ct, i);
+        const uint32_t el = frag_elem<FMT>(even, ct, i);
         x[i] = x[i] * rs * __ldg(p.norm_w + k0 + kb * 32 + el);
       }
       amax = fmaxf(amax, fabsf(x[i]));
@@ -584,7 +340,6 @@ __device__ __forceinline__ void stage_activations(const GvParams &p, uint8_t *ac
     }
     // byte offset of (block, virtual row, digit, chunk) in the staged layout
     auto act_off = [&](uint32_t vrow, uint32_t digit) -> size_t {
-      if constexpr (DIAG) return (((size_t)kb * NT + vrow) * 2 + digit) * 32 + ct * 8;
       return ((size_t)(kb * ncp + 2 * vrow + digit) * 4 + ct) * 8;
     };
     if (live) {
@@ -620,11 +375,6 @@ __device__ __forceinline__ void stage_activations(const GvParams &p, uint8_t *ac
         }
       }
     }
-  }
-  if constexpr (DIAG) {
-    // lanes whose MMA columns belong to another lane's block read these zeros
-    if (tid < 8) reinterpret_cast<uint32_t *>(act + (size_t)p.gran_per_split * 8 * NT * 64)[tid] = 0u;
-    return;
   }
   // idle MMA columns read an all-zero column; idle virtual rows get scale 0
   const uint32_t ncols = 2 * nvr;
@@ -700,19 +450,19 @@ __global__ void __launch_bounds__(GV_WARPS * 32) stage_acts_kernel(const GvParam
   uint8_t *base = p.staged + (size_t)blockIdx.y * p.staged_bytes;
   float *esc0 = reinterpret_cast<float *>(base + (size_t)nblk_alloc * ncp * 32);
   float *sx0 = esc0 + (size_t)nblk_alloc * NV;
-  stage_activations<FMT, AMODE, NT, false, GV_WARPS * 32>(p, base + (size_t)b0 * ncp * 32, esc0 + (size_t)b0 * NV, sx0 + (size_t)b0 * NV,
+  stage_activations<FMT, AMODE, NT, GV_WARPS * 32>(p, base + (size_t)b0 * ncp * 32, esc0 + (size_t)b0 * NV, sx0 + (size_t)b0 * NV,
                                                           gs0 * 256 + b0 * 32, nb, ncp, tid, nscale);
 }
 
 // MINB: CTAs per SM the register budget is kept under -- 2 where this launch's CTA and the next launch's share an
 // SM, 1 for the plans whose shared memory fills the SM anyway (then up to 120 registers instead of 56).
-template <int FMT, int AMODE, int NT, bool DIAG, int MINB>
+template <int FMT, int AMODE, int NT, int MINB>
 __global__ void __launch_bounds__(GV_THREADS, MINB) qgemv_blocks_kernel(const GvParams p) {
-  constexpr int PS = gv_pair_stride(FMT, DIAG);
+  constexpr int PS = gv_pair_stride(FMT);
   constexpr uint32_t RAWROW = gv_raw_row(FMT);
   constexpr uint32_t GB = granule_bytes(FMT);
   constexpr uint32_t STAGE_BYTES = (GV_ROWS / 2) * PS;
-  constexpr uint32_t NV = DIAG ? NT : NT * 4, NC8 = NT * 8;
+  constexpr uint32_t NV = NT * 4, NC8 = NT * 8;
   extern __shared__ __align__(128) uint8_t smem[];
 
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
@@ -725,7 +475,7 @@ __global__ void __launch_bounds__(GV_THREADS, MINB) qgemv_blocks_kernel(const Gv
 
   uint8_t *ring = smem;
   uint8_t *act = ring + (size_t)S * STAGE_BYTES;
-  float *esc = reinterpret_cast<float *>(act + (DIAG ? (size_t)nblk_alloc * NT * 64 + 32 : (size_t)nblk_alloc * ncp * 32));
+  float *esc = reinterpret_cast<float *>(act + (size_t)nblk_alloc * ncp * 32);
   float *sx = esc + nblk_alloc * NV;
   float *red = sx + (FMT != CUTB_Q8_0 ? nblk_alloc * NV : 0);  // two buffers of [GV_WARPS][16][NV]
   uint64_t *bars = reinterpret_cast<uint64_t *>(red + 2 * GV_WARPS * GV_ROWS * NV);  // full[S], empty[S]
@@ -812,9 +562,7 @@ __global__ void __launch_bounds__(GV_THREADS, MINB) qgemv_blocks_kernel(const Gv
   // C may belong to the previous kernel of the stream: wait for it to finish.
   asm volatile("griddepcontrol.wait;" ::: "memory");
   bool dead = false;
-  bool fetched = false;
-  if constexpr (!DIAG) fetched = p.staged != nullptr;
-  if (fetched) {
+  if (p.staged) {
     // the launch before this one staged the activations of every K split once; fetch this split's
     // (the same bytes this CTA would have produced) with bulk copies
     const uint32_t abar = full_u + 4 * S * 8;
@@ -838,25 +586,17 @@ __global__ void __launch_bounds__(GV_THREADS, MINB) qgemv_blocks_kernel(const Gv
       rms_scales<AMODE != GV_A_HALF>(p, red, tid);
       nscale = red + GV_WARPS * 16;
     }
-    stage_activations<FMT, AMODE, NT, DIAG, GV_WARPS * 32>(p, act, esc, sx, gs0 * 256, ng * 8, ncp, tid, nscale);
+    stage_activations<FMT, AMODE, NT, GV_WARPS * 32>(p, act, esc, sx, gs0 * 256, ng * 8, ncp, tid, nscale);
   }
   asm volatile("bar.sync 1, %0;" ::"n"(GV_WARPS * 32) : "memory");
 
   const uint32_t act_u = smem_u32(act), act_stride = ncp * 32, esc_u = smem_u32(esc), sx_u = smem_u32(sx);
   // per-lane activation fragment offsets (idle lanes read zeros)
   uint32_t aoff[NT];
-  // diagonal variant: MMA column g belongs to the block pair of lane g >> 1, digit g & 1
-  const bool mine = (t == (g >> 1));
-  const uint32_t zero_u = act_u + nblk_alloc * NT * 64;
-  const uint32_t pass_a = mine ? NT * 64u : 0u, gran_a = mine ? 8u * NT * 64u : 0u;
 #pragma unroll
   for (int nt = 0; nt < NT; ++nt) {
-    if constexpr (DIAG) {
-      aoff[nt] = mine ? (((2 * t) * NT + nt) * 2 + (g & 1)) * 32 : 0u;
-    } else {
-      const uint32_t col = nt * 8 + g;
-      aoff[nt] = ((col < ncols ? col : ncols) * 4 + t) * 8;
-    }
+    const uint32_t col = nt * 8 + g;
+    aoff[nt] = ((col < ncols ? col : ncols) * 4 + t) * 8;
   }
 
   uint32_t slot = 0, parity = 0;
@@ -874,20 +614,8 @@ __global__ void __launch_bounds__(GV_THREADS, MINB) qgemv_blocks_kernel(const Gv
       const uint32_t gq = gs0 + c * GV_KC + warp;  // this warp's granule of the chunk
       if (!dead && gq < gs1) {
         const uint32_t kb0 = (gq - gs0) * 8;  // first 32-weight block of the granule inside the split
-        if constexpr (DIAG) {
-          uint32_t actp[NT], escp[NT], sxp[NT];
-#pragma unroll
-          for (int nt = 0; nt < NT; ++nt) {
-            actp[nt] = mine ? act_u + (gq - gs0) * gran_a + aoff[nt] : zero_u;
-            escp[nt] = esc_u + ((kb0 + 2 * t) * NT + nt) * 4;
-            sxp[nt] = sx_u + ((kb0 + 2 * t) * NT + nt) * 4;
-          }
-          compute_granule_diag<FMT, NT>(ring_u + slot * STAGE_BYTES + warp * GB + g * PS, actp, pass_a, escp, sxp,
-                                            NT * 4, t, tot);
-        } else {
-          compute_stage<FMT, NT, PS>(ring_u + slot * STAGE_BYTES + warp * GB, 1, act_u + kb0 * act_stride, act_stride,
-                                     aoff, esc_u + kb0 * NV * 4, sx_u + kb0 * NV * 4, g, t, tot);
-        }
+        compute_stage<FMT, NT, PS>(ring_u + slot * STAGE_BYTES + warp * GB, 1, act_u + kb0 * act_stride, act_stride, aoff,
+                                   esc_u + kb0 * NV * 4, sx_u + kb0 * NV * 4, g, t, tot);
       }
       __syncwarp();
       asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.u32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(
@@ -901,23 +629,9 @@ __global__ void __launch_bounds__(GV_THREADS, MINB) qgemv_blocks_kernel(const Gv
     float *rbuf = red + (size_t)(tile & 1) * GV_WARPS * GV_ROWS * NV;
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
-      if constexpr (DIAG) {
-        // the four lanes of a quad hold partial sums of the same virtual row
-        float a = tot[nt][0], b = tot[nt][1];
-        a += __shfl_xor_sync(0xffffffffu, a, 1);
-        b += __shfl_xor_sync(0xffffffffu, b, 1);
-        a += __shfl_xor_sync(0xffffffffu, a, 2);
-        b += __shfl_xor_sync(0xffffffffu, b, 2);
-        if (t == 0) {
-          float *r = rbuf + ((size_t)warp * GV_ROWS) * NV + nt;
-          r[(2 * g) * NV] = a;      // MMA row g = tile row 2g
-          r[(2 * g + 1) * NV] = b;  // MMA row g + 8 = tile row 2g + 1
-        }
-      } else {
-        float *r = rbuf + ((size_t)warp * GV_ROWS) * NV + nt * 4 + t;
-        r[(2 * g) * NV] = tot[nt][0];
-        r[(2 * g + 1) * NV] = tot[nt][1];
-      }
+      float *r = rbuf + ((size_t)warp * GV_ROWS) * NV + nt * 4 + t;
+      r[(2 * g) * NV] = tot[nt][0];      // MMA row g = tile row 2g
+      r[(2 * g + 1) * NV] = tot[nt][1];  // MMA row g + 8 = tile row 2g + 1
     }
     asm volatile("bar.sync 1, %0;" ::"n"(GV_WARPS * 32) : "memory");
     const uint32_t row_base = r0 + tile * GV_ROWS;
@@ -1039,7 +753,9 @@ int gv_amode(const cutb_qmatmul_desc &d) {
 
 struct GvPlan {
   uint32_t nt, nvr, ncp, grid_x, ksplit, gran_per_split, stages;
-  bool diag, overlap, pair;
+  bool overlap;
+  bool row;      // one or two virtual rows: qgemv_row.cu
+  RowPlan rp;
   size_t smem;
   // activations staged once per launch by stage_acts_kernel (otherwise by every CTA)
   bool prestage;
@@ -1047,26 +763,27 @@ struct GvPlan {
   uint64_t partial_bytes;   // split-K partial sums, rounded up to 256: the blobs follow them in the workspace
 };
 
-size_t gv_smem_bytes(int fmt, bool diag, uint32_t stages, uint32_t nt, uint32_t ncp, uint32_t gran_per_split) {
+size_t gv_smem_bytes(int fmt, uint32_t stages, uint32_t nt, uint32_t ncp, uint32_t gran_per_split) {
   const size_t nblk = (size_t)gran_per_split * 8;
-  const size_t nv = diag ? nt : nt * 4;
-  size_t b = (size_t)stages * (GV_ROWS / 2) * gv_pair_stride(fmt, diag);
-  b += diag ? nblk * nt * 64 + 32 : nblk * ncp * 32;
+  const size_t nv = nt * 4;
+  size_t b = (size_t)stages * (GV_ROWS / 2) * gv_pair_stride(fmt);
+  b += nblk * ncp * 32;
   b += nblk * nv * 4 * (fmt != CUTB_Q8_0 ? 2 : 1);
   b += (size_t)2 * GV_WARPS * GV_ROWS * nv * 4;
   b += 4 * stages * 8 + 8;  // full / empty barriers of both K halves of every slot; arrival of pre-staged activations
   return b;
 }
 
+uint64_t gv_partial_bytes(const cutb_qmatmul_desc &d, uint32_t ksplit) {
+  return ksplit > 1 ? ((uint64_t)ksplit * d.M * d.N * sizeof(float) + 255) / 256 * 256 : 0;
+}
+
 bool gv_plan(const cutb_qmatmul_desc &d, const DeviceInfo &di, GvPlan *pl) {
   const bool af32 = gv_amode(d) == GV_A_F32_TWO;  // two virtual rows per activation row
   pl->nvr = af32 ? 2 * d.M : d.M;
   if (pl->nvr == 0 || pl->nvr > 16) return false;
-  // one virtual row: the diagonal variant (nt = virtual rows); otherwise 4 virtual rows per MMA n-tile
-  // measured: with two virtual rows the diagonal variant only pays for two fp16 rows of Q8_0
-  // (elsewhere its second row costs registers and spills: Q4_K 13.4 -> 10.5 us, fp32 rows 10 % faster shared-k)
-  pl->diag = pl->nvr == 1 || (pl->nvr == 2 && !af32 && d.format == CUTB_Q8_0);
-  pl->nt = pl->diag ? pl->nvr : (pl->nvr <= 4 ? 1 : (pl->nvr <= 8 ? 2 : 4));
+  pl->row = pl->nvr <= 2;
+  pl->nt = pl->nvr <= 4 ? 1 : (pl->nvr <= 8 ? 2 : 4);  // 4 virtual rows per MMA n-tile
   const uint32_t ncols = 2 * pl->nvr;
   pl->ncp = ncols < pl->nt * 8 ? ncols + 1 : ncols;
   const uint32_t G = d.K / 256;
@@ -1085,31 +802,40 @@ bool gv_plan(const cutb_qmatmul_desc &d, const DeviceInfo &di, GvPlan *pl) {
   if (const char *e = getenv("CUTB_GV_STAGES")) max_stages = (uint32_t)atoi(e) < 2 ? 2u : (uint32_t)atoi(e);  // tuning override
   for (uint32_t ks = want; ks <= G; ++ks) {
     const uint32_t gps = (G + ks - 1) / ks;
+    if (pl->row) {
+      pl->ksplit = (G + gps - 1) / gps;
+      if (!row_matvec_plan(d, gv_amode(d), di, pl->ksplit, gps, &pl->rp)) continue;
+      pl->gran_per_split = gps;
+      pl->stages = pl->rp.depth;
+      pl->prestage = false;
+      pl->staged_bytes = 0;
+      pl->partial_bytes = gv_partial_bytes(d, pl->ksplit);
+      return true;
+    }
     // (whatever this launch's own overlap flag says: a CTA above half an SM keeps the NEXT launch from becoming
     // resident under this one's tail.  Measured on the 32-layer decode step: a four-slot ring for the launches that
     // do not overlap themselves cost 17 % of the step, 540 -> 451 tok/s.)
-    const bool pair = gv_smem_bytes(d.format, pl->diag, 2, pl->nt, pl->ncp, gps) <= half;
+    const bool pair = gv_smem_bytes(d.format, 2, pl->nt, pl->ncp, gps) <= half;
     for (uint32_t st = pair ? 2 : max_stages; st >= 2; --st) {
-      const size_t sm = gv_smem_bytes(d.format, pl->diag, st, pl->nt, pl->ncp, gps);
+      const size_t sm = gv_smem_bytes(d.format, st, pl->nt, pl->ncp, gps);
       if (sm <= limit) {
         pl->gran_per_split = gps;
         pl->ksplit = (G + gps - 1) / gps;
         pl->stages = st;
         pl->smem = sm;
-        pl->pair = pair;
         // A split forced by shared memory (many activation rows, long K) must not push the launch into a
         // second wave: CTAs this large sit one to an SM, so give every CTA more rows instead.
         if (!pair && (uint64_t)pl->grid_x * pl->ksplit > (uint32_t)di.sm_count) {
           const uint32_t gx = (uint32_t)di.sm_count / pl->ksplit;
           pl->grid_x = gx ? gx : 1;
         }
-        const uint32_t nv = pl->diag ? pl->nt : pl->nt * 4;
+        const uint32_t nv = pl->nt * 4;
         // From three virtual rows up the staging, repeated by every CTA, outweighs the mat-vec (measured:
         // 11008 x 4096 Q4_0, batch 8: 17.6 us, of which about 10 us staging): stage once, in a launch of its own.
-        pl->prestage = !pl->diag && pl->nvr >= 3 && !(d.flags & CUTB_FLAG_STAGE_PER_CTA);
+        pl->prestage = !(d.flags & CUTB_FLAG_STAGE_PER_CTA);
         if (const char *e = getenv("CUTB_GV_PRESTAGE")) pl->prestage = pl->prestage && atoi(e) != 0;  // tuning override
         pl->staged_bytes = gps * 8 * (pl->ncp * 32 + nv * 4 * (d.format != CUTB_Q8_0 ? 2 : 1));
-        pl->partial_bytes = pl->ksplit > 1 ? ((uint64_t)pl->ksplit * d.M * d.N * sizeof(float) + 255) / 256 * 256 : 0;
+        pl->partial_bytes = gv_partial_bytes(d, pl->ksplit);
         return true;
       }
     }
@@ -1139,7 +865,7 @@ int gv_launch_prestage(const GvParams &p, const GvPlan &pl, cudaStream_t stream)
   return CUTB_OK;
 }
 
-template <int FMT, int AMODE, int NT, bool DIAG, int MINB>
+template <int FMT, int AMODE, int NT, int MINB>
 int gv_launch_inst(const GvParams &p, const GvPlan &pl, cudaStream_t stream) {
   static bool configured[64] = {};  // per device: the attribute is set once on each
   int dev = 0;
@@ -1147,14 +873,12 @@ int gv_launch_inst(const GvParams &p, const GvPlan &pl, cudaStream_t stream) {
   if (dev < 0 || dev >= 64 || !configured[dev]) {
     DeviceInfo di;
     if (int rc = get_device_info(&di)) return rc;
-    CUTB_CUDA_TRY(cudaFuncSetAttribute(qgemv_blocks_kernel<FMT, AMODE, NT, DIAG, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    CUTB_CUDA_TRY(cudaFuncSetAttribute(qgemv_blocks_kernel<FMT, AMODE, NT, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)di.smem_optin));
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
-  if constexpr (!DIAG) {
-    if (pl.prestage)
-      if (int rc = gv_launch_prestage<FMT, AMODE, NT>(p, pl, stream)) return rc;
-  }
+  if (pl.prestage)
+    if (int rc = gv_launch_prestage<FMT, AMODE, NT>(p, pl, stream)) return rc;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(pl.grid_x, pl.ksplit);
   cfg.blockDim = dim3(GV_THREADS);
@@ -1165,20 +889,19 @@ int gv_launch_inst(const GvParams &p, const GvPlan &pl, cudaStream_t stream) {
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pl.overlap ? 1 : 0;
-  CUTB_CUDA_TRY(cudaLaunchKernelEx(&cfg, qgemv_blocks_kernel<FMT, AMODE, NT, DIAG, MINB>, p));
+  CUTB_CUDA_TRY(cudaLaunchKernelEx(&cfg, qgemv_blocks_kernel<FMT, AMODE, NT, MINB>, p));
   return CUTB_OK;
 }
 
 template <int FMT, int AMODE>
 int gv_launch_nt(const GvParams &p, const GvPlan &pl, cudaStream_t stream) {
-  if (pl.diag) return pl.nt == 1 ? gv_launch_inst<FMT, AMODE, 1, true, 2>(p, pl, stream) : gv_launch_inst<FMT, AMODE, 2, true, 2>(p, pl, stream);
   // measured: the 56-register build is the faster one for 4 and 8 virtual rows even where shared memory leaves room
   // for one CTA only (11008 x 4096 Q4_0, batch 8: 12.2 us against 13.7 with 96 registers); 16 rows gain from the
   // larger budget (34.9 -> 28.2 us): no spills, four independent MMA chains per block
   switch (pl.nt) {
-    case 1: return gv_launch_inst<FMT, AMODE, 1, false, 2>(p, pl, stream);
-    case 2: return gv_launch_inst<FMT, AMODE, 2, false, 2>(p, pl, stream);
-    default: return gv_launch_inst<FMT, AMODE, 4, false, 1>(p, pl, stream);  // 16 virtual rows never leave room for a second CTA
+    case 1: return gv_launch_inst<FMT, AMODE, 1, 2>(p, pl, stream);
+    case 2: return gv_launch_inst<FMT, AMODE, 2, 2>(p, pl, stream);
+    default: return gv_launch_inst<FMT, AMODE, 4, 1>(p, pl, stream);  // 16 virtual rows never leave room for a second CTA
   }
 }
 
@@ -1335,7 +1058,8 @@ int qgemv_blocks_launch(const cutb_qmatmul_desc &d, cudaStream_t stream, const c
     }
   }
   int rc;
-  switch (d.format) {
+  if (pl.row) rc = row_matvec_launch(p, d.format, amode, pl.rp, pl.overlap, stream);
+  else switch (d.format) {
     case CUTB_Q8_0: rc = gv_launch_a<CUTB_Q8_0>(p, pl, amode, stream); break;
     case CUTB_Q4_0: rc = gv_launch_a<CUTB_Q4_0>(p, pl, amode, stream); break;
     default: rc = gv_launch_a<CUTB_Q4_K>(p, pl, amode, stream); break;

@@ -1,0 +1,95 @@
+"""The mat-vec of one row and of two fp16 rows (qgemv_row.cu) at the edges of its tiles, stages, groups and loads, against the checker's
+dequantised weights in 64 bits.
+
+Tolerances: a 16-bit level leaves an error of at most max|x of a block| / 65024 per element, uniform, so relative to a block of normal
+values (maximum about 2.5 sigma) 2.5 / 65024 / sqrt(3) = 2.2e-5 of the norm: four times that.  Two levels leave the fp32 sums: 2^-24 times
+the square root of some thousand terms at worst, 2e-6."""
+import numpy as np
+import pytest
+
+from cut_b200 import _lib as L
+from cut_b200 import synth
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+FMTS = [synth.Q8_0, synth.Q4_0, synth.Q4_K]
+TOL = {16: 9e-5, 32: 2e-6}
+
+
+def _run(fmt, A, W, N, *, shift=0, flags=0, norm=None, fusion=(0, 0), D=None):
+    import torch
+
+    from cut_b200 import ops
+
+    M, K = A.shape
+    wide = torch.zeros(M, K + 8, dtype=torch.float16 if A.dtype == np.float16 else torch.float32, device="cuda")
+    a = wide[:, shift: shift + K]  # rows that start `shift` elements past an aligned address, K + 8 apart
+    a.copy_(torch.from_numpy(A))
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    d, C, keep = ops.make_desc(a, torch.from_numpy(W).cuda(), fmt, N, fusion_type=fusion[0], fusion_op=fusion[1], status=status, flags=flags,
+                               D=None if D is None else torch.from_numpy(D).cuda())
+    if norm is not None:
+        norm = torch.from_numpy(norm).cuda()
+        d.flags |= L.FLAG_A_RMSNORM
+        d.a_norm_weight, d.a_norm_eps = norm.data_ptr(), 1e-5
+    ws = torch.empty(max(ops.workspace_bytes(d), 16), dtype=torch.uint8, device="cuda")
+    d.workspace, d.workspace_bytes = ws.data_ptr(), ws.numel()
+    ops.launch(d)
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    return C.cpu().numpy().astype(np.float64)
+
+
+def _case(fmt, M, K, N, dtype, seed):
+    W = synth.make_weights(fmt, N, K, seed)
+    return synth.make_activations(M, K, seed + 1, dtype), W, O.dequant_rows(fmt, W, N, K).astype(np.float64)
+
+
+def _err(got, want):
+    return float(np.linalg.norm(got - want) / np.linalg.norm(want))
+
+
+@pytest.mark.parametrize("fmt", FMTS)
+@pytest.mark.parametrize("M,dtype,flags", [(1, np.float16, 0), (2, np.float16, 0), (1, np.float32, 0), (2, np.float32, L.FLAG_ACT_16BIT)])
+@pytest.mark.parametrize("K,N", [(256, 1), (512, 17), (1280, 2400), (2048, 1500), (4096, 1201), (4352, 1300), (8192, 1250), (14336, 1216), (256, 19100)])
+def test_tiles_stages_and_groups(fmt, M, dtype, flags, K, N):
+    """One row to a tile, ragged tiles, stages that part of the warps share, granules beyond the last stage, more tiles than a block sums up
+    at a time, K split and whole."""
+    A, W, dense = _case(fmt, M, K, N, dtype, K + N + fmt)
+    levels = 32 if dtype == np.float32 and not flags else 16
+    assert _err(_run(fmt, A, W, N, flags=flags), A.astype(np.float64) @ dense.T) <= TOL[levels]
+
+
+@pytest.mark.parametrize("fmt", FMTS)
+@pytest.mark.parametrize("dtype,shift", [(np.float16, 1), (np.float16, 4), (np.float32, 1), (np.float32, 2)])
+def test_rows_at_any_element(fmt, dtype, shift):
+    K, N = 4096, 1300
+    A, W, dense = _case(fmt, 1, K, N, dtype, shift + fmt)
+    want = A.astype(np.float64) @ dense.T
+    assert _err(_run(fmt, A, W, N, shift=shift), want) <= TOL[32 if dtype == np.float32 else 16]
+
+
+@pytest.mark.parametrize("fmt", FMTS)
+@pytest.mark.parametrize("K,N", [(2304, 1300), (4096, 1184), (4096, 200)])  # (the last one splits K: the squares of the whole row)
+def test_rms_meets_the_sums(fmt, K, N):
+    A, W, dense = _case(fmt, 1, K, N, np.float32, K + fmt)
+    w = (1.0 + 0.1 * np.random.default_rng(3).normal(size=K)).astype(np.float32)
+    x = A.astype(np.float64)
+    want = (x / np.sqrt((x * x).mean() + 1e-5) * w) @ dense.T + 0.5
+    got = _run(fmt, A, W, N, norm=w, fusion=(L.FUSION_BINARY, 0), D=np.full((1, N), 0.5, np.float32))
+    assert _err(got, want) <= TOL[32]
+
+
+@pytest.mark.parametrize("fmt", FMTS)
+def test_values_at_the_ends_of_the_range(fmt):
+    """Values so small that the inverse of a block's scale leaves the range of fp32 (as precise as subnormal scales are), one block 1e35 times
+    the others, and one NaN, which every output shows."""
+    K, N = 4096, 1200
+    A, W, dense = _case(fmt, 1, K, N, np.float32, 9 + fmt)
+    small = (A * np.float32(1e-36)).astype(np.float32)
+    assert _err(_run(fmt, small, W, N), small.astype(np.float64) @ dense.T) <= 0.05  # steps of 3e-39 beside values of 1e-36: 1 %, and fp32's own
+    large = A.copy()
+    large[0, 32:64] *= np.float32(1e35)
+    assert _err(_run(fmt, large, W, N), large.astype(np.float64) @ dense.T) <= TOL[32]
+    A[0, 777] = np.nan
+    assert np.isnan(_run(fmt, A, W, N)).all()
