@@ -88,4 +88,8 @@ struct RowPlan {
 bool row_matvec_plan(const cutb_qmatmul_desc &d, int amode, const DeviceInfo &di, uint32_t ksplit, uint32_t gran_per_split, RowPlan *pl);
 int row_matvec_launch(const GvParams &p, int format, int amode, const RowPlan &pl, bool overlap, cudaStream_t stream);
 
+// Three to eight fp16 rows (qgemv_few.cu).
+bool few_matvec_plan(const cutb_qmatmul_desc &d, const DeviceInfo &di, uint32_t ksplit, uint32_t gran_per_split, RowPlan *pl);
+int few_matvec_launch(const GvParams &p, int format, const RowPlan &pl, bool overlap, cudaStream_t stream);
+
 }  // namespace cutb

@@ -755,6 +755,7 @@ struct GvPlan {
   uint32_t nt, nvr, ncp, grid_x, ksplit, gran_per_split, stages;
   bool overlap;
   bool row;      // one or two virtual rows: qgemv_row.cu
+  bool few;      // three to eight fp16 rows, where fp16 MMAs are the faster: qgemv_few.cu
   RowPlan rp;
   size_t smem;
   // activations staged once per launch by stage_acts_kernel (otherwise by every CTA)
@@ -783,6 +784,7 @@ bool gv_plan(const cutb_qmatmul_desc &d, const DeviceInfo &di, GvPlan *pl) {
   pl->nvr = af32 ? 2 * d.M : d.M;
   if (pl->nvr == 0 || pl->nvr > 16) return false;
   pl->row = pl->nvr <= 2;
+  pl->few = false;
   pl->nt = pl->nvr <= 4 ? 1 : (pl->nvr <= 8 ? 2 : 4);  // 4 virtual rows per MMA n-tile
   const uint32_t ncols = 2 * pl->nvr;
   pl->ncp = ncols < pl->nt * 8 ? ncols + 1 : ncols;
@@ -836,6 +838,8 @@ bool gv_plan(const cutb_qmatmul_desc &d, const DeviceInfo &di, GvPlan *pl) {
         if (const char *e = getenv("CUTB_GV_PRESTAGE")) pl->prestage = pl->prestage && atoi(e) != 0;  // tuning override
         pl->staged_bytes = gps * 8 * (pl->ncp * 32 + nv * 4 * (d.format != CUTB_Q8_0 ? 2 : 1));
         pl->partial_bytes = gv_partial_bytes(d, pl->ksplit);
+        // (the scratch asked for and refused without stays that of the digits, whichever kernel runs)
+        pl->few = few_matvec_plan(d, di, pl->ksplit, gps, &pl->rp);
         return true;
       }
     }
@@ -1059,6 +1063,7 @@ int qgemv_blocks_launch(const cutb_qmatmul_desc &d, cudaStream_t stream, const c
   }
   int rc;
   if (pl.row) rc = row_matvec_launch(p, d.format, amode, pl.rp, pl.overlap, stream);
+  else if (pl.few) rc = few_matvec_launch(p, d.format, pl.rp, pl.overlap, stream);
   else switch (d.format) {
     case CUTB_Q8_0: rc = gv_launch_a<CUTB_Q8_0>(p, pl, amode, stream); break;
     case CUTB_Q4_0: rc = gv_launch_a<CUTB_Q4_0>(p, pl, amode, stream); break;

@@ -679,17 +679,7 @@ int row_matvec_launch(const GvParams &g, int format, int amode, const RowPlan &p
   p.depth = pl.depth;
   p.groups = pl.groups;
   CUtensorMap map;
-  EncodeTiledFn encode = nullptr;
-  if (int rc = tc_encode_fn(&encode)) return rc;
-  const uint32_t gb = granule_bytes(format);
-  const cuuint64_t dims[3] = {gb / 4, p.N, p.K / 256}, strides[2] = {p.row_bytes, gb};
-  const cuuint32_t box[3] = {gb / 4, RW_ROWS, rw_granules(format)}, step[3] = {1, 1, 1};
-  const CUresult r = encode(&map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<uint8_t *>(p.W), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    set_last_error("qgemv: cuTensorMapEncodeTiled failed with %d for the weight (N=%u row bytes=%llu)", (int)r, p.N, (unsigned long long)p.row_bytes);
-    return CUTB_ERR_CUDA;
-  }
+  if (int rc = make_tmap_granules(&map, p.W, format, p.N, p.K, p.row_bytes, RW_ROWS, rw_granules(format))) return rc;
   switch (format) {
     case CUTB_Q8_0: return row_launch_fmt<CUTB_Q8_0>(map, p, amode, pl, overlap, stream);
     case CUTB_Q4_0: return row_launch_fmt<CUTB_Q4_0>(map, p, amode, pl, overlap, stream);

@@ -117,5 +117,23 @@ int make_tmap_sw128(CUtensorMap *map, CUtensorMapDataType type, const void *base
   return CUTB_OK;
 }
 
+
+// 3-D map over rows of GGUF blocks, seen as [granule of 256 weights][row][32-bit word]: boxes of `box_rows` rows x `box_granules`
+// granules.  Rows past N and granules past K read as zero.
+int make_tmap_granules(CUtensorMap *map, const void *W, int format, uint32_t N, uint32_t K, uint64_t row_bytes, uint32_t box_rows, uint32_t box_granules) {
+  EncodeTiledFn encode = nullptr;
+  if (int rc = tc_encode_fn(&encode)) return rc;
+  const uint32_t gb = granule_bytes(format);
+  const cuuint64_t dims[3] = {gb / 4, N, K / 256}, strides[2] = {row_bytes, gb};
+  const cuuint32_t box[3] = {gb / 4, box_rows, box_granules}, step[3] = {1, 1, 1};
+  const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<void *>(W), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    set_last_error("qgemv: cuTensorMapEncodeTiled failed with %d for the weight (N=%u row bytes=%llu)", (int)r, N, (unsigned long long)row_bytes);
+    return CUTB_ERR_CUDA;
+  }
+  return CUTB_OK;
+}
+
 }  // namespace
 }  // namespace cutb

@@ -1,4 +1,4 @@
-"""The mat-vec of one row and of two fp16 rows (qgemv_row.cu) at the edges of its tiles, stages, groups and loads, against the checker's
+"""The mat-vecs of one row and of two fp16 rows (qgemv_row.cu), and of three to eight fp16 rows (qgemv_few.cu), at the edges of its tiles, stages, groups and loads, against the checker's
 dequantised weights in 64 bits.
 
 Tolerances: a 16-bit level leaves an error of at most max|x of a block| / 65024 per element, uniform, so relative to a block of normal
@@ -93,3 +93,42 @@ def test_values_at_the_ends_of_the_range(fmt):
     assert _err(_run(fmt, large, W, N), large.astype(np.float64) @ dense.T) <= TOL[32]
     A[0, 777] = np.nan
     assert np.isnan(_run(fmt, A, W, N)).all()
+
+
+@pytest.mark.parametrize("fmt", [synth.Q4_0, synth.Q4_K])
+@pytest.mark.parametrize("M", [3, 4, 5, 8])
+@pytest.mark.parametrize("K,N", [(256, 2), (512, 1200), (1280, 2401), (2048, 9500), (4096, 200), (4096, 5000), (3072, 19100), (5120, 9600)])
+def test_a_few_rows(fmt, M, K, N):
+    """One tile and several per group of warps, a group without one, granules beyond the last stage, K split and whole, a longer K; rows
+    that start on 16 bytes and not.  Products of fp16 and 4-bit values are exact, sums have fp32's error, some 1e-6 of the largest partial
+    sum: up to sixteen times the result's where minima or offsets cancel."""
+    A, W, dense = _case(fmt, M, K, N, np.float16, M + K + N + fmt)
+    want = A.astype(np.float64) @ dense.T
+    tol = TOL[16] if M <= 4 and K > 3072 else 2e-5  # (some of these stay with the digits)
+    assert _err(_run(fmt, A, W, N), want) <= tol
+    assert _err(_run(fmt, A, W, N, shift=3), want) <= tol
+
+
+@pytest.mark.parametrize("fmt", [synth.Q4_0, synth.Q4_K])
+@pytest.mark.parametrize("M", [3, 7])
+def test_a_few_rows_in_pairs(fmt, M):
+    """Gate and up rows side by side, the last tile of the matrix a part of one; a tiny and a large row beside ordinary ones."""
+    K, N = 1024, 2 * 1189
+    A, W, dense = _case(fmt, M, K, N, np.float16, M + fmt)
+    A[0] = (A[0].astype(np.float32) * 1e-3).astype(np.float16)
+    A[1] = (A[1].astype(np.float32) * 1e3).astype(np.float16)
+    import torch
+
+    from cut_b200 import ops
+
+    out = torch.zeros(M, N // 2, device="cuda")
+    d, _, keep = ops.make_desc(torch.from_numpy(A).cuda(), torch.from_numpy(W).cuda(), fmt, N, C_out=out, fusion_type=L.FUSION_UNARY, fusion_op=130,
+                               flags=L.FLAG_GLU_PAIRS)
+    ws = torch.empty(max(ops.workspace_bytes(d), 16), dtype=torch.uint8, device="cuda")
+    d.workspace, d.workspace_bytes = ws.data_ptr(), ws.numel()
+    ops.launch(d)
+    torch.cuda.synchronize()
+    y = A.astype(np.float64) @ dense.T
+    want, got = np.maximum(y[:, 0::2], 0.0) * y[:, 1::2], out.cpu().numpy().astype(np.float64)
+    for m in range(M):
+        assert _err(got[m], want[m]) <= 4e-5, m
