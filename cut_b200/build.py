@@ -16,7 +16,7 @@ LIB = os.path.join(HERE, "libcutb.so")
 # layer operators and the layer-list models over dense bf16 weights: what a model without quantized weights needs
 LAYER_SOURCES = ["cabi_layers.cu", "common.cu", "layer_ops.cu", "mixer_ops.cu", "dense_matvec.cu", "dense_gemm.cu", "window_attention.cu",
                  "latent_attention.cu", "moe.cu", "expert_matvec.cu"]
-QUANT_SOURCES = ["cabi.cu", "qgemv_blocks.cu", "qgemv_row.cu", "qgemv_few.cu", "qmatmul_generic.cu", "dequant.cu", "transpose_q4.cu",
+QUANT_SOURCES = ["cabi.cu", "qgemv_blocks.cu", "qgemv_row.cu", "qgemv_few.cu", "qgemm_few.cu", "qmatmul_generic.cu", "dequant.cu", "transpose_q4.cu",
                  "qgemm_tc.cu", "qgemm_skinny.cu", "repack.cu", "attention.cu", "attention_prefill.cu", "qgemv_planes.cu", "qgemv_rows.cu"]
 SOURCES = QUANT_SOURCES + LAYER_SOURCES
 LAYERS_LIB = os.path.join(HERE, "libcutb_layers.so")

@@ -44,6 +44,12 @@ int qgemm_tc_launch(const cutb_qmatmul_desc &d, cudaStream_t stream);
 bool qgemm_skinny_applies(const cutb_qmatmul_desc &d);
 uint64_t qgemm_skinny_workspace(const cutb_qmatmul_desc &d);
 int qgemm_skinny_launch(const cutb_qmatmul_desc &d, cudaStream_t stream);
+// and for up to 64 rows over GGUF blocks, weights through tensor memory (qgemm_few.cu): where the scratch holds what it needs.  `direct`:
+// fp16 rows that start on 16 bytes each, which the kernel reads where they are
+bool qgemm_few_supported(const cutb_qmatmul_desc &d);
+uint64_t qgemm_few_workspace(const cutb_qmatmul_desc &d, bool direct);
+bool qgemm_few_fits(const cutb_qmatmul_desc &d);
+int qgemm_few_launch(const cutb_qmatmul_desc &d, cudaStream_t stream);
 
 int dequant_launch(int format, const void *raw, float *out, uint32_t rows, uint32_t cols, uint32_t ldo,
                    cudaStream_t stream);

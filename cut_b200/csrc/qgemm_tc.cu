@@ -455,7 +455,10 @@ uint64_t tc_cast_bytes(const cutb_qmatmul_desc &d) {
 }  // namespace
 
 uint64_t qgemm_tc_workspace(const cutb_qmatmul_desc &d) {
-  if (qgemm_skinny_applies(d)) return qgemm_skinny_workspace(d);
+  if (qgemm_skinny_applies(d)) {
+    const uint64_t skinny = qgemm_skinny_workspace(d), few = qgemm_few_supported(d) ? qgemm_few_workspace(d, d.a_dtype == CUTB_F16) : 0;
+    return skinny > few ? skinny : few;
+  }
   // fp32 activations are rounded to fp16 rows of K elements first; a K split adds its planes of partial sums
   DeviceInfo di;
   const uint32_t sms = get_device_info(&di) == CUTB_OK ? (uint32_t)di.sm_count : 148u;
@@ -465,6 +468,7 @@ uint64_t qgemm_tc_workspace(const cutb_qmatmul_desc &d) {
 }
 
 int qgemm_tc_launch(const cutb_qmatmul_desc &d, cudaStream_t stream) {
+  if (qgemm_few_supported(d) && qgemm_few_fits(d)) return qgemm_few_launch(d, stream);
   if (qgemm_skinny_applies(d)) return qgemm_skinny_launch(d, stream);
   DeviceInfo di;
   if (int rc = get_device_info(&di)) return rc;

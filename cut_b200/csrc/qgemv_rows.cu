@@ -1,10 +1,10 @@
-// Matmul of a few activation rows (9 to 32, held as fp16) over native GGUF blocks: batched decode.
+// Matmul of a few activation rows (9 to 16, held as fp16) over native GGUF blocks: batched decode.
 //
 // C[m, n] = epilogue(sum_k A[m, k] * dequant(W)[n, k]).  The mat-vec of fewer rows (qgemv_blocks.cu) turns activations into
 // int8 digits, two MMA columns per row; from nine rows up fp16 MMAs on the quants themselves cost less: a nibble becomes an fp16
 // integer with one logic operation per two weights and one exact subtraction, the activations enter as they are, and a block's
-// exact products (24-bit sums) are scaled in fp32 (up to 16 rows; from 17 rows up the scaling of every output costs more than
-// scaling the weights, so weights are rounded to fp16 once, as the tensor-core GEMMs do).
+// exact products (24-bit sums) are scaled in fp32.  From 17 rows up that scaling of every output costs more than scaling the weights,
+// and qgemm_few.cu takes over.
 //
 //  * Work is dealt in units of 128 weight rows x 256 k, equal contiguous runs to one CTA per SM (stream-K).  A unit is one stage
 //    of a ring: the raw block bytes (one 2-D TMA box) and the activations of these 256 k, already in MMA fragment order.
@@ -18,7 +18,7 @@
 //    sums behind them) and clears the counters.  Weight stages are in flight while it runs (programmatic dependent launch).
 //
 // Bound by the latency of the chain shared load -> widen -> MMA -> scale at four warps per scheduler, and by about 5 us of start,
-// staging and the meeting of the shares; 8192 x 8192 Q4_0, 32 rows: 26 us = 1.5 TB/s.
+// staging and the meeting of the shares; 8192 x 8192 Q4_0, 12 rows: 22 us = 1.7 TB/s.
 // Every wait is bounded; on expiry CUTB_ERR_TIMEOUT is recorded and the kernel runs to its end without waiting.
 #include <cuda.h>
 #include <cuda_fp16.h>
@@ -30,12 +30,11 @@
 namespace cutb {
 namespace {
 
+constexpr int GR_NT = 2;  // groups of eight activation rows
 constexpr uint32_t GR_ROWS = 128, GR_PITCH = 132, GR_WARPS = 16, GR_THREADS = (GR_WARPS + 1) * 32;
 __host__ __device__ constexpr uint32_t gr_chunk(int fmt) { return fmt == CUTB_Q8_0 ? 272u : 144u; }  // bytes of 256 k of a row
-// weights rounded to fp16 with their scale (instead of exact products scaled in fp32)
-__host__ __device__ constexpr bool gr_prescale(int nt) { return nt >= 4; }
-__host__ __device__ constexpr bool gr_sums(int fmt, int nt) { return fmt == CUTB_Q4_K && !gr_prescale(nt); }
-__host__ __device__ constexpr uint32_t gr_act_bytes(int fmt, int nt) { return 4096u * nt + (gr_sums(fmt, nt) ? 256u * nt : 0u); }
+__host__ __device__ constexpr bool gr_sums(int fmt) { return fmt == CUTB_Q4_K; }
+__host__ __device__ constexpr uint32_t gr_act_bytes(int fmt, int nt) { return 4096u * nt + (gr_sums(fmt) ? 256u * nt : 0u); }
 __host__ __device__ constexpr uint32_t gr_stage(int fmt, int nt) { return GR_ROWS * gr_chunk(fmt) + gr_act_bytes(fmt, nt); }
 __host__ __device__ constexpr uint32_t gr_red(int nt) { return 8u * 1024u * nt + 8u * nt * GR_PITCH * 4u; }  // the k groups' sums, and a tile
 
@@ -106,12 +105,12 @@ template <int FMT, bool AF32, int NT> __global__ void __launch_bounds__(256) row
       }
     }
     v[i] = __half_as_ushort(x);
-    if constexpr (gr_sums(FMT, NT)) sum += __half2float(x);
+    if constexpr (gr_sums(FMT)) sum += __half2float(x);
   }
   uint8_t *unit = p.acts + (size_t)(kb / 8) * gr_act_bytes(FMT, NT);
   *reinterpret_cast<uint4 *>(unit + (((kb % 8) * NT + nt) * 32 + lane) * 16) =
       make_uint4(v[0] | (uint32_t)v[1] << 16, v[2] | (uint32_t)v[3] << 16, v[4] | (uint32_t)v[5] << 16, v[6] | (uint32_t)v[7] << 16);
-  if constexpr (gr_sums(FMT, NT)) {
+  if constexpr (gr_sums(FMT)) {
     sum += __shfl_xor_sync(0xffffffffu, sum, 1);
     sum += __shfl_xor_sync(0xffffffffu, sum, 2);
     if (t == 0) reinterpret_cast<float *>(unit + 4096 * NT)[((kb % 8) * NT + nt) * 8 + g] = sum;
@@ -148,7 +147,7 @@ __device__ __forceinline__ void gr_bytes(uint32_t x, uint32_t &p01, uint32_t &p2
 }
 
 // One block (32 k) of a warp: its 32 rows (four per lane: f[row] = halves 0-1, 2-3 | 4-5, 6-7) and every group of eight
-// activation rows.  sc / mn: the rows' scales and minima, as fp32 or (PRE) applied already.
+// activation rows.  sc / mn: the rows' scales and minima.
 template <int FMT, int NT>
 __device__ __forceinline__ void gr_block(float (&acc)[2][NT][4], const uint32_t (&f)[4][4], const float (&sc)[4], const float (&mn)[4], uint32_t act,
                                          uint32_t sums) {
@@ -156,23 +155,18 @@ __device__ __forceinline__ void gr_block(float (&acc)[2][NT][4], const uint32_t 
   for (int nt = 0; nt < NT; ++nt) {
     const uint4 b = gr_lds4(act + nt * 512);
     float2 sx = make_float2(0.f, 0.f);
-    if constexpr (gr_sums(FMT, NT)) sx = *reinterpret_cast<const float2 *>(__cvta_shared_to_generic(sums + nt * 32));
+    if constexpr (gr_sums(FMT)) sx = *reinterpret_cast<const float2 *>(__cvta_shared_to_generic(sums + nt * 32));
 #pragma unroll
     for (int mt = 0; mt < 2; ++mt) {
       const uint32_t (&r0)[4] = f[2 * mt], (&r1)[4] = f[2 * mt + 1];
-      if constexpr (gr_prescale(NT)) {
-        gr_mma(acc[mt][nt], r0[0], r1[0], r0[1], r1[1], b.x, b.y);
-        gr_mma(acc[mt][nt], r0[2], r1[2], r0[3], r1[3], b.z, b.w);
-      } else {
-        float c[4] = {0.f, 0.f, 0.f, 0.f};
-        gr_mma(c, r0[0], r1[0], r0[1], r1[1], b.x, b.y);
-        gr_mma(c, r0[2], r1[2], r0[3], r1[3], b.z, b.w);
+      float c[4] = {0.f, 0.f, 0.f, 0.f};
+      gr_mma(c, r0[0], r1[0], r0[1], r1[1], b.x, b.y);
+      gr_mma(c, r0[2], r1[2], r0[3], r1[3], b.z, b.w);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int r = 2 * mt + (e >> 1);
-          acc[mt][nt][e] = fmaf(sc[r], c[e], acc[mt][nt][e]);
-          if constexpr (gr_sums(FMT, NT)) acc[mt][nt][e] = fmaf(-mn[r], (e & 1) ? sx.y : sx.x, acc[mt][nt][e]);
-        }
+      for (int e = 0; e < 4; ++e) {
+        const int r = 2 * mt + (e >> 1);
+        acc[mt][nt][e] = fmaf(sc[r], c[e], acc[mt][nt][e]);
+        if constexpr (gr_sums(FMT)) acc[mt][nt][e] = fmaf(-mn[r], (e & 1) ? sx.y : sx.x, acc[mt][nt][e]);
       }
     }
   }
@@ -181,7 +175,6 @@ __device__ __forceinline__ void gr_block(float (&acc)[2][NT][4], const uint32_t 
 template <int FMT, int NT>
 __global__ void __launch_bounds__(GR_THREADS, 1) qgemv_rows_kernel(const __grid_constant__ CUtensorMap map_w, const GrParams p) {
   constexpr uint32_t CHUNK = gr_chunk(FMT), WB = GR_ROWS * CHUNK, AB = gr_act_bytes(FMT, NT), STAGE = WB + AB;
-  constexpr bool PRE = gr_prescale(NT);
   extern __shared__ __align__(128) uint8_t gr_raw[];
   uint8_t *gr_smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(gr_raw) + 127) & ~uintptr_t(127));  // (copied boxes)
   __shared__ uint32_t last_s;
@@ -258,16 +251,7 @@ __global__ void __launch_bounds__(GR_THREADS, 1) qgemv_rows_kernel(const __grid_
           const uint32_t x = __byte_perm(w1, w4, t == 3 ? 0x5432u : 0x3210u);
           gr_low<8>(x, f0[r][0], f0[r][1]), gr_high<8>(x, f0[r][2], f0[r][3]);
           gr_low<8>(w5, f1[r][0], f1[r][1]), gr_high<8>(w5, f1[r][2], f1[r][3]);
-          if constexpr (PRE) {
-            const __half2 d0 = u32_as_h2(__byte_perm(w0, 0, 0x1010)), d1 = u32_as_h2(__byte_perm(w4, 0, 0x3232));
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              f0[r][i] = h2_as_u32(__hmul2(u32_as_h2(f0[r][i]), d0));
-              f1[r][i] = h2_as_u32(__hmul2(u32_as_h2(f1[r][i]), d1));
-            }
-          } else {
-            s0[r] = h2f_bits(w0 & 0xFFFFu), s1[r] = h2f_bits(w4 >> 16);
-          }
+          s0[r] = h2f_bits(w0 & 0xFFFFu), s1[r] = h2f_bits(w4 >> 16);
         } else if constexpr (FMT == CUTB_Q8_0) {
           // pairs of 34-byte blocks = 17 aligned words: {d0,u0} {u1,u2} ... {u13,u14} {u15,d1} then 8 words of block 1
           const uint32_t w0 = gr_lds(pa), w8 = gr_lds(pa + 32);
@@ -275,16 +259,7 @@ __global__ void __launch_bounds__(GR_THREADS, 1) qgemv_rows_kernel(const __grid_
           gr_bytes(__byte_perm(gr_lds(pa + 20 + 4 * t), w0, t == 3 ? 0x7610u : 0x3210u), f0[r][2], f0[r][3]);
           gr_bytes(gr_lds(pa + 36 + 4 * t), f1[r][0], f1[r][1]);
           gr_bytes(gr_lds(pa + 52 + 4 * t), f1[r][2], f1[r][3]);
-          if constexpr (PRE) {
-            const __half2 d0 = u32_as_h2(__byte_perm(w0, 0, 0x1010)), d1 = u32_as_h2(__byte_perm(w8, 0, 0x3232));
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              f0[r][i] = h2_as_u32(__hmul2(u32_as_h2(f0[r][i]), d0));
-              f1[r][i] = h2_as_u32(__hmul2(u32_as_h2(f1[r][i]), d1));
-            }
-          } else {
-            s0[r] = h2f_bits(w0 & 0xFFFFu), s1[r] = h2f_bits(w8 >> 16);
-          }
+          s0[r] = h2f_bits(w0 & 0xFFFFu), s1[r] = h2f_bits(w8 >> 16);
         } else {
           const uint4 h = gr_lds4(pa);
           const uint32_t x = gr_lds(pa + 16 + 32 * kg + 4 * t), y = gr_lds(pa + 32 + 32 * kg + 4 * t);
@@ -297,14 +272,6 @@ __global__ void __launch_bounds__(GR_THREADS, 1) qgemv_rows_kernel(const __grid_
           s0[r] = d * (float)(sc & 0xFFu), s1[r] = d * (float)(sc >> 8), m0[r] = dmin * (float)(mn & 0xFFu), m1[r] = dmin * (float)(mn >> 8);
           gr_low<0>(x, f0[r][0], f0[r][1]), gr_low<0>(y, f0[r][2], f0[r][3]);
           gr_high<0>(x, f1[r][0], f1[r][1]), gr_high<0>(y, f1[r][2], f1[r][3]);
-          if constexpr (PRE) {
-            const __half2 a0 = __float2half2_rn(s0[r]), a1 = __float2half2_rn(s1[r]), b0 = __float2half2_rn(-m0[r]), b1 = __float2half2_rn(-m1[r]);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              f0[r][i] = h2_as_u32(__hfma2(u32_as_h2(f0[r][i]), a0, b0));
-              f1[r][i] = h2_as_u32(__hfma2(u32_as_h2(f1[r][i]), a1, b1));
-            }
-          }
         }
       }
       gr_block<FMT, NT>(acc, f0, s0, m0, st + act0, st + sum0);
@@ -428,7 +395,7 @@ struct GrPlan {
 
 GrPlan gr_plan(const cutb_qmatmul_desc &d, uint32_t sms, size_t smem) {
   GrPlan pl{};
-  pl.nt = d.M <= 16 ? 2 : 4;
+  pl.nt = GR_NT;
   pl.tiles = (d.N + GR_ROWS - 1) / GR_ROWS;
   const uint32_t total = pl.tiles * (d.K / 256);
   pl.grid = total < sms ? total : sms;
@@ -493,10 +460,6 @@ template <int FMT, int NT> int gr_launch(const cutb_qmatmul_desc &d, const GrPar
   return CUTB_OK;
 }
 
-template <int FMT> int gr_dispatch(const cutb_qmatmul_desc &d, const GrParams &p, const GrPlan &pl, cudaStream_t stream) {
-  return pl.nt == 2 ? gr_launch<FMT, 2>(d, p, pl, stream) : gr_launch<FMT, 4>(d, p, pl, stream);
-}
-
 }  // namespace
 
 bool qgemv_rows_supported(const cutb_qmatmul_desc &d) {
@@ -514,13 +477,10 @@ bool qgemv_rows_supported(const cutb_qmatmul_desc &d) {
 //                  10.2; 16384 x 1024 alone loses 3 % up to 12 rows, and wins 25 % from 13); and where both are small, 1024 x 1000
 //                  7.2 -> 6.2, 2048 x 768 8.1 -> 7.1.  Q4_K the same within 4 % either way (its minima cost a second product): stays.
 //                  Eight rows, which fill the int8 kernel's columns: 12.8 -> 14.3: stays.
-//   17 to 32 fp16 rows  Q8_0 from 8 M weights on 24 tiles (3072 x 4096 x 0.84 to 0.88, 4096 x 3072 x 1.01) and 14 M weights on any (8192 x
-//                  1536 15.9 -> 17.0, 4096 x 2048 x 1.03; 14336 x 1024 x 0.85 to 0.92, 8192 x 8192 42 -> 27).  Q4_0 from 16 M weights on
-//                  48 tiles (4096 x 6144 x 0.93 to 0.98, 8192 x 8192 x 0.86, 28672 x 8192 72 -> 63), or 32 with K up to 4096 (4096 x 4096
-//                  x 0.92 to 0.97, but 6144 x 4096 x 0.99 to 1.04, 8192 x 4096 18.5 -> 20.3, 14336 x 4096 x 0.99 to 1.01, 16384 x 2048
-//                  19.4 -> 21.9).  Q4_K 4096 x 4096 x 1.03, 11008 x 4096 x 1.06: stays.
+//   17 to 32 fp16 rows  The kernel is the tensor-core GEMM's for few rows (qgemm_few.cu) on either side; the line is where the variant that
+//                  is reported for them changes.
 //   fp32 rows      Rounded to fp16 by either kernel; here in the same pass that orders them.  All three formats gain on all of 35 weights
-//                  from 512 x 512 to 28672 x 8192: x 0.44 to 0.94 (9 and 16 rows), x 0.48 to 0.98 (17 to 32 rows, 8192 x 512 x 1.01).
+//                  from 512 x 512 to 28672 x 8192: x 0.44 to 0.94 (9 and 16 rows); 17 to 32 rows take qgemm_few.cu.
 bool qgemv_rows_faster(const cutb_qmatmul_desc &d) {
   if (d.a_dtype == CUTB_F32) return true;
   if (d.format == CUTB_Q4_K) return false;
@@ -533,6 +493,7 @@ bool qgemv_rows_faster(const cutb_qmatmul_desc &d) {
 }
 
 uint64_t qgemv_rows_workspace(const cutb_qmatmul_desc &d) {
+  if (d.M > 8 * GR_NT) return qgemm_few_workspace(d, false);
   DeviceInfo di;
   uint32_t sms = 148;
   size_t smem = 232448;
@@ -546,6 +507,7 @@ bool qgemv_rows_fits(const cutb_qmatmul_desc &d) {
 }
 
 int qgemv_rows_launch(const cutb_qmatmul_desc &d, cudaStream_t stream) {
+  if (d.M > 8 * GR_NT) return qgemm_few_launch(d, stream);
   DeviceInfo di;
   if (int rc = get_device_info(&di)) return rc;
   const GrPlan pl = gr_plan(d, (uint32_t)di.sm_count, di.smem_optin);
@@ -558,9 +520,9 @@ int qgemv_rows_launch(const cutb_qmatmul_desc &d, cudaStream_t stream) {
   p.arrived = reinterpret_cast<uint32_t *>(p.acts + pl.acts);
   p.shares = reinterpret_cast<float *>(p.acts + pl.acts + pl.arrived);
   switch (d.format) {
-    case CUTB_Q8_0: return gr_dispatch<CUTB_Q8_0>(d, p, pl, stream);
-    case CUTB_Q4_0: return gr_dispatch<CUTB_Q4_0>(d, p, pl, stream);
-    default: return gr_dispatch<CUTB_Q4_K>(d, p, pl, stream);
+    case CUTB_Q8_0: return gr_launch<CUTB_Q8_0, GR_NT>(d, p, pl, stream);
+    case CUTB_Q4_0: return gr_launch<CUTB_Q4_0, GR_NT>(d, p, pl, stream);
+    default: return gr_launch<CUTB_Q4_K, GR_NT>(d, p, pl, stream);
   }
 }
 
