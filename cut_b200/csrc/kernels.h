@@ -50,6 +50,10 @@ bool qgemm_few_supported(const cutb_qmatmul_desc &d);
 uint64_t qgemm_few_workspace(const cutb_qmatmul_desc &d, bool direct);
 bool qgemm_few_fits(const cutb_qmatmul_desc &d);
 int qgemm_few_launch(const cutb_qmatmul_desc &d, cudaStream_t stream);
+// and for many rows over GGUF blocks, tiles of 256 weight rows by pairs of CTAs, weights through tensor memory (qgemm_wide.cu).  _plan: the
+// activation rows of a tile and an estimate of the time (us), 0 where it cannot run; fp16 rows `stride` bytes apart.
+uint32_t qgemm_wide_plan(const cutb_qmatmul_desc &d, float *time);
+int qgemm_wide_launch(const cutb_qmatmul_desc &d, const void *a16, uint64_t stride, uint32_t T, cudaStream_t stream);
 
 int dequant_launch(int format, const void *raw, float *out, uint32_t rows, uint32_t cols, uint32_t ldo,
                    cudaStream_t stream);

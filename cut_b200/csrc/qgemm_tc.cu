@@ -40,6 +40,9 @@
 // Every wait is bounded; on expiry the CTA records CUTB_ERR_TIMEOUT in the
 // caller's status word, skips its remaining work, frees its tensor memory and
 // returns.
+//
+// Blocks go to qgemm_few.cu (up to 64 rows) and qgemm_wide.cu instead where those are faster (qgemm_tc_launch); what stays here are the planes,
+// and products whose few tiles need their K shared out.
 #include <cuda.h>
 #include <cuda_fp16.h>
 
@@ -431,7 +434,7 @@ uint32_t tc_ksub(uint32_t mb) { return mb <= 2 ? 2u : 1u; }
 // with partial sums and of those without, but for one (Q4_K 527 x 8192 x 2048 32.5, best 31.1).  us, one block and K whole as plans for
 // few rows were -> now: Q8_0 333 x 11008 x 4096 94 -> 40 (3 blocks, 4 shares), 256 x 8192 x 8192 82 -> 54 (2, 2), 150 x 4096 x 4096 42 ->
 // 20 (2, 4); Q4_K 512 x 4096 x 4096 34 -> 28 (2, 2), 1500 x 4096 x 4096 92 -> 48 (3, 1); Q4_0 200 x 4096 x 4096 33 -> 19 (2, 4).
-void tc_shape_plan(const cutb_qmatmul_desc &d, uint32_t sm_count, bool split, uint32_t *mb_out, uint32_t *ksplit_out) {
+float tc_shape_plan(const cutb_qmatmul_desc &d, uint32_t sm_count, bool split, uint32_t *mb_out, uint32_t *ksplit_out) {
   static const struct { float stage[TC_MAX_MB], fixed[TC_MAX_MB]; } q8 = {{0.555f, 0.57f, 0.63f, 0.71f}, {6.f, 8.f, 9.f, 10.f}},
       q4 = {{0.41f, 0.45f, 0.59f, 0.69f}, {6.f, 8.f, 9.f, 10.f}}, planes = {{0.58f, 0.56f, 0.65f, 0.71f}, {6.f, 8.f, 9.f, 11.f}};
   const auto &cost = d.layout == CUTB_LAYOUT_KN_PLANES ? planes : (d.format == CUTB_Q8_0 ? q8 : q4);
@@ -448,6 +451,7 @@ void tc_shape_plan(const cutb_qmatmul_desc &d, uint32_t sm_count, bool split, ui
       if (t < best) best = t, *mb_out = mb, *ksplit_out = ks;
     }
   }
+  return best;
 }
 uint64_t tc_cast_bytes(const cutb_qmatmul_desc &d) {
   return d.a_dtype == CUTB_F32 ? (((uint64_t)d.M * d.K * sizeof(__half) + 15) & ~(uint64_t)15) : 0;
@@ -490,13 +494,13 @@ int qgemm_tc_launch(const cutb_qmatmul_desc &d, cudaStream_t stream) {
   p.ldb = d.ldb;
   p.lds = d.lds;
   p.blocksK = (d.K + 31) / 32;
-  tc_shape_plan(d, (uint32_t)di.sm_count, true, &p.mb, &p.ksplit);
+  float time = tc_shape_plan(d, (uint32_t)di.sm_count, true, &p.mb, &p.ksplit);
   const uint64_t cast_bytes = tc_cast_bytes(d), partial_bytes = p.ksplit > 1 ? (uint64_t)p.ksplit * d.M * d.N * sizeof(float) : 0;
   p.partial = nullptr;
   if (p.ksplit > 1) {
     // without room for the partial sums: the best plan that leaves K whole (it asks for none)
     if (!d.workspace || d.workspace_bytes < cast_bytes + partial_bytes || reinterpret_cast<uintptr_t>(d.workspace) % 16 != 0) {
-      tc_shape_plan(d, (uint32_t)di.sm_count, false, &p.mb, &p.ksplit);
+      time = tc_shape_plan(d, (uint32_t)di.sm_count, false, &p.mb, &p.ksplit);
     } else {
       p.partial = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(d.workspace) + cast_bytes);
     }
@@ -522,6 +526,13 @@ int qgemm_tc_launch(const cutb_qmatmul_desc &d, cudaStream_t stream) {
     set_last_error("qgemm: shared memory too small for the tile rings");
     return CUTB_ERR_UNSUPPORTED;
   }
+  // Pairs of CTAs with the weights in tensor memory, unless this kernel's shares of K fill the SMs better.  The estimates of this one are
+  // up to 15 % low, hence the margin.  us, this kernel / that one, of 50 random shapes: Q8_0 333 x 11008 x 4096 55.9 / 60.8 and Q4_0 272 x
+  // 12032 x 1248 27.0 / 44.2 stay; Q4_K 512 x 4096 x 14336 62.2 / 53.8, x 6144 45.3 / 28.3, 157 x 2560 x 23552 55.5 / 28.7, Q8_0 565 x 6912
+  // x 28352 301 / 181, Q4_0 1763 x 4096 x 26880 364 / 294 go there.
+  float wide_time = 0.f;
+  uint32_t wide = qgemm_wide_plan(d, &wide_time);
+  if (wide && wide_time > 1.08f * time) wide = 0;
   const void *a16 = d.A;
   uint64_t stride = (uint64_t)d.lda * sizeof(__half);
   if (d.a_dtype == CUTB_F32) {
@@ -535,6 +546,7 @@ int qgemm_tc_launch(const cutb_qmatmul_desc &d, cudaStream_t stream) {
     a16 = d.workspace;
     stride = (uint64_t)d.K * sizeof(__half);
   }
+  if (wide) return qgemm_wide_launch(d, a16, stride, wide, stream);
   CUtensorMap map;
   if (int rc = make_tmap_a(&map, a16, d.M, d.K, stride)) return rc;
   int rc;
