@@ -623,8 +623,8 @@ int sk_launch(const CUtensorMap &mapA, const CUtensorMap &mapW, const SkParams &
 
 }  // namespace
 
-// Up to 64 tokens always (blocks whose scratch holds what qgemm_few.cu needs go there first); up to 128 when the prefill kernel's 128-row tiles would leave more than half of the SMs
-// idle (there its one-pass epilogue beats this kernel's split and fix-up once the SMs are covered).
+// Up to 64 tokens always (blocks whose scratch holds what qgemm_few.cu needs go there first); up to 128 when the prefill kernel's 128-row
+// tiles would leave more than half of the SMs idle (there its one-pass epilogue beats this kernel's split and fix-up once the SMs are covered).
 bool qgemm_skinny_applies(const cutb_qmatmul_desc &d) {
   if (d.M > 128 || d.K % SK_UNIT_K != 0) return false;
   if (d.M <= 64) return true;

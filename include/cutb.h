@@ -82,8 +82,8 @@ enum {
                                CUTB_LAYOUT_KN_PLANES (K % 128 == 0; above four rows what CUTB_VARIANT_AUTO picks there) */
   CUTB_VARIANT_GEMV_PLANES = 3, /* decode over CUTB_LAYOUT_KN_PLANES (the reference's run-time layout), M <= 4: coalesced
                                    column groups, K split over warps and blocks */
-  CUTB_VARIANT_ROWS_MMA = 4 /* batched decode: fp16 warp MMAs on the quants of GGUF blocks (K % 256 == 0), 9 <= M <= 32, operands as
-                               CUTB_VARIANT_GEMM_TC rounds them (up to 16 rows the weights are exact); needs the scratch of
+  CUTB_VARIANT_ROWS_MMA = 4 /* batched decode over GGUF blocks (K % 256 == 0), 9 <= M <= 32: up to 16 rows fp16 warp MMAs on the quants
+                               (weights exact), above 16 tcgen05 MMAs, operands as CUTB_VARIANT_GEMM_TC rounds them; needs the scratch of
                                cutb_qmatmul_workspace_bytes.  What CUTB_VARIANT_AUTO picks where it measured faster */
 };
 
@@ -137,10 +137,10 @@ enum { CUTB_FLAG_NO_OVERLAP = 1, CUTB_FLAG_ACT_16BIT = 2, CUTB_FLAG_A_RMSNORM = 
  * CUTB_ERR_RANGE in *status (the output then holds inf / NaN where such a value took part);
  * weight products below 6e-8 flush to zero.  Callers whose activations can exceed the fp16
  * range select CUTB_VARIANT_GENERIC, or scale A down and C up.  Accumulation and C are fp32.
- * Up to 128 activation rows CUTB_VARIANT_GEMM_TC runs a kernel of its own (tokens as the MMA's M
- * operand, K shared out over all SMs); it is launched with programmatic stream serialization
- * like the decode mat-vec (it waits for the previous kernel only before it reads A and before it
- * stores), which CUTB_FLAG_NO_OVERLAP switches off.
+ * Up to 128 activation rows CUTB_VARIANT_GEMM_TC runs kernels of their own (K shared out over all SMs);
+ * they are launched with programmatic stream serialization
+ * like the decode mat-vec (they wait for the previous kernel only before they read A and before they
+ * store), which CUTB_FLAG_NO_OVERLAP switches off.
  */
 typedef struct cutb_qmatmul_desc {
   int32_t format;      /* CUTB_Q8_0 / CUTB_Q4_0 / CUTB_Q4_K */
