@@ -77,6 +77,11 @@ __device__ __forceinline__ void pack_digits(const int (&v)[8], uint32_t (&hi)[2]
 }
 
 constexpr float GV_QMAX = 32512.f;
+// Steps of the second level (the residual of fp32 rows, at most half a step of the first) per step e of the first.  Two digits hold 32639, so the
+// residual x - x^ e, up to e (1/2 + 32512 r) with r the error of e times its inverse (2^-23 where that is approximated) and of x times it
+// (2^-24 where the product is rounded by itself), must not reach e * 32639 / GV_STEPS2.  With 2 * 32512 steps it did.
+constexpr float GV_STEPS2 = 64000.f;
+static_assert(GV_STEPS2 * (0.5f + 32512.f * (0x1p-23f + 0x1p-24f)) < 32639.f, "the second level wraps");
 
 // One activation row at either precision, or two at one 16-bit level (qgemv_row.cu).
 struct RowPlan {

@@ -323,8 +323,8 @@ __device__ __forceinline__ void stage_activations(const GvParams &p, uint8_t *ac
     probe += __shfl_xor_sync(0xffffffffu, probe, 1);
     probe += __shfl_xor_sync(0xffffffffu, probe, 2);
     const bool finite = (amax < __int_as_float(0x7f800000)) && (probe == probe);
-    const float inv = (amax > 0.f && finite) ? GV_QMAX / amax : 0.f;
-    float e = finite ? amax * (1.0f / GV_QMAX) : __int_as_float(0x7fc00000);
+    const float e = finite ? amax * (1.0f / GV_QMAX) : __int_as_float(0x7fc00000);
+    const float inv = (amax > 0.f && finite) ? 1.0f / e : 0.f;  // (of e itself: both roundings in one, see GV_STEPS2)
     int v[8], isum = 0;
     uint32_t whi[2], wlo[2];
 #pragma unroll
@@ -351,8 +351,8 @@ __device__ __forceinline__ void stage_activations(const GvParams &p, uint8_t *ac
       }
     }
     if constexpr (TWO) {
-      // second 16-bit level: the residual x - x^ e, at scale e / 65024
-      const float e2 = e * (1.0f / (2.f * GV_QMAX)), inv2 = inv * (2.f * GV_QMAX);
+      // second 16-bit level: the residual x - x^ e, at scale e / GV_STEPS2
+      const float e2 = e * (1.0f / GV_STEPS2), inv2 = inv * GV_STEPS2;
       int w[8], isum2 = 0;
       uint32_t rhi[2], rlo[2];
 #pragma unroll

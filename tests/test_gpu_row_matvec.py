@@ -95,6 +95,31 @@ def test_values_at_the_ends_of_the_range(fmt):
     assert np.isnan(_run(fmt, A, W, N)).all()
 
 
+def _near_halves(rng, rows, K):
+    """fp32 rows whose values lie close to halfway between two steps of their block's 16-bit scale (maximum / 32512), in blocks whose maximum
+    times that scale's inverse is as far from 32512 as rounding leaves it: the residuals that the second level holds are the largest there are."""
+    q = np.float32(32512)
+    most = (1 + rng.random(1 << 18)).astype(np.float32)
+    off = (q / most).astype(np.float64) * (most * (np.float32(1) / q)).astype(np.float64) - 1
+    most = most[np.argsort(-np.abs(off))[: rows * K // 32]]
+    step = (most * (np.float32(1) / q)).astype(np.float64)[:, None]
+    at = rng.integers(24000, 32400, (most.size, 32)) + 0.5 + rng.uniform(-0.012, 0.012, (most.size, 32))
+    x = (at * step * rng.choice([-1.0, 1.0], at.shape)).astype(np.float32)
+    x[:, 0] = most
+    return x.reshape(rows, K)
+
+
+@pytest.mark.parametrize("fmt", FMTS)
+@pytest.mark.parametrize("M,K,N", [(1, 4096, 1200), (1, 1280, 300), (2, 4096, 1200), (4, 2048, 600), (8, 1024, 600)])
+def test_residuals_that_fill_the_second_level(fmt, M, K, N):
+    """The second level of fp32 rows holds the residual of the first in two int8 digits, which wrap above 32639."""
+    W, A = synth.make_weights(fmt, N, K, M), _near_halves(np.random.default_rng(K + M), M, K)
+    want = A.astype(np.float64) @ O.dequant_rows(fmt, W, N, K).astype(np.float64).T
+    got = _run(fmt, A, W, N)
+    for m in range(M):
+        assert _err(got[m], want[m]) <= TOL[32], m
+
+
 @pytest.mark.parametrize("fmt", [synth.Q4_0, synth.Q4_K])
 @pytest.mark.parametrize("M", [3, 4, 5, 8])
 @pytest.mark.parametrize("K,N", [(256, 2), (512, 1200), (1280, 2401), (2048, 9500), (4096, 200), (4096, 5000), (3072, 19100), (5120, 9600)])
