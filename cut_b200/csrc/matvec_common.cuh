@@ -77,6 +77,7 @@ __device__ __forceinline__ void pack_digits(const int (&v)[8], uint32_t (&hi)[2]
 }
 
 constexpr float GV_QMAX = 32512.f;
+constexpr float GV_MOST = 3e38f;  // of a scale's inverse: below 1e-34 the scale stays at what it can hold
 // Steps of the second level (the residual of fp32 rows, at most half a step of the first) per step e of the first.  Two digits hold 32639, so the
 // residual x - x^ e, up to e (1/2 + 32512 r) with r the error of e times its inverse (2^-23 where that is approximated) and of x times it
 // (2^-24 where the product is rounded by itself), must not reach e * 32639 / GV_STEPS2.  With 2 * 32512 steps it did.

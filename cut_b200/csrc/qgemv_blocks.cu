@@ -323,8 +323,8 @@ __device__ __forceinline__ void stage_activations(const GvParams &p, uint8_t *ac
     probe += __shfl_xor_sync(0xffffffffu, probe, 1);
     probe += __shfl_xor_sync(0xffffffffu, probe, 2);
     const bool finite = (amax < __int_as_float(0x7f800000)) && (probe == probe);
-    const float e = finite ? amax * (1.0f / GV_QMAX) : __int_as_float(0x7fc00000);
-    const float inv = (amax > 0.f && finite) ? 1.0f / e : 0.f;  // (of e itself: both roundings in one, see GV_STEPS2)
+    const float e = finite ? fmaxf(amax * (1.0f / GV_QMAX), 1.0f / GV_MOST) : __int_as_float(0x7fc00000);
+    const float inv = finite ? fminf(1.0f / e, GV_MOST) : 0.f;  // (of e itself: both roundings in one, see GV_STEPS2)
     int v[8], isum = 0;
     uint32_t whi[2], wlo[2];
 #pragma unroll
@@ -352,7 +352,9 @@ __device__ __forceinline__ void stage_activations(const GvParams &p, uint8_t *ac
     }
     if constexpr (TWO) {
       // second 16-bit level: the residual x - x^ e, at scale e / GV_STEPS2
-      const float e2 = e * (1.0f / GV_STEPS2), inv2 = inv * GV_STEPS2;
+      const float e2 = e * (1.0f / GV_STEPS2);
+      float inv2 = inv * GV_STEPS2;
+      if (inv2 > GV_MOST) inv2 = 0.f;  // (blocks below 1e-30: one level)
       int w[8], isum2 = 0;
       uint32_t rhi[2], rlo[2];
 #pragma unroll

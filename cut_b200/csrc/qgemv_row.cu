@@ -45,7 +45,6 @@ constexpr uint32_t RW_MAX_DEPTH = 8;
 constexpr uint32_t RW_SUMS = RW_WARPS + 4;  // floats from one row's sums to the next: a thread reads them sixteen bytes at a time
 constexpr uint32_t RW_GROUP = 8;                     // tiles whose sums a block keeps before it writes them out
 constexpr float RW_LEVEL2 = 1.0f / GV_STEPS2;         // the second level's scale beside the first's
-constexpr float RW_MOST = 3e38f;
 constexpr float RW_MAGIC = 12582912.f;               // 1.5 * 2^23: x + RW_MAGIC holds rint(x) in its low bits, |x| < 2^22
 
 
@@ -193,9 +192,8 @@ __device__ __forceinline__ void stage_row(const RowParams &p, uint8_t *act, floa
       amax = max_or_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
       amax = max_or_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
       const bool finite = amax < __int_as_float(0x7f800000);
-      // (below 1e-34 the scale stays at what its inverse can hold)
-      const float e = finite ? fmaxf(amax * (1.0f / GV_QMAX), 1.0f / RW_MOST) : __int_as_float(0x7fc00000);
-      const float inv = finite ? fminf(reciprocal(e), RW_MOST) : 0.f;  // (of e itself: both roundings in one, see GV_STEPS2)
+      const float e = finite ? fmaxf(amax * (1.0f / GV_QMAX), 1.0f / GV_MOST) : __int_as_float(0x7fc00000);
+      const float inv = finite ? fminf(reciprocal(e), GV_MOST) : 0.f;  // (of e itself: both roundings in one, see GV_STEPS2)
       const uint32_t pass = kb >> 3 << 1 | (kb & 1), pr = (kb & 7) >> 1;  // [granule][pass], the lane pair
       const bool even = (kb & 1) == 0;
       // v: floats whose low 16 bits are the integers.  A block's digits become eight words in the order in which the weights' aligned words
@@ -240,7 +238,7 @@ __device__ __forceinline__ void stage_row(const RowParams &p, uint8_t *act, floa
       if constexpr (FMT != CUTB_Q8_0) sum = e * (float)sum_of(v);
       if constexpr (S::TWO) {  // the residual x - x^ e in steps of e / GV_STEPS2
         float inv2 = inv * GV_STEPS2;
-        if (inv2 > RW_MOST) inv2 = 0.f;  // (blocks below 1e-30: one level)
+        if (inv2 > GV_MOST) inv2 = 0.f;  // (blocks below 1e-30: one level)
         float r[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) r[i] = fmaf(fmaf(-(v[i] - RW_MAGIC), e, x[i]), inv2, RW_MAGIC);

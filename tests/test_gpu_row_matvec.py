@@ -120,6 +120,20 @@ def test_residuals_that_fill_the_second_level(fmt, M, K, N):
         assert _err(got[m], want[m]) <= TOL[32], m
 
 
+@pytest.mark.parametrize("fmt", FMTS)
+@pytest.mark.parametrize("M", [2, 4, 8])
+@pytest.mark.parametrize("size,tol", [(1e-29, TOL[32]), (1e-31, TOL[16]), (1e-36, 0.05)])
+def test_rows_of_small_values(fmt, M, size, tol):
+    """Several fp32 rows, one of them so small that the inverse of a block's scale leaves the range of fp32: first the second level's (its steps
+    are then left out: 16 bits), then the first's (steps of 3e-39 beside values of 1e-36: 1 %, and fp32's own subnormal values)."""
+    K, N = 2048, 600
+    A, W, dense = _case(fmt, M, K, N, np.float32, 9 + fmt)
+    A[M - 1] *= np.float32(size)
+    want, got = A.astype(np.float64) @ dense.T, _run(fmt, A, W, N)
+    for m in range(M):
+        assert _err(got[m], want[m]) <= (tol if m == M - 1 else TOL[32]), m
+
+
 @pytest.mark.parametrize("fmt", [synth.Q4_0, synth.Q4_K])
 @pytest.mark.parametrize("M", [3, 4, 5, 8])
 @pytest.mark.parametrize("K,N", [(256, 2), (512, 1200), (1280, 2401), (2048, 9500), (4096, 200), (4096, 5000), (3072, 19100), (5120, 9600)])
