@@ -378,7 +378,7 @@ bool few_matvec_plan(const cutb_qmatmul_desc &d, const DeviceInfo &di, uint32_t 
   const uint32_t tiles = (d.N + FW_ROWS - 1) / FW_ROWS;
   pl->grid_x = tiles < sms ? tiles : sms;
   pl->groups = 1;
-  pl->fixed = false;
+  pl->fixed = pl->beside = false;
   const size_t stage = (size_t)FW_GRANULES * FW_ROWS * granule_bytes(d.format);
   const size_t fixed = (size_t)gran_per_split * cp * (512 + 32) + (size_t)FW_WARPS * cp * FW_ROWS * 4 + FW_MAX_DEPTH * (FW_GROUPS + 1) * 8;
   const size_t half = di.smem_per_sm > 2048 ? di.smem_per_sm / 2 - 1024 : di.smem_optin / 2;

@@ -8,8 +8,8 @@
 // have come from L2, 0.5 us until they are digits.  So the copies run ahead of that chain, and what follows it is short:
 //  * The weights come through a ring of 18 KB stages, 16 rows of eight granules of 256 weights (four of Q8_0), one tensor copy each:
 //    the weight seen as [granule][row][bytes] lands with rows 144 (272) bytes apart, on which the fragment loads meet no bank twice.
-//    A block keeps under half an SM, so that the next launch's block fills its ring (92 KB) beside this one.  A chain that only
-//    copies takes 5.0 to 5.2 us a launch this way, 5.4 with sixteen padded row copies a stage, 7.7 with row copies of 576 bytes.
+//    The ring is as deep as the SM allows (row_matvec_plan).  A chain that only copies takes 5.0 to 5.2 us a launch with five stages,
+//    5.4 with sixteen padded row copies a stage, 7.7 with row copies of 576 bytes.
 //  * Sixteen warps in two groups (Q8_0: four) take stages in turn, a granule per warp, and meet no other warp until the block's sums
 //    are complete: a warp's partial sums go to shared memory per tile, and the epilogue runs once per eight tiles.  A barrier and an
 //    epilogue per tile cost 0.35 us each.
@@ -21,11 +21,11 @@
 //  * A warp stages the activations of the granules that it multiplies, eight neighbouring elements to a lane (whole lines per load:
 //    every block asks L2 for the same 8 KB at once; four-byte loads in block order took twice as long), and goes on without a barrier.
 //    A fused RMSNorm stages x * weight; 1 / rms, a factor of the whole row, meets the sums in the epilogue.
-// Measured, us a launch in a graph of 8 to 32 (before: 16 rows per tile through qgemv_blocks.cu's ring, a barrier per tile): Q4_0
-// 11008 x 4096 8.1 -> 6.5, Q4_0 28672 x 8192 33.6 -> 29, Q8_0 4096 x 4096 with fp32 rows 5.95 -> 5.75.  With the weights in L2 the first
-// takes 4.9: what is left is the wait for stages that were not copied ahead.  Tried and slower for the first: a lane to a row's blocks
-// with dp4a (8.8), rings of cp.async per warp (7.5), the last warp of a group refilling the slot (6.4), eight warps with a unit each in
-// registers before the wait (6.5), releasing the successor after the staging (7.7), stages of four granules (6.5); this: 6.0.
+// Measured, us a launch in a graph over cycled weights (before: 16 rows per tile through qgemv_blocks.cu's ring, a barrier per tile): Q4_0
+// 11008 x 4096 (32 weights) 8.1 -> 6.4, Q4_0 28672 x 8192 (8) 33.4 -> 24.2, Q8_0 4096 x 4096 with fp32 rows (16) 5.95 -> 5.2.  Tried with
+// five stages and slower for the first, in a run where this took 6.0: a lane to a row's blocks with dp4a (8.8), rings of cp.async per
+// warp (7.5), the last warp of a group refilling the slot (6.4), eight warps with a unit each in registers before the wait (6.5),
+// releasing the successor after the staging (7.7), stages of four granules (6.5).
 //
 // Activations are block floating point as in qgemv_blocks.cu: per 32-k block one fp32 scale e and 16-bit integers
 // x^ = rint(x / e), |x^| <= 32512, as two balanced int8 digits; fp32 rows take a second such level for the residual.  The integer dot
@@ -54,6 +54,7 @@ __host__ __device__ constexpr uint32_t rw_granules(int fmt) { return fmt == CUTB
 struct RowParams : GvParams {
   uint32_t depth;   // stages of the ring
   uint32_t groups;  // tiles per group
+  uint32_t box;     // granules of a copy
 };
 
 // int8 MMAs: D = A * B, and D += A * B
@@ -418,8 +419,10 @@ __device__ __forceinline__ void unit_dot(const Unit<FMT> &u, uint32_t x, uint32_
 }
 
 // FIXED: sixteen granules (K = 4096, or such a split): as many stages to a tile as there are groups, one granule per warp for good.
-template <int FMT, int AMODE, int NR, bool FIXED>
-__global__ void __launch_bounds__(RW_THREADS, 2) qgemv_row_kernel(const __grid_constant__ CUtensorMap weights, const RowParams p) {
+// MINB: blocks per SM that the registers are kept for: 2 (56 registers) only where the next launch's block is to copy beside this one, since
+// all instantiations but the fixed ones of a single level spill there (up to 136 bytes a thread).
+template <int FMT, int AMODE, int NR, bool FIXED, int MINB>
+__global__ void __launch_bounds__(RW_THREADS, MINB) qgemv_row_kernel(const __grid_constant__ CUtensorMap weights, const RowParams p) {
   using S = RowShape<FMT, AMODE, NR>;
   constexpr int NV = S::NV;
   constexpr uint32_t NW = RW_WARPS, GPS = S::GPS, STAGE = S::STAGE, GROUPS = NW / GPS;
@@ -465,7 +468,7 @@ __global__ void __launch_bounds__(RW_THREADS, 2) qgemv_row_kernel(const __grid_c
         }
         if (lane == 0) {
           const uint32_t full = full_u + (slot * GROUPS + issued % GROUPS) * 8;
-          mbar_arrive_expect_tx(full, STAGE);
+          mbar_arrive_expect_tx(full, p.box * S::UNIT);
           tma_load_3d(ring_u + slot * STAGE, &weights, 0, row, gs0 + c * GPS, full);
         }
         __syncwarp();
@@ -522,8 +525,9 @@ __global__ void __launch_bounds__(RW_THREADS, 2) qgemv_row_kernel(const __grid_c
       }
     }
   }
-  // With whole rounds of granules a warp has staged just what it will read, else it reads what warps of other groups staged.
-  if (FIXED || ng % NW == 0) __syncwarp();
+  // A warp stages every sixteenth granule.  Where each group has as many stages of every tile, these are the ones it multiplies; else its
+  // stages shift from tile to tile, and it reads what warps of other groups staged.
+  if (FIXED || cpt % GROUPS == 0) __syncwarp();
   else asm volatile("bar.sync 1, %0;" ::"n"(RW_CONSUMERS) : "memory");
 
   // Where this lane reads its column: lanes without one read zeros, at a place in the row that the lanes beside them leave free.
@@ -605,7 +609,7 @@ __global__ void __launch_bounds__(RW_THREADS, 2) qgemv_row_kernel(const __grid_c
   }
 }
 
-template <int FMT, int AMODE, int NR, bool FIXED>
+template <int FMT, int AMODE, int NR, bool FIXED, int MINB>
 int row_launch_inst(const CUtensorMap &map, const RowParams &p, const RowPlan &pl, bool overlap, cudaStream_t stream) {
   static bool configured[64] = {};  // per device: the attribute is set once on each
   int dev = 0;
@@ -613,7 +617,7 @@ int row_launch_inst(const CUtensorMap &map, const RowParams &p, const RowPlan &p
   if (dev < 0 || dev >= 64 || !configured[dev]) {
     DeviceInfo di;
     if (int rc = get_device_info(&di)) return rc;
-    CUTB_CUDA_TRY(cudaFuncSetAttribute(qgemv_row_kernel<FMT, AMODE, NR, FIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)di.smem_optin));
+    CUTB_CUDA_TRY(cudaFuncSetAttribute(qgemv_row_kernel<FMT, AMODE, NR, FIXED, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)di.smem_optin));
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
   cudaLaunchConfig_t cfg = {};
@@ -626,15 +630,17 @@ int row_launch_inst(const CUtensorMap &map, const RowParams &p, const RowPlan &p
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = overlap ? 1 : 0;
-  CUTB_CUDA_TRY(cudaLaunchKernelEx(&cfg, qgemv_row_kernel<FMT, AMODE, NR, FIXED>, map, p));
+  CUTB_CUDA_TRY(cudaLaunchKernelEx(&cfg, qgemv_row_kernel<FMT, AMODE, NR, FIXED, MINB>, map, p));
   return CUTB_OK;
 }
 
 template <int FMT, int AMODE>
 int row_launch_mode(const CUtensorMap &map, const RowParams &p, const RowPlan &pl, bool overlap, cudaStream_t stream) {
-  if constexpr (AMODE != GV_A_F32_TWO)
-    if (p.M == 2) return row_launch_inst<FMT, AMODE, 2, false>(map, p, pl, overlap, stream);
-  return pl.fixed ? row_launch_inst<FMT, AMODE, 1, true>(map, p, pl, overlap, stream) : row_launch_inst<FMT, AMODE, 1, false>(map, p, pl, overlap, stream);
+  if constexpr (AMODE != GV_A_F32_TWO) {
+    if (p.M == 2) return row_launch_inst<FMT, AMODE, 2, false, 1>(map, p, pl, overlap, stream);
+    if (pl.beside) return row_launch_inst<FMT, AMODE, 1, true, 2>(map, p, pl, overlap, stream);
+  }
+  return pl.fixed ? row_launch_inst<FMT, AMODE, 1, true, 1>(map, p, pl, overlap, stream) : row_launch_inst<FMT, AMODE, 1, false, 1>(map, p, pl, overlap, stream);
 }
 
 template <int FMT>
@@ -658,16 +664,24 @@ bool row_matvec_plan(const cutb_qmatmul_desc &d, int amode, const DeviceInfo &di
   const size_t stage = (size_t)rw_granules(d.format) * RW_ROWS * granule_bytes(d.format);
   const size_t fixed = (size_t)gran_per_split * (nv * 512 + nr * 64) + nv * 512 + (size_t)nr * (pl->groups * RW_ROWS * RW_SUMS + RW_WARPS) * 4 +
                        RW_MAX_DEPTH * (RW_WARPS / rw_granules(d.format) + 1) * 8;
-  // Under half an SM where each group of warps has a stage there: the next launch's block starts its copies beside this one.  A block
-  // above that half keeps it out (measured on a 32-layer decode step with a larger ring: 540 -> 451 tok/s).
-  const size_t half = di.smem_per_sm > 2048 ? di.smem_per_sm / 2 - 1024 : di.smem_optin / 2;
   const uint32_t need = RW_WARPS / rw_granules(d.format);  // a slot for each group of warps at least
-  const size_t room = fixed + need * stage <= half ? half : di.smem_optin;
+  const uint32_t used = per_block * ((gran_per_split + rw_granules(d.format) - 1) / rw_granules(d.format));  // stages of a block
+  const uint32_t most = used > need ? used : need;
+  pl->fixed = gran_per_split == RW_WARPS && d.K / 256 % RW_WARPS == 0;
+  // The ring takes what the SM has, up to eight stages.  Four or five under half an SM, so that the next launch's block can start its copies
+  // beside this one, were the slower plan almost everywhere, by 14 % on average of 346 one-row shapes.  us a launch, half an SM (56 registers) /
+  // all of it: Q4_0 28672 x 8192 29.1 / 24.2, Q4_K 4096 x 14336 11.3 / 9.6, its fp32 rows at 32 bits 12000 x 14336 46.8 / 22.8, Q8_0 8000 x
+  // 8192 16.0 / 13.7; a token of eight layers of a Q8_0 decoder (hidden 4096) 548 / 487, Q4_K 412 / 378, Q4_0 388 / 363, hidden 2048 270 / 233.
+  // Only where a launch that starts early has all of a block's stages under half an SM at K = 4096 do neighbours gain: chains of Q4_0 4096 x
+  // 4096 3.46 / 3.83, Q8_0 2368 x 4096 3.1 / 3.6.  (The same for any K gained 0.1 us in chains and lost 12 % of the hidden 2048 decoder.)
+  const size_t half = di.smem_per_sm > 2048 ? di.smem_per_sm / 2 - 1024 : di.smem_optin / 2;
+  pl->beside = pl->fixed && nv == 1 && !(d.flags & CUTB_FLAG_NO_OVERLAP) && fixed + most * stage <= half;
+  const size_t room = di.smem_optin;
   if (fixed + need * stage > room) return false;
   const size_t fit = (room - fixed) / stage;
   pl->depth = fit > RW_MAX_DEPTH ? RW_MAX_DEPTH : (uint32_t)fit;
+  if (pl->depth > most) pl->depth = most;
   pl->smem = fixed + pl->depth * stage;
-  pl->fixed = gran_per_split == RW_WARPS && d.K / 256 % RW_WARPS == 0;
   return true;
 }
 
@@ -676,8 +690,9 @@ int row_matvec_launch(const GvParams &g, int format, int amode, const RowPlan &p
   static_cast<GvParams &>(p) = g;
   p.depth = pl.depth;
   p.groups = pl.groups;
+  p.box = p.gran_per_split < rw_granules(format) ? p.gran_per_split : rw_granules(format);
   CUtensorMap map;
-  if (int rc = make_tmap_granules(&map, p.W, format, p.N, p.K, p.row_bytes, RW_ROWS, rw_granules(format))) return rc;
+  if (int rc = make_tmap_granules(&map, p.W, format, p.N, p.K, p.row_bytes, RW_ROWS, p.box)) return rc;
   switch (format) {
     case CUTB_Q8_0: return row_launch_fmt<CUTB_Q8_0>(map, p, amode, pl, overlap, stream);
     case CUTB_Q4_0: return row_launch_fmt<CUTB_Q4_0>(map, p, amode, pl, overlap, stream);
