@@ -323,8 +323,15 @@ __device__ __forceinline__ void stage_activations(const GvParams &p, uint8_t *ac
     probe += __shfl_xor_sync(0xffffffffu, probe, 1);
     probe += __shfl_xor_sync(0xffffffffu, probe, 2);
     const bool finite = (amax < __int_as_float(0x7f800000)) && (probe == probe);
-    const float e = finite ? fmaxf(amax * (1.0f / GV_QMAX), 1.0f / GV_MOST) : __int_as_float(0x7fc00000);
-    const float inv = finite ? fminf(1.0f / e, GV_MOST) : 0.f;  // (of e itself: both roundings in one, see GV_STEPS2)
+    float e = amax * (1.0f / GV_QMAX), inv;
+    if constexpr (TWO) {
+      e = fmaxf(e, 1.0f / GV_MOST);
+      inv = finite ? 1.0f / e : 0.f;  // (of e itself: both roundings in one, see GV_STEPS2)
+    } else {
+      if constexpr (AF32) e = fmaxf(e, 1.0f / GV_MOST);
+      inv = finite ? fminf(GV_QMAX / amax, GV_MOST) : 0.f;
+    }
+    if (!finite) e = __int_as_float(0x7fc00000);
     int v[8], isum = 0;
     uint32_t whi[2], wlo[2];
 #pragma unroll
