@@ -1,5 +1,5 @@
-// Decode mat-vec of 2 to 16 activation rows over native GGUF blocks (qgemv_row.cu: one row, two at 16 bits), and the plan and
-// launch of both.
+// Decode mat-vec of 2 to 16 activation rows over native GGUF blocks, and the plan and launch of all that are (qgemv_row.cu: one row, most
+// launches of two at 16 bits; qgemv_few.cu: most of three to eight fp16 rows).
 //
 // C[m, n] = sum_k A[m, k] * dequant(W)[n, k], W = N rows of Q8_0 / Q4_0 / Q4_K
 // blocks.  Replaces the reference's M = 1 variants MatMulQ4GemvKPar8 /
@@ -763,7 +763,7 @@ int gv_amode(const cutb_qmatmul_desc &d) {
 struct GvPlan {
   uint32_t nt, nvr, ncp, grid_x, ksplit, gran_per_split, stages;
   bool overlap;
-  bool row;      // one or two virtual rows: qgemv_row.cu
+  bool row;      // one or two virtual rows, but for the smallest launches of two: qgemv_row.cu
   bool few;      // three to eight fp16 rows, where fp16 MMAs are the faster: qgemv_few.cu
   RowPlan rp;
   size_t smem;
@@ -803,6 +803,10 @@ bool gv_plan(const cutb_qmatmul_desc &d, const DeviceInfo &di, GvPlan *pl) {
   uint32_t want = 1;
   if (pl->grid_x * 2 <= (uint32_t)di.sm_count) want = (uint32_t)di.sm_count / pl->grid_x;
   if (want > G) want = G;
+  // Two rows with one tile of up to eight granules for a block: the staging of a whole block by all of its threads is what counts, and this
+  // kernel's is the shorter one.  us a launch, qgemv_row.cu / here: Q4_K 2368 x 512 3.7 / 3.1, 2368 x 1024 3.7 / 3.2, Q4_0 2368 x 2048 3.97 / 3.6,
+  // Q8_0 1000 x 1024 5.6 / 5.4; from there on that one is faster (Q4_0 1500 x 3072 3.7 / 4.9, Q8_0 8000 x 512 5.0 / 5.8, Q4_K 2368 x 3072 4.0 / 4.5).
+  if (d.M == 2 && pl->row && tiles <= pl->grid_x && (G + want - 1) / want <= 8) pl->row = false;
   const size_t limit = di.smem_optin;
   // Two CTAs per SM (this launch's and the next one's, which prefetches while
   // this one computes) need <= half of the SM's shared memory each; when that
@@ -843,7 +847,7 @@ bool gv_plan(const cutb_qmatmul_desc &d, const DeviceInfo &di, GvPlan *pl) {
         const uint32_t nv = pl->nt * 4;
         // From three virtual rows up the staging, repeated by every CTA, outweighs the mat-vec (measured:
         // 11008 x 4096 Q4_0, batch 8: 17.6 us, of which about 10 us staging): stage once, in a launch of its own.
-        pl->prestage = !(d.flags & CUTB_FLAG_STAGE_PER_CTA);
+        pl->prestage = pl->nvr >= 3 && !(d.flags & CUTB_FLAG_STAGE_PER_CTA);
         if (const char *e = getenv("CUTB_GV_PRESTAGE")) pl->prestage = pl->prestage && atoi(e) != 0;  // tuning override
         pl->staged_bytes = gps * 8 * (pl->ncp * 32 + nv * 4 * (d.format != CUTB_Q8_0 ? 2 : 1));
         pl->partial_bytes = gv_partial_bytes(d, pl->ksplit);

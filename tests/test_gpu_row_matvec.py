@@ -62,10 +62,11 @@ def test_tiles_stages_and_groups(fmt, M, dtype, flags, K, N):
 
 @pytest.mark.parametrize("fmt", FMTS)
 @pytest.mark.parametrize("M,dtype,flags", [(1, np.float16, 0), (2, np.float16, 0), (1, np.float32, 0), (1, np.float32, L.FLAG_NO_OVERLAP)])
-@pytest.mark.parametrize("K,N", [(3072, 4900), (3584, 2400), (768, 700), (4096, 2300), (4096, 4800), (13312, 1300)])
+@pytest.mark.parametrize("K,N", [(3072, 4900), (3584, 2400), (768, 700), (4096, 2300), (4096, 4800), (13312, 1300), (2048, 2368), (2304, 2368)])
 def test_rings_and_granules(fmt, M, dtype, flags, K, N):
     """Tiles of whole stages whose last granules are missing (a warp reads what it staged itself), of an odd number of stages (it does not),
-    splits of fewer granules than a stage has, rings that hold all of a block's stages and a part of them, a launch that starts early and not."""
+    splits of fewer granules than a stage has, rings that hold all of a block's stages and a part of them, a launch that starts early and not;
+    two rows on both sides of the line between the kernels (eight granules to a block)."""
     A, W, dense = _case(fmt, M, K, N, dtype, K + N + fmt)
     assert _err(_run(fmt, A, W, N, flags=flags), A.astype(np.float64) @ dense.T) <= TOL[32 if dtype == np.float32 else 16]
 
