@@ -88,7 +88,7 @@ static_assert(GV_STEPS2 * (0.5f + 32512.f * (0x1p-23f + 0x1p-24f)) < 32639.f, "t
 struct RowPlan {
   uint32_t grid_x, depth, groups;
   bool fixed;
-  bool beside;  // (qgemv_row.cu) the next launch's block is to fit beside this one's
+  bool beside;  // the next launch's block is to fit beside this one's
   size_t smem;
 };
 // false: no shared-memory plan for this K split

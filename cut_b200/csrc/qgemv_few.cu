@@ -63,34 +63,65 @@ __device__ __forceinline__ uint4 load_halves(const __half *at) {
   asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(at) : "memory");
   return v;
 }
-__device__ __noinline__ uint4 load_halves_one_by_one(const __half *at) {
-  uint32_t w[8];
+// A granule (256 halves) of up to four rows that do not all start on sixteen bytes, into shared memory: [row][512 bytes], word by word as they
+// lie.  Rows that start on a word are copied asynchronously (complete behind cp.async.wait_all); of one that starts between two words the
+// last word is made of its last and first half.
+__device__ __noinline__ void copy_rows(uint8_t *to, const __half *A, uint32_t lda, uint32_t rows, uint32_t lane) {
+  uint32_t w[4][4];  // (all loads are in flight)
+  auto between = [&](uint32_t m) { return (reinterpret_cast<uintptr_t>(A + (size_t)m * lda) & 2) != 0; };
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    uint16_t a;
-    asm volatile("ld.global.u16 %0, [%1];" : "=h"(a) : "l"(at + i) : "memory");
-    w[i] = a;
+  for (uint32_t m = 0; m < 4; ++m) {
+    if (m >= rows) continue;
+    const __half *row = A + (size_t)m * lda;
+    if (!between(m)) {
+      const uint32_t dst = smem_u32(to) + m * 512 + lane * 4;
+#pragma unroll
+      for (uint32_t i = 0; i < 4; ++i)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 128 * i), "l"(row + 2 * lane + 64 * i) : "memory");
+      continue;
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < 4; ++i) {
+      const uint32_t at = 1 + 2 * lane + 64 * i;
+      if (at < 255) {
+        asm volatile("ld.global.u32 %0, [%1];" : "=r"(w[m][i]) : "l"(row + at) : "memory");
+      } else {
+        uint16_t last, first;
+        asm volatile("ld.global.u16 %0, [%1];" : "=h"(last) : "l"(row + 255) : "memory");
+        asm volatile("ld.global.u16 %0, [%1];" : "=h"(first) : "l"(row) : "memory");
+        w[m][i] = last | (uint32_t)first << 16;
+      }
+    }
   }
-  return make_uint4(w[0] | w[1] << 16, w[2] | w[3] << 16, w[4] | w[5] << 16, w[6] | w[7] << 16);
+#pragma unroll
+  for (uint32_t m = 0; m < 4; ++m) {
+    if (m >= rows || !between(m)) continue;
+    uint16_t *row = reinterpret_cast<uint16_t *>(to + m * 512);
+#pragma unroll
+    for (uint32_t i = 0; i < 4; ++i) {
+      const uint32_t at = 1 + 2 * lane + 64 * i;
+      row[at] = (uint16_t)w[m][i];
+      row[(at + 1) & 255] = (uint16_t)(w[m][i] >> 16);
+    }
+  }
 }
 
 // Fragments: sixteen bytes per block, column (activation row, padded to CP) and lane t of a quad, the operands of the block's two MMAs
 // (Q4_0: the low nibbles' and the high nibbles'; Q4_K: the lane's first and last four bytes).
-template <int FMT, int CP>
-__device__ __forceinline__ void stage_granule(const FewParams &p, uint8_t *frag, float *off, uint32_t gs0, uint32_t gran, uint32_t lane, bool aligned) {
+template <int FMT, int CP, bool ALIGNED>
+__device__ __forceinline__ void stage_granule(const FewParams &p, uint8_t *frag, float *off, uint32_t gs0, uint32_t gran, uint32_t lane) {
   const uint32_t kb = lane >> 2, q = lane & 3;
   const __half *A = reinterpret_cast<const __half *>(p.A) + (size_t)(gs0 + gran) * 256 + lane * 8;
   uint4 x[CP];
-#pragma unroll
-  for (int m = 0; m < CP; ++m) x[m] = make_uint4(0, 0, 0, 0);
-  if (aligned) {
+  if constexpr (ALIGNED) {
 #pragma unroll
     for (int m = 0; m < CP; ++m)
-      if ((uint32_t)m < p.M) x[m] = load_halves(A + (size_t)m * p.lda);
+      x[m] = (uint32_t)m < p.M ? load_halves(A + (size_t)m * p.lda) : make_uint4(0, 0, 0, 0);
   } else {
 #pragma unroll
     for (int m = 0; m < CP; ++m)
-      if ((uint32_t)m < p.M) x[m] = load_halves_one_by_one(A + (size_t)m * p.lda);
+      x[m] = (uint32_t)m < p.M ? *reinterpret_cast<const uint4 *>(frag + (size_t)gran * CP * 512 + m * 512 + lane * 16) : make_uint4(0, 0, 0, 0);
+    __syncwarp();
   }
   uint8_t *to = frag + (size_t)(gran * 8 + kb) * CP * 64;
   const bool even = (kb & 1) == 0;
@@ -199,8 +230,9 @@ __device__ __forceinline__ void unit_few(uint32_t unit, uint32_t x, uint32_t o, 
   }
 }
 
-template <int FMT, int CP>
-__global__ void __launch_bounds__(FW_THREADS, 2) qgemv_few_kernel(const __grid_constant__ CUtensorMap weights, const FewParams p) {
+// ALIGNED: all rows start on sixteen bytes.  MINB: blocks per SM that the registers are kept for.
+template <int FMT, int CP, bool ALIGNED, int MINB>
+__global__ void __launch_bounds__(FW_THREADS, MINB) qgemv_few_kernel(const __grid_constant__ CUtensorMap weights, const FewParams p) {
   constexpr uint32_t GB = granule_bytes(FMT), UNIT = FW_ROWS * GB, GPS = FW_GRANULES, STAGE = GPS * UNIT, GROUPS = FW_GROUPS;
   extern __shared__ __align__(128) uint8_t smem[];
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
@@ -268,8 +300,17 @@ __global__ void __launch_bounds__(FW_THREADS, 2) qgemv_few_kernel(const __grid_c
 
   // What came before read only the (constant) weights; activations, D and C may be the predecessor's.
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  const bool aligned = reinterpret_cast<uintptr_t>(p.A) % 16 == 0 && p.lda % 8 == 0;
-  for (uint32_t gran = warp; gran < ng; gran += FW_WARPS) stage_granule<FMT, CP>(p, frag, off, gs0, gran, lane, aligned);
+  // Rows that start anywhere go to where the fragments will be first: one after the other, element by element, they took 0.3 us each.  us a
+  // launch, rows K + 2 and (odd) K + 9 apart: Q4_0 4096 x 2048 with 8 rows 6.8 -> 5.6, Q4_K 14336 x 1792 with 5 rows 11.8 -> 10.1, Q4_0
+  // 2368 x 4096 with 8 odd rows 8.7 -> 7.7 (the digits of qgemv_blocks.cu, at 16 bits: 6.2).
+  if constexpr (!ALIGNED) {
+    for (uint32_t gran = warp; gran < ng; gran += FW_WARPS)
+      for (uint32_t h = 0; h < p.M; h += 4)
+        copy_rows(frag + (size_t)gran * CP * 512 + h * 512, reinterpret_cast<const __half *>(p.A) + (size_t)(gs0 + gran) * 256 + (size_t)h * p.lda, p.lda, p.M - h, lane);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+  }
+  for (uint32_t gran = warp; gran < ng; gran += FW_WARPS) stage_granule<FMT, CP, ALIGNED>(p, frag, off, gs0, gran, lane);
   asm volatile("bar.sync 1, %0;" ::"n"(FW_CONSUMERS) : "memory");
 
   const uint32_t group = warp / GPS, wg = warp % GPS, gtid = tid - group * GPS * 32;
@@ -332,7 +373,7 @@ __global__ void __launch_bounds__(FW_THREADS, 2) qgemv_few_kernel(const __grid_c
   }
 }
 
-template <int FMT, int CP>
+template <int FMT, int CP, bool ALIGNED, int MINB>
 int few_launch_inst(const CUtensorMap &map, const FewParams &p, const RowPlan &pl, bool overlap, cudaStream_t stream) {
   static bool configured[64] = {};  // per device: the attribute is set once on each
   int dev = 0;
@@ -340,7 +381,7 @@ int few_launch_inst(const CUtensorMap &map, const FewParams &p, const RowPlan &p
   if (dev < 0 || dev >= 64 || !configured[dev]) {
     DeviceInfo di;
     if (int rc = get_device_info(&di)) return rc;
-    CUTB_CUDA_TRY(cudaFuncSetAttribute(qgemv_few_kernel<FMT, CP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)di.smem_optin));
+    CUTB_CUDA_TRY(cudaFuncSetAttribute(qgemv_few_kernel<FMT, CP, ALIGNED, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)di.smem_optin));
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
   cudaLaunchConfig_t cfg = {};
@@ -353,12 +394,17 @@ int few_launch_inst(const CUtensorMap &map, const FewParams &p, const RowPlan &p
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = overlap ? 1 : 0;
-  CUTB_CUDA_TRY(cudaLaunchKernelEx(&cfg, qgemv_few_kernel<FMT, CP>, map, p));
+  CUTB_CUDA_TRY(cudaLaunchKernelEx(&cfg, qgemv_few_kernel<FMT, CP, ALIGNED, MINB>, map, p));
   return CUTB_OK;
 }
 
+template <int FMT, bool ALIGNED> int few_launch_rows(const CUtensorMap &map, const FewParams &p, const RowPlan &pl, bool overlap, cudaStream_t stream) {
+  if (pl.beside) return p.M <= 4 ? few_launch_inst<FMT, 4, ALIGNED, 2>(map, p, pl, overlap, stream) : few_launch_inst<FMT, 8, ALIGNED, 2>(map, p, pl, overlap, stream);
+  return p.M <= 4 ? few_launch_inst<FMT, 4, ALIGNED, 1>(map, p, pl, overlap, stream) : few_launch_inst<FMT, 8, ALIGNED, 1>(map, p, pl, overlap, stream);
+}
 template <int FMT> int few_launch_fmt(const CUtensorMap &map, const FewParams &p, const RowPlan &pl, bool overlap, cudaStream_t stream) {
-  return p.M <= 4 ? few_launch_inst<FMT, 4>(map, p, pl, overlap, stream) : few_launch_inst<FMT, 8>(map, p, pl, overlap, stream);
+  const bool aligned = reinterpret_cast<uintptr_t>(p.A) % 16 == 0 && p.lda % 8 == 0;
+  return aligned ? few_launch_rows<FMT, true>(map, p, pl, overlap, stream) : few_launch_rows<FMT, false>(map, p, pl, overlap, stream);
 }
 
 }  // namespace
@@ -378,14 +424,19 @@ bool few_matvec_plan(const cutb_qmatmul_desc &d, const DeviceInfo &di, uint32_t 
   const uint32_t tiles = (d.N + FW_ROWS - 1) / FW_ROWS;
   pl->grid_x = tiles < sms ? tiles : sms;
   pl->groups = 1;
-  pl->fixed = pl->beside = false;
+  pl->fixed = false;
   const size_t stage = (size_t)FW_GRANULES * FW_ROWS * granule_bytes(d.format);
   const size_t fixed = (size_t)gran_per_split * cp * (512 + 32) + (size_t)FW_WARPS * cp * FW_ROWS * 4 + FW_MAX_DEPTH * (FW_GROUPS + 1) * 8;
   const size_t half = di.smem_per_sm > 2048 ? di.smem_per_sm / 2 - 1024 : di.smem_optin / 2;
-  const size_t room = fixed + 4 * stage <= half ? half : di.smem_optin;
+  // Beside the next launch's block (56 registers, some spilled) where that leaves four stages, but for Q4_K's wide columns: us a launch, beside /
+  // alone, Q4_K 8000 x 1024 with 8 rows 5.6 / 5.3, Q4_0 8000 x 1024 with 8 rows 4.9 / 5.1, 4096 x 2048 with 3 rows 3.8 / 4.1.
+  pl->beside = (cp == 4 || d.format == CUTB_Q4_0) && fixed + 4 * stage <= half;
+  const size_t room = pl->beside ? half : di.smem_optin;
   if (fixed + 2 * stage > room) return false;
   const size_t fit = (room - fixed) / stage;
   pl->depth = fit > FW_MAX_DEPTH ? FW_MAX_DEPTH : (uint32_t)fit;
+  const uint32_t used = (tiles + pl->grid_x - 1) / pl->grid_x * ((gran_per_split + FW_GRANULES - 1) / FW_GRANULES);  // stages of a block
+  if (!pl->beside && pl->depth > used) pl->depth = used > 2 ? used : 2;
   pl->smem = fixed + pl->depth * stage;
   return true;
 }
