@@ -352,7 +352,8 @@ __global__ void __launch_bounds__(FW_THREADS, MINB) qgemv_few_kernel(const __gri
       for (uint32_t w = 0; w < GPS; ++w) sum += at[w * CP * FW_ROWS];
       sum *= FW_UNIT;
       if (p.glu) {  // (gate, up) row pairs are neighbouring lanes: one output per pair
-        const float up = __shfl_down_sync(__activemask(), sum, 1);
+        // (an odd number of rows leaves half of the last warp)
+        const float up = __shfl_down_sync((o & ~31u) + 32 <= FW_ROWS * p.M ? 0xffffffffu : 0x0000ffffu, sum, 1);
         if (!(row & 1) && n < r1) p.C[(size_t)m * p.ldc + (n >> 1)] = apply_epilogue(sum, CUTB_FUSION_UNARY, p.fusion_op, 0.f) * up;
         continue;
       }

@@ -115,3 +115,10 @@ def test_the_reading_finds_what_it_is_for():
     assert not split_warps("if (!dead && !warp_wait(b, p)) { dead = true; break; }")
     assert not split_warps("if (lane == 0) { if (!mbar_spin_bounded(b, p)) break; }")
     assert not split_warps("if (!dead && !mbar_spin_bounded(b, p)) { give_up(); dead = true; }")
+
+
+def test_shuffles_name_their_lanes():
+    """The lanes of a shuffle or a vote are stated: which of them happen to be together is the compiler's choice."""
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu*"))):
+        with open(path) as f:
+            assert "__activemask" not in _without_comments(f.read()), path
