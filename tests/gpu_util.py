@@ -36,3 +36,13 @@ def run_blocks(fmt, A_np, W_np, N, *, variant=L.VARIANT_AUTO, D_np=None, fusion_
     torch.cuda.synchronize()
     st = int(status.item()) if with_status else 0
     return C_out.cpu().numpy(), used, st
+
+
+def kernels_of(run) -> list[str]:
+    """Names of the kernels that `run` launches."""
+    from torch.profiler import ProfilerActivity, profile
+
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        run()
+        torch.cuda.synchronize()
+    return [e.name for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA]

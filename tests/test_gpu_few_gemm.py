@@ -13,7 +13,8 @@ from oracle import oracle as O
 pytestmark = pytest.mark.gpu
 
 
-def _run(fmt, A, W, N, *, variant=L.VARIANT_GEMM_TC, scratch=None, stride=0, glu=False):
+def _run(fmt, A, W, N, *, variant=L.VARIANT_GEMM_TC, scratch=None, stride=0, glu=False, kernel="qgemm_few_kernel"):
+    """scratch: its bytes (None: what the query asks for); kernel: the one that has to run."""
     import torch
 
     from cut_b200 import ops
@@ -28,15 +29,31 @@ def _run(fmt, A, W, N, *, variant=L.VARIANT_GEMM_TC, scratch=None, stride=0, glu
     if glu:
         out = torch.full((M, N // 2), float("nan"), device="cuda")
         d.C, d.ldc = out.data_ptr(), N // 2
-    need = ops.workspace_bytes(d)
-    ws = torch.full((max(need, 16),), 0xFF, dtype=torch.uint8, device="cuda")  # (NaNs: nothing may be read before it is written)
-    d.workspace, d.workspace_bytes = ws.data_ptr(), need if scratch is None else scratch
-    ops.launch(d)
+    need = ops.workspace_bytes(d) if scratch is None else scratch
+    ws = torch.full((need + 4096,), 0xFF, dtype=torch.uint8, device="cuda")  # (NaNs: nothing may be read before it is written)
+    ws[need:] = 0xA5
+    d.workspace, d.workspace_bytes = ws.data_ptr(), need
+    from gpu_util import kernels_of
+
+    names = kernels_of(lambda: ops.launch(d))
+    assert any(kernel in n for n in names), names
     first = out.cpu().numpy().copy()
     ops.launch(d)
     torch.cuda.synchronize()
-    assert int(status.item()) == 0 and np.array_equal(first, out.cpu().numpy())
+    assert int(status.item()) == 0 and np.array_equal(first, out.cpu().numpy(), equal_nan=True)
+    assert bool((ws[need:] == 0xA5).all())  # nothing behind the scratch was written
     return first.astype(np.float64)
+
+
+def _shares(M, K, N):
+    """Rows that are read in place ask for scratch where several blocks share a tile."""
+    import torch
+
+    tiles, nk = -(-N // 128), K // 256
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    per = -(-tiles * nk // min(tiles * nk, sms))
+    whole = -(-per // nk) * nk
+    return (whole if whole <= per + 6 else per) % nk != 0
 
 
 @pytest.mark.parametrize("fmt", [synth.Q8_0, synth.Q4_0, synth.Q4_K])
@@ -52,11 +69,12 @@ def test_tiles_units_and_shares(fmt, M, K, N, act):
     err = lambda got: float(np.linalg.norm(got - want) / np.linalg.norm(want))
     assert err(_run(fmt, A, W, N)) <= tol
     if act == np.float16:
-        assert err(_run(fmt, A, W, N, scratch=0)) <= tol
+        shared = K > 256 and _shares(M, K, N)
+        assert err(_run(fmt, A, W, N, scratch=0, kernel="qgemm_skinny_kernel" if shared else "qgemm_few_kernel")) <= tol
         if 17 <= M <= 32:  # rows that do not start on 16 bytes
             assert err(_run(fmt, A, W, N, variant=L.VARIANT_ROWS_MMA, stride=1)) <= tol
-    else:
-        assert err(_run(fmt, A, W, N, scratch=(M * K * 2 + 15) // 16 * 16 + (1 << 25))) <= tol
+    else:  # room for the rows as fp16 and for nothing else
+        assert err(_run(fmt, A, W, N, scratch=(M * K * 2 + 15) // 16 * 16, kernel="qgemm_skinny_kernel")) <= tol
 
 
 @pytest.mark.parametrize("M,K,N", [(20, 4096, 2816), (64, 256, 38000), (48, 1024, 258)])
@@ -68,3 +86,19 @@ def test_paired_rows(M, K, N):
     got = _run(synth.Q4_0, A, W, N, glu=True)
     # (both factors carry the weights' rounding, silu's slope is at most 1.1)
     assert np.linalg.norm(got - want) <= 2.1 * 5e-4 * np.linalg.norm(np.abs(gate * up)) + 1e-6
+
+
+@pytest.mark.parametrize("fmt", [synth.Q8_0, synth.Q4_0, synth.Q4_K])
+@pytest.mark.parametrize("M,K,N", [(18, 512, 700), (61, 2048, 2178)])
+def test_what_is_not_finite_stays_in_its_row(fmt, M, K, N):
+    """An infinity, a NaN, fp16 subnormals and zeros beside ordinary rows."""
+    W, A = synth.make_weights(fmt, N, K, M), synth.make_activations(M, K, 7, np.float16)
+    A[3, 100], A[M - 1, K - 1], A[5] = np.inf, np.nan, 0
+    A[6] = (np.arange(K) % 64 - 31).astype(np.float16) * np.float16(6e-8)
+    with np.errstate(invalid="ignore"):
+        prod = A.astype(np.float64) @ O.dequant_rows(fmt, W, N, K).astype(np.float64).T
+    got = _run(fmt, A, W, N)
+    assert not np.isfinite(got[3]).any() and np.isnan(got[M - 1]).all() and (got[5] == 0).all()
+    tol = 2e-3 if fmt == synth.Q4_K else 5e-4
+    for rows in ([6], [m for m in range(M - 1) if m not in (3, 5, 6)]):
+        assert np.linalg.norm(got[rows] - prod[rows]) <= tol * np.linalg.norm(prod[rows])

@@ -1,5 +1,5 @@
-"""The mat-vecs of one row and of two fp16 rows (qgemv_row.cu), and of three to eight fp16 rows (qgemv_few.cu), at the edges of its tiles, stages, groups and loads, against the checker's
-dequantised weights in 64 bits.
+"""The mat-vecs of one row and of two fp16 rows (qgemv_row.cu), and of three to eight fp16 rows (qgemv_few.cu), at the edges of their tiles,
+stages, groups and loads, against the checker's dequantised weights in 64 bits.
 
 Tolerances: a 16-bit level leaves an error of at most max|x of a block| / 65024 per element, uniform, so relative to a block of normal
 values (maximum about 2.5 sigma) 2.5 / 65024 / sqrt(3) = 2.2e-5 of the norm: four times that.  Two levels leave the fp32 sums: 2^-24 times
@@ -182,3 +182,78 @@ def test_a_few_rows_in_pairs(fmt, M):
     want, got = np.maximum(y[:, 0::2], 0.0) * y[:, 1::2], out.cpu().numpy().astype(np.float64)
     for m in range(M):
         assert _err(got[m], want[m]) <= 4e-5, m
+
+
+@pytest.mark.parametrize("fmt", [synth.Q4_0, synth.Q4_K])
+@pytest.mark.parametrize("M,shift", [(3, 0), (5, 0), (7, 0), (8, 0), (3, 1), (8, 2)])
+def test_what_is_not_finite_stays_in_its_row(fmt, M, shift):
+    """An infinity, a NaN and fp16 subnormals (6e-8 to 2e-6) beside an ordinary row and the idle columns of an odd number of rows."""
+    K, N = 1280, 2401
+    A, W, dense = _case(fmt, M, K, N, np.float16, M + fmt)
+    A[0, 700], A[M - 1, K - 1] = np.inf, np.nan
+    small = (np.arange(K) % 64 - 31).astype(np.float16) * np.float16(6e-8)
+    if M > 3:
+        A[2] = small
+    with np.errstate(invalid="ignore"):
+        want = A.astype(np.float64) @ dense.T
+    got = _run(fmt, A, W, N, shift=shift)
+    assert not np.isfinite(got[0]).any() and np.isnan(got[M - 1]).all()
+    for m in range(1, M - 1):
+        assert _err(got[m], want[m]) <= 2e-5, m
+    A[0] = 0
+    assert (_run(fmt, A, W, N, shift=shift)[0] == 0).all()
+
+
+@pytest.mark.parametrize("fmt,M,dtype,flags,K,N,kernel", [
+    (synth.Q8_0, 1, np.float16, 0, 4096, 4096, "qgemv_row_kernel"), (synth.Q4_K, 1, np.float32, 0, 14336, 4096, "qgemv_row_kernel"),
+    (synth.Q4_0, 1, np.float32, L.FLAG_ACT_16BIT, 512, 500, "qgemv_row_kernel"), (synth.Q4_0, 2, np.float16, 0, 2304, 2368, "qgemv_row_kernel"),
+    (synth.Q4_0, 2, np.float16, 0, 2048, 2368, "qgemv_blocks_kernel"), (synth.Q8_0, 2, np.float32, L.FLAG_ACT_16BIT, 4096, 500, "qgemv_blocks_kernel"),
+    (synth.Q8_0, 2, np.float32, L.FLAG_ACT_16BIT, 512, 4096, "qgemv_row_kernel"), (synth.Q4_K, 2, np.float32, 0, 4096, 4096, "qgemv_blocks_kernel"),
+    (synth.Q4_0, 3, np.float16, 0, 4096, 11008, "qgemv_few_kernel"), (synth.Q8_0, 3, np.float16, 0, 4096, 11008, "qgemv_blocks_kernel"),
+    (synth.Q4_K, 4, np.float16, 0, 3072, 11008, "qgemv_few_kernel"), (synth.Q4_0, 4, np.float16, 0, 4096, 5000, "qgemv_few_kernel"),
+    (synth.Q4_0, 4, np.float16, 0, 4096, 2368, "qgemv_blocks_kernel"), (synth.Q4_0, 4, np.float16, 0, 4096, 14336, "qgemv_blocks_kernel"),
+    (synth.Q4_K, 5, np.float16, 0, 5120, 9600, "qgemv_few_kernel"), (synth.Q4_K, 6, np.float16, 0, 5120, 5000, "qgemv_blocks_kernel"),
+    (synth.Q4_0, 8, np.float16, 0, 4096, 200, "qgemv_few_kernel"), (synth.Q4_0, 4, np.float16, 0, 8192, 5000, "qgemv_blocks_kernel")])
+def test_the_kernel_that_runs(fmt, M, dtype, flags, K, N, kernel):
+    """Both sides of the lines between the mat-vecs: the launched kernel, by its name."""
+    import torch
+
+    from cut_b200 import ops
+    from gpu_util import kernels_of
+
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the lines are drawn for 148 multiprocessors")
+    A = torch.zeros((M, K), dtype=torch.float16 if dtype == np.float16 else torch.float32, device="cuda")
+    d, out, keep = ops.make_desc(A, torch.zeros(N * synth.row_bytes(fmt, K), dtype=torch.uint8, device="cuda"), fmt, N, flags=flags)
+    ws = torch.empty(max(ops.workspace_bytes(d), 16), dtype=torch.uint8, device="cuda")
+    d.workspace, d.workspace_bytes = ws.data_ptr(), ws.numel()
+    names = [n for n in kernels_of(lambda: ops.launch(d)) if "qgemv" in n]
+    assert len(names) == 1 and kernel in names[0], names
+
+
+@pytest.mark.parametrize("fmt,M,dtype,K,N", [(synth.Q4_0, 1, np.float16, 4096, 2401), (synth.Q8_0, 1, np.float32, 2304, 1200), (synth.Q4_K, 2, np.float16, 4096, 2500),
+                                             (synth.Q4_0, 3, np.float16, 4096, 1300), (synth.Q4_K, 8, np.float16, 1024, 2401), (synth.Q4_0, 5, np.float16, 4096, 300)])
+def test_scatter_into_two_outputs(fmt, M, dtype, K, N):
+    """The epilogue that stores its slice into every rank's output, with two buffers of this GPU as the ranks' (the exchange between ranks is not
+    launched): the plain launch's bits, and nothing beside the slice."""
+    import ctypes as C
+
+    import torch
+
+    from cut_b200 import ops
+
+    A, W, _ = _case(fmt, M, K, N, dtype, M + K)
+    a, w, at, total = torch.from_numpy(A).cuda(), torch.from_numpy(W).cuda(), 37, N + 100
+    d, plain, keep = ops.make_desc(a, w, fmt, N, variant=L.VARIANT_GEMV_MMA)
+    ws = torch.empty(max(ops.workspace_bytes(d), 16), dtype=torch.uint8, device="cuda")
+    d.workspace, d.workspace_bytes = ws.data_ptr(), ws.numel()
+    ops.launch(d)
+    outs, flags = torch.full((2, M, total), 5.0, device="cuda"), torch.zeros(64, dtype=torch.int64, device="cuda")
+    ps = L.PeerScatter()
+    ps.world, ps.rank, ps.ldc_total, ps.n_offset = 2, 0, total, at
+    for r in range(2):
+        ps.C_peers[r], ps.flag_peers[r] = outs[r].data_ptr(), flags.data_ptr() + 256 * r
+    L.check(L.lib().cutb_qmatmul_scatter(C.byref(d), C.byref(ps), None))
+    torch.cuda.synchronize()
+    for o in outs:
+        assert torch.equal(o[:, at: at + N], plain) and bool((o[:, :at] == 5.0).all()) and bool((o[:, at + N:] == 5.0).all())

@@ -32,11 +32,14 @@ def _run(fmt, A, W, N, *, D=None, glu=False):
         d.C, d.ldc = out.data_ptr(), N // 2
     ws = torch.full((max(ops.workspace_bytes(d), 16),), 0xFF, dtype=torch.uint8, device="cuda")
     d.workspace, d.workspace_bytes = ws.data_ptr(), ws.numel()
-    ops.launch(d)
+    from gpu_util import kernels_of
+
+    names = kernels_of(lambda: ops.launch(d))
+    assert any("qgemm_wide_kernel" in n for n in names), names
     first = out.cpu().numpy().copy()
     ops.launch(d)
     torch.cuda.synchronize()
-    assert int(status.item()) == 0 and np.array_equal(first, out.cpu().numpy())
+    assert int(status.item()) == 0 and np.array_equal(first, out.cpu().numpy(), equal_nan=True)
     return first.astype(np.float64)
 
 
@@ -63,3 +66,19 @@ def test_paired_rows(M, K, N):
     got = _run(synth.Q4_0, A, W, N, glu=True)
     # (both factors carry the weights' rounding, silu's slope is at most 1.1)
     assert np.linalg.norm(got - want) <= 2.1 * 5e-4 * np.linalg.norm(np.abs(gate * up)) + 1e-6
+
+
+@pytest.mark.parametrize("fmt", [synth.Q8_0, synth.Q4_0, synth.Q4_K])
+@pytest.mark.parametrize("M,K,N", [(70, 512, 20000), (290, 1024, 6000)])
+def test_what_is_not_finite_stays_in_its_row(fmt, M, K, N):
+    """An infinity, a NaN, fp16 subnormals and zeros beside ordinary rows, in the last rows of a tile among them."""
+    W, A = synth.make_weights(fmt, N, K, M), synth.make_activations(M, K, 7, np.float16)
+    A[3, 100], A[M - 1, K - 1], A[5] = np.inf, np.nan, 0
+    A[6] = (np.arange(K) % 64 - 31).astype(np.float16) * np.float16(6e-8)
+    with np.errstate(invalid="ignore"):
+        prod = A.astype(np.float64) @ O.dequant_rows(fmt, W, N, K).astype(np.float64).T
+    got = _run(fmt, A, W, N)
+    assert not np.isfinite(got[3]).any() and np.isnan(got[M - 1]).all() and (got[5] == 0).all()
+    tol = 2e-3 if fmt == synth.Q4_K else 5e-4
+    for rows in ([6], [m for m in range(M - 1) if m not in (3, 5, 6)]):
+        assert np.linalg.norm(got[rows] - prod[rows]) <= tol * np.linalg.norm(prod[rows])
