@@ -20,8 +20,9 @@ int qgemv_blocks_launch(const cutb_qmatmul_desc &d, cudaStream_t stream, const c
 // Publishes this rank's peer stores of the step and waits (bounded) for every rank's.
 int peer_exchange_launch(const cutb_peer_scatter &peers, uint64_t *step_counter, int *status, cudaStream_t stream);
 
-// Matmul of 9 to 32 activation rows, as fp16 MMAs over GGUF blocks (qgemv_rows.cu).  qgemv_rows_faster: of the shapes that it takes,
-// those where it beats the other kernels.  It runs only where the caller's workspace holds what it needs (qgemv_rows_fits).
+// Matmul of 9 to 16 activation rows, as fp16 MMAs over GGUF blocks (qgemv_rows.cu), and under the same name of 17 to 32 rows, which take
+// qgemm_few.cu.  qgemv_rows_faster: of the shapes that it takes, those where it beats the other kernels (above 16 rows: where its name is
+// reported; the kernel is the same on either side).  It runs only where the caller's workspace holds what it needs (qgemv_rows_fits).
 bool qgemv_rows_supported(const cutb_qmatmul_desc &d);
 bool qgemv_rows_faster(const cutb_qmatmul_desc &d);
 uint64_t qgemv_rows_workspace(const cutb_qmatmul_desc &d);

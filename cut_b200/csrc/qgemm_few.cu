@@ -16,7 +16,7 @@
 //    out by a kernel before it, which then also clears a counter per tile: the last of a tile's CTAs adds the shares, and the kernel
 //    behind is not needed.
 //
-// Bound by issue slots of the conversion (about 1000 cycles a unit, whose bytes HBM needs 770 for), and by some 7 us of two dependent
+// Bound by the chain of the conversion (about 1000 cycles a unit, whose bytes HBM needs 770 for; issue slots are half busy), and by some 7 us of two dependent
 // launches and the chain copy -> widen -> MMA -> share -> sum.  us a call in a chain, what ran before (MMAs of registers up
 // to 32 rows, else qgemm_skinny.cu) -> here: Q4_0 4096 x 4096 32 rows 13.7 -> 8.5, 64 rows 17.7 -> 10.6; 8192 x 28672 32 rows 62.7 -> 48.7;
 // Q8_0 8192 x 11008 64 rows 58.4 -> 27.0; Q4_K 4096 x 28672 64 rows 48.4 -> 34.0; Q4_0 4096 x 4096 with 50 fp32 rows 21.3 -> 11.9.  Over

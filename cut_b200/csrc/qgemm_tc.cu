@@ -527,7 +527,7 @@ int qgemm_tc_launch(const cutb_qmatmul_desc &d, cudaStream_t stream) {
     return CUTB_ERR_UNSUPPORTED;
   }
   // Pairs of CTAs with the weights in tensor memory, unless this kernel's shares of K fill the SMs better.  The estimates of this one are
-  // up to 15 % low, hence the margin.  us, this kernel / that one, of 50 random shapes: Q8_0 333 x 11008 x 4096 55.9 / 60.8 and Q4_0 272 x
+  // up to 15 % low, hence the margin.  us with the weights in L2, this kernel / that one: Q8_0 333 x 11008 x 4096 55.9 / 60.8 and Q4_0 272 x
   // 12032 x 1248 27.0 / 44.2 stay; Q4_K 512 x 4096 x 14336 62.2 / 53.8, x 6144 45.3 / 28.3, 157 x 2560 x 23552 55.5 / 28.7, Q8_0 565 x 6912
   // x 28352 301 / 181, Q4_0 1763 x 4096 x 26880 364 / 294 go there.
   float wide_time = 0.f;

@@ -15,10 +15,10 @@
 //    commit, whose cost (some 600 cycles) bounded pieces of 64 k.  16 converter warps, four groups, the g-th 64 k of every unit each.
 //  * Up to 128 rows there are two accumulators.  A tile is finished by the converters once a unit of the next one is on its way.
 //
-// Bound by the tensor cores and, up to some 160 rows a tile, by the issue slots of the conversion (a unit of 256 k takes 0.9 us with 64 rows,
-// 1.4 us with 256, of which the MMAs need 1.1).  us, what ran before -> here: Q4_K 512 x 4096 x 14336 62 -> 54, x 28672 120 -> 103,
-// x 6144 45 -> 28, x 4096 34 -> 25; Q8_0 512 x 4096 x 11008 64 -> 46; Q4_0 130 x 4096 x 11008 40 -> 24; 50 random shapes of 65 to 2048 rows
-// 1.35 times as fast on average.  Two issuers, converters that take 128 k of every other unit, and an epilogue that holds the tile in registers
+// Bound by the tensor cores (69 % busy at 512 rows) and, up to some 160 rows a tile, by the chain of the conversion: load, widen, store, hand over
+// (a unit of 256 k takes 0.9 us with 64 rows, 1.4 us with 256, of which the MMAs need 1.1; issue slots are half busy).  us with the weights
+// in L2, what ran before -> here: Q4_K 512 x 4096 x 14336 62 -> 54 (cycled weights 70 -> 64), x 28672 120 -> 103, x 6144 45 -> 28, x 4096
+// 34 -> 25; Q8_0 512 x 4096 x 11008 64 -> 46; Q4_0 130 x 4096 x 11008 40 -> 24.  Two issuers, converters that take 128 k of every other unit, and an epilogue that holds the tile in registers
 // (it spilled) gained nothing.
 //
 // Every wait is bounded; on expiry CUTB_ERR_TIMEOUT is recorded.  Both CTAs stay until copies, MMAs and signals between them are through.

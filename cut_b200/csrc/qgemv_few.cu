@@ -3,8 +3,8 @@
 // C[m, n] = epilogue(sum_k A[m, k] * dequant(W)[n, k]), the reference's M = 1 variant (operators/impl/matmul/MatMulQ4GemvKPar8.cu:8-98)
 // for a few rows at a time.
 //
-// Bound by issue slots and shared memory (some 250 instructions and 90 cycles of shared memory for 16 rows of 256 weights, whose bytes
-// HBM needs 100 cycles for), and, where a launch is short, by the same chain of latencies as qgemv_row.cu.  What keeps both low:
+// Bound by latency (issue slots 37 % busy, shared memory 90 of the 100 cycles that HBM needs for 16 rows of 256 weights): the chain load ->
+// MMA -> scale at four warps per scheduler, and, where a launch is short, the same hand-over and staging as in qgemv_row.cu.  What keeps them low:
 //  * Quants enter m16n8k16 without a conversion: the bits of a nibble in the low mantissa bits of a half are the subnormal q * 2^-24,
 //    exact, and one logic operation makes two of them (high nibbles: 16 q, in MMAs of their own).  Q4_0's offset times a block's sum of
 //    activations is the accumulator's start, Q4_K's minima take the same sums; the sums are MMAs with a constant.  The activations
@@ -12,11 +12,11 @@
 //  * So there is nothing to quantise: a warp loads the granules (256 k) that fall to it, puts them into fragment order in shared memory,
 //    and no launch goes before this one (the int8 digits of qgemv_blocks.cu take a launch of their own from three rows up).
 //  * Weights come as in qgemv_row.cu: stages of 16 rows by eight granules by one tensor copy each.  The block keeps under half an SM where
-//    that leaves four stages (up to four rows of 4096), else it takes a deep ring (8 rows of 4096, Q4_0 11008 x 4096: 12.3 us a launch
-//    with eight stages alone on the SM, 15.1 with two beside the next launch's block).
+//    that leaves four stages (up to four rows of 4096), else it takes a deep ring and the registers it likes (8 rows of 4096, Q4_0
+//    11008 x 4096: 11.7 us a launch with eight stages alone on the SM, 12.1 with 56 registers, 15.1 with two stages beside the next block).
 //  * Two groups of eight warps take a tile each, a granule per warp and stage; stages of both tiles come in turn.  A group meets in
 //    barriers of its own, once to add up a tile and once before it writes the next tile's sums.
-// us a launch, int8 digits -> here (graphs of 2 to 32): Q4_0 11008 x 4096 3 rows 14.6 -> 10.0, 8 rows 12.9 -> 12.2; 4096 x 4096 3 rows 8.6 ->
+// us a launch, int8 digits -> here (graphs of 2 to 32): Q4_0 11008 x 4096 3 rows 14.6 -> 10.0, 8 rows 12.9 -> 11.7; 4096 x 4096 3 rows 8.6 ->
 // 5.7, 8 rows 8.2 -> 7.2; 14336 x 2048 13.8 -> 8.9 and 12.5 -> 9.7; Q4_K 28672 x 1024 19.5 -> 12.2 and 23.7 -> 12.5.  Relative error against
 // 64 bits 7e-7 (Q4_0) and 8e-6 (Q4_K) where the digits have 2.2e-5.  Q8_0 gained nothing (8 rows of 4096 x 4096 7.9 -> 9.4).
 //
