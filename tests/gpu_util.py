@@ -1,6 +1,8 @@
 """Shared helpers of the GPU parity tests (torch = device memory only)."""
 from __future__ import annotations
 
+import ctypes
+
 import numpy as np
 import torch
 
@@ -38,11 +40,32 @@ def run_blocks(fmt, A_np, W_np, N, *, variant=L.VARIANT_AUTO, D_np=None, fusion_
     return C_out.cpu().numpy(), used, st
 
 
-def kernels_of(run) -> list[str]:
-    """Names of the kernels that `run` launches."""
-    from torch.profiler import ProfilerActivity, profile
+class _KernelNode(ctypes.Structure):  # CUDA_KERNEL_NODE_PARAMS
+    _fields_ = [("func", ctypes.c_void_p), ("grid", ctypes.c_uint * 3), ("block", ctypes.c_uint * 3), ("shared", ctypes.c_uint),
+                ("params", ctypes.c_void_p), ("extra", ctypes.c_void_p), ("kern", ctypes.c_void_p), ("ctx", ctypes.c_void_p)]
 
-    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+
+def kernels_of(run) -> list[str]:
+    """(Mangled) names of the kernels that `run` launches, from a recording of it that is not executed."""
+    cu = ctypes.CDLL("libcuda.so.1")
+
+    def ok(rc):
+        assert rc == 0, rc
+
+    recording = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(recording):
         run()
-        torch.cuda.synchronize()
-    return [e.name for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+    graph, n = ctypes.c_void_p(recording.raw_cuda_graph()), ctypes.c_size_t(0)
+    ok(cu.cuGraphGetNodes(graph, None, ctypes.byref(n)))
+    nodes = (ctypes.c_void_p * n.value)()
+    ok(cu.cuGraphGetNodes(graph, nodes, ctypes.byref(n)))
+    names = []
+    for node in nodes:
+        kind, p, name = ctypes.c_int(-1), _KernelNode(), ctypes.c_char_p()
+        ok(cu.cuGraphNodeGetType(ctypes.c_void_p(node), ctypes.byref(kind)))
+        if kind.value != 0:  # not a kernel
+            continue
+        ok(cu.cuGraphKernelNodeGetParams_v2(ctypes.c_void_p(node), ctypes.byref(p)))
+        ok(cu.cuKernelGetName(ctypes.byref(name), ctypes.c_void_p(p.kern)) if p.kern else cu.cuFuncGetName(ctypes.byref(name), ctypes.c_void_p(p.func)))
+        names.append(name.value.decode())
+    return names

@@ -33,14 +33,15 @@ def _run(fmt, A, W, N, *, variant=L.VARIANT_GEMM_TC, scratch=None, stride=0, glu
     ws = torch.full((need + 4096,), 0xFF, dtype=torch.uint8, device="cuda")  # (NaNs: nothing may be read before it is written)
     ws[need:] = 0xA5
     d.workspace, d.workspace_bytes = ws.data_ptr(), need
-    from gpu_util import kernels_of
-
-    names = kernels_of(lambda: ops.launch(d))
-    assert any(kernel in n for n in names), names
+    ops.launch(d)
     first = out.cpu().numpy().copy()
     ops.launch(d)
     torch.cuda.synchronize()
     assert int(status.item()) == 0 and np.array_equal(first, out.cpu().numpy(), equal_nan=True)
+    from gpu_util import kernels_of
+
+    names = kernels_of(lambda: ops.launch(d))
+    assert any(kernel in n for n in names), names
     assert bool((ws[need:] == 0xA5).all())  # nothing behind the scratch was written
     return first.astype(np.float64)
 

@@ -32,14 +32,15 @@ def _run(fmt, A, W, N, *, D=None, glu=False):
         d.C, d.ldc = out.data_ptr(), N // 2
     ws = torch.full((max(ops.workspace_bytes(d), 16),), 0xFF, dtype=torch.uint8, device="cuda")
     d.workspace, d.workspace_bytes = ws.data_ptr(), ws.numel()
-    from gpu_util import kernels_of
-
-    names = kernels_of(lambda: ops.launch(d))
-    assert any("qgemm_wide_kernel" in n for n in names), names
+    ops.launch(d)
     first = out.cpu().numpy().copy()
     ops.launch(d)
     torch.cuda.synchronize()
     assert int(status.item()) == 0 and np.array_equal(first, out.cpu().numpy(), equal_nan=True)
+    from gpu_util import kernels_of
+
+    names = kernels_of(lambda: ops.launch(d))
+    assert any("qgemm_wide_kernel" in n for n in names), names
     return first.astype(np.float64)
 
 
